@@ -38,6 +38,7 @@ inline cudaStream_t S(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 #include "sk_device.cuh"
+#include "coulomb.cuh"
 
 // One thread per matrix element (mu, nu); the value is the reference's
 // lower-triangle element for (max, min), so both triangles are written
@@ -243,7 +244,7 @@ __global__ void monopoles_kernel(int norb, int nat, const double *P, const doubl
 // with arbitrary element strides, a two-level batch index and optional split-K
 // (atomic accumulation).  64x64x16 tiles, 256 threads, 4x4 outputs per thread.
 // ----------------------------------------------------------------------------
-enum { EPI_STORE = 0, EPI_ATOMIC = 1, EPI_RV = 2 };
+enum { EPI_STORE = 0, EPI_ATOMIC = 1 };
 
 struct GemmP {
     int M, N, K;
@@ -256,13 +257,6 @@ struct GemmP {
     double alpha, beta;
     int nb2;     // batch index z_b -> (z_b / nb2, z_b % nb2)
     int ksplit;  // gridDim.z = nbatch * ksplit
-    int bscale_sqrt_omega;  // multiply B(k, n) by sqrt(omega[k])
-    const double *omega;
-    // EPI_RV: C(m,n) = omega[m]^p * v(m,n) + fac * sqrt(omega[m])^s * alpha * acc
-    const double *v;
-    long long ldv;
-    double fac;
-    int rv_square;  // 1: omega^2 v + fac sqrt(omega) acc (Hermitian), 0: omega v + fac acc
 };
 
 constexpr int BM = 64, BN = 64, BK = 16;
@@ -313,7 +307,6 @@ __global__ void __launch_bounds__(256) dgemm_kernel(GemmP p) {
             double bv = 0.0;
             if (gn < p.N && gkb < k1) {
                 bv = B[(long long)gkb * p.sbk + gn * p.sbn];
-                if (p.bscale_sqrt_omega) bv *= sqrt(p.omega[gkb]);
             }
             Bs[kb][nn] = bv;
         }
@@ -344,12 +337,8 @@ __global__ void __launch_bounds__(256) dgemm_kernel(GemmP p) {
             const double val = p.alpha * acc[i][j];
             if (EPI == EPI_STORE) {
                 *c = (p.beta == 0.0) ? val : val + p.beta * (*c);
-            } else if (EPI == EPI_ATOMIC) {
-                atomicAdd(c, val);
             } else {
-                const double om = p.omega[m];
-                const double vv = p.v[m * p.ldv + n];
-                *c = p.rv_square ? om * om * vv + p.fac * sqrt(om) * val : om * vv + p.fac * val;
+                atomicAdd(c, val);
             }
         }
     }
@@ -371,22 +360,9 @@ int launch_gemm(GemmP p, int epi, int nbatch, cudaStream_t st) {
     if (grid.y > 65535u || grid.z > 65535u) return fail(DFTB_ERR_BAD_SIZE, "gemm: grid too large");
     if (epi == EPI_STORE)
         dgemm_kernel<EPI_STORE><<<grid, 256, 0, st>>>(p);
-    else if (epi == EPI_ATOMIC)
-        dgemm_kernel<EPI_ATOMIC><<<grid, 256, 0, st>>>(p);
     else
-        dgemm_kernel<EPI_RV><<<grid, 256, 0, st>>>(p);
+        dgemm_kernel<EPI_ATOMIC><<<grid, 256, 0, st>>>(p);
     return check_launch("dgemm_kernel");
-}
-
-// choose a K split so that about 4 CTAs per SM are in flight
-int pick_ksplit(int M, int N, int K, int nbatch) {
-    const long long tiles = (long long)cdiv(M, BM) * cdiv(N, BN) * nbatch;
-    long long want = (148LL * 4 + tiles - 1) / tiles;
-    const long long maxs = (K + 4 * BK - 1) / (4 * BK);  // at least 4 k-tiles per split
-    if (want > maxs) want = maxs;
-    if (want < 1) want = 1;
-    if (want * nbatch > 65535) want = 65535 / nbatch;
-    return (int)(want < 1 ? 1 : want);
 }
 
 // ----------------------------------------------------------------------------
@@ -412,13 +388,6 @@ __global__ void prefix_kernel(int nat, const int *opa, int *first) {
 // adjacent pairs of q with 16-byte stores (each warp stores 512 contiguous bytes of one row p).  Atoms with up
 // to TC_MAXO orbitals (s and p shells) take the staged path; larger ones read their rows from global memory.
 constexpr int TC_TP = 64, TC_TQ = 128, TC_THREADS = 256, TC_MAXO = 4, TC_ATOMS = 8, TC_ROWS = 4;
-
-__device__ __forceinline__ void cp_async8(void *dst, const double *src, bool valid) {
-    // 8-byte asynchronous copy; with src-size 0 the destination is zero-filled and nothing is read
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(valid ? 8 : 0)
-                 : "memory");
-}
 
 struct TcStage {
     double c1[TC_MAXO][TC_TP], s1[TC_MAXO][TC_TP], c2[TC_MAXO][TC_TQ], s2[TC_MAXO][TC_TQ];
@@ -573,7 +542,7 @@ __global__ void tc_diag_kernel(int n, const int *first, const double *C, const d
     q[(size_t)A * n + p] = 0.5 * acc;
 }
 
-// cuBLAS for plain FP64 GEMMs (the Coulomb product's two, the transition charges' S.C).  The library is resolved at run
+// cuBLAS for plain FP64 GEMMs (the wide Coulomb product's two, the transition charges' S.C).  The library is resolved at run
 // time (dlopen / dlsym, reusing the copy the process has already loaded), so the shared library
 // loads without it and the product falls back to dgemm_kernel.
 using blas_create_t = cublasStatus_t (*)(cublasHandle_t *);
@@ -755,32 +724,66 @@ __global__ void rv_inplace_kernel(long long total, int nvec, const double *omega
     us[i] = omega[i / nvec] * vs[i] + fac * us[i];
 }
 
-//   T = q_ov . (s o V)   (split-K, atomic), G = gamma . T,  us = epilogue(q_ov^T G)
-// The non-Hermitian form (s = 1) runs its two large GEMMs in cuBLAS when it is available:
-// row-major X (r x c) is the column-major X^T, so T^T = V^T q_ov^T and us^T = G^T q_ov.
+template <int NT, bool HERM>
+int launch_qv(const QvP &p, unsigned rows, unsigned ks, unsigned cols, cudaStream_t st) {
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        if (cudaFuncSetAttribute(qv_kernel<NT, HERM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 Skinny<NT>::SMEM) != cudaSuccess)
+            return fail(DFTB_ERR_CUDA, "coulomb: shared memory");
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    qv_kernel<NT, HERM><<<dim3(rows, ks, cols), QV_THREADS, Skinny<NT>::SMEM, st>>>(p);
+    return check_launch("qv_kernel");
+}
+
+template <int NT>
+int launch_qv(const QvP &p, unsigned rows, unsigned ks, unsigned cols, cudaStream_t st) {
+    return p.omega ? launch_qv<NT, true>(p, rows, ks, cols, st) : launch_qv<NT, false>(p, rows, ks, cols, st);
+}
+
+// T = Q (s o V) for up to 32 columns at a time (T zeroed by the caller): the columns of Q are cut so that two
+// CTAs per SM are in flight
+int skinny_product(int M, int K, const double *Q, const double *V, int ncol, double *T, const double *omega,
+                   cudaStream_t st) {
+    const unsigned rows = cdiv(M, QV_M), cols = cdiv(ncol, 32);
+    const long long want = 296 / ((long long)rows * cols);
+    const long long chunks = cdiv(K, QV_K);
+    long long ks = want < 1 ? 1 : (want > chunks ? chunks : want);
+    const long long per = (chunks + ks - 1) / ks;
+    ks = (chunks + per - 1) / per;
+    const QvP p{M, K, Q, V, ncol, ncol, T, ncol, omega, (int)(per * QV_K)};
+    switch (cols > 1 ? 4 : (int)cdiv(ncol, 8)) {
+        case 1: return launch_qv<1>(p, rows, (unsigned)ks, cols, st);
+        case 2: return launch_qv<2>(p, rows, (unsigned)ks, cols, st);
+        case 3: return launch_qv<3>(p, rows, (unsigned)ks, cols, st);
+        default: return launch_qv<4>(p, rows, (unsigned)ks, cols, st);
+    }
+}
+
+//   T = q_ov . (s o V)   (atomic over the column ranges), G = gamma . T,  us = epilogue(q_ov^T G)
+// The non-Hermitian form (s = 1) of more than COULOMB_SKINNY columns runs its two large GEMMs in cuBLAS when it
+// is available: row-major X (r x c) is the column-major X^T, so T^T = V^T q_ov^T and us^T = G^T q_ov.  The line is
+// where a second block of 32 columns would read q_ov again (C1014H90: 30 columns 8.4 ms here, 16 columns 5.3 ms here
+// and 8.1 ms in cuBLAS, 60 columns 12.6 ms in cuBLAS and 17 ms in two blocks).  The Hermitian form has no cuBLAS
+// route and takes as many blocks as it needs.
+constexpr int COULOMB_SKINNY = 32;
 int coulomb_product(int nat, int nov, int nvec, const double *gamma, const double *q_ov, const double *omega,
                     const double *vs, double *us, double *T, double *G, int hermitian, cudaStream_t st) {
-    cublasHandle_t bh = hermitian ? nullptr : blas_handle(st);
+    // T and G are adjacent in the workspace: one memset zeroes both
+    const size_t bytes = (size_t)((char *)G - (char *)T) + sizeof(double) * (size_t)nat * nvec;
+    cudaError_t e = cudaMemsetAsync(T, 0, bytes, st);
+    if (e != cudaSuccess) return fail(DFTB_ERR_CUDA, "memset T");
+    int rc;
+    cublasHandle_t bh = hermitian || nvec <= COULOMB_SKINNY ? nullptr : blas_handle(st);
     if (bh) {
         const double one = 1.0, zero = 0.0;
         if (blas().dgemm(bh, CUBLAS_OP_N, CUBLAS_OP_N, nvec, nat, nov, &one, vs, nvec, q_ov, nov, &zero, T, nvec) !=
             CUBLAS_STATUS_SUCCESS)
             return fail(DFTB_ERR_CUDA, "coulomb: cublasDgemm (q_ov V) failed");
-        GemmP g = gemm_defaults();
-        g.M = nat;
-        g.N = nvec;
-        g.K = nat;
-        g.A = gamma;
-        g.sam = nat;
-        g.sak = 1;
-        g.B = T;
-        g.sbk = nvec;
-        g.sbn = 1;
-        g.C = G;
-        g.scm = nvec;
-        g.scn = 1;
-        int rc = launch_gemm(g, EPI_STORE, 1, st);
-        if (rc) return rc;
+        if ((rc = skinny_product(nat, nat, gamma, T, nvec, G, nullptr, st))) return rc;
         if (blas().dgemm(bh, CUBLAS_OP_N, CUBLAS_OP_T, nvec, nov, nat, &one, G, nvec, q_ov, nov, &zero, us, nvec) !=
             CUBLAS_STATUS_SUCCESS)
             return fail(DFTB_ERR_CUDA, "coulomb: cublasDgemm (q_ov^T G) failed");
@@ -788,60 +791,18 @@ int coulomb_product(int nat, int nov, int nvec, const double *gamma, const doubl
         rv_inplace_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(total, nvec, omega, vs, us, 4.0);
         return check_launch("rv_inplace_kernel");
     }
-    cudaError_t e = cudaMemsetAsync(T, 0, sizeof(double) * (size_t)nat * nvec, st);
-    if (e != cudaSuccess) return fail(DFTB_ERR_CUDA, "memset T");
-    GemmP p = gemm_defaults();
-    p.M = nat;
-    p.N = nvec;
-    p.K = nov;
-    p.A = q_ov;
-    p.sam = nov;
-    p.sak = 1;
-    p.B = vs;
-    p.sbk = nvec;
-    p.sbn = 1;
-    p.C = T;
-    p.scm = nvec;
-    p.scn = 1;
-    p.bscale_sqrt_omega = hermitian;
-    p.omega = omega;
-    p.ksplit = pick_ksplit(nat, nvec, nov, 1);
-    int rc = launch_gemm(p, EPI_ATOMIC, 1, st);
-    if (rc) return rc;
-    GemmP g = gemm_defaults();
-    g.M = nat;
-    g.N = nvec;
-    g.K = nat;
-    g.A = gamma;
-    g.sam = nat;
-    g.sak = 1;
-    g.B = T;
-    g.sbk = nvec;
-    g.sbn = 1;
-    g.C = G;
-    g.scm = nvec;
-    g.scn = 1;
-    rc = launch_gemm(g, EPI_STORE, 1, st);
-    if (rc) return rc;
-    GemmP u = gemm_defaults();
-    u.M = nov;
-    u.N = nvec;
-    u.K = nat;
-    u.A = q_ov;  // (q_ov)^T: element (ia, A) at A*nov + ia
-    u.sam = 1;
-    u.sak = nov;
-    u.B = G;
-    u.sbk = nvec;
-    u.sbn = 1;
-    u.C = us;
-    u.scm = nvec;
-    u.scn = 1;
-    u.omega = omega;
-    u.v = vs;
-    u.ldv = nvec;
-    u.fac = 4.0;
-    u.rv_square = hermitian;
-    return launch_gemm(u, EPI_RV, 1, st);
+    if ((rc = skinny_product(nat, nov, q_ov, vs, nvec, T, hermitian ? omega : nullptr, st))) return rc;
+    if ((rc = skinny_product(nat, nat, gamma, T, nvec, G, nullptr, st))) return rc;
+    const QgP p{nov, nat, q_ov, G, nvec, nvec, omega, vs, us, 4.0, hermitian};
+    const unsigned cols = cdiv(nvec, 32);
+    const dim3 grid(cdiv(nov, QG_THREADS), cols);
+    switch (cols > 1 ? 4 : (int)cdiv(nvec, 8)) {
+        case 1: qg_kernel<1><<<grid, QG_THREADS, 0, st>>>(p); break;
+        case 2: qg_kernel<2><<<grid, QG_THREADS, 0, st>>>(p); break;
+        case 3: qg_kernel<3><<<grid, QG_THREADS, 0, st>>>(p); break;
+        default: qg_kernel<4><<<grid, QG_THREADS, 0, st>>>(p); break;
+    }
+    return check_launch("qg_kernel");
 }
 
 // Exchange terms in the transition-charge form, accumulated into us:
