@@ -9,20 +9,21 @@
 // 2. For each modulus the symmetric residues A' mod p_i and B' mod p_i (|r| <= 128, int8) are multiplied on
 //    the tensor cores with exact int32 accumulation (K < 2^17), and the epilogue keeps the product's residue
 //    mod p_i as int8.
-// 3. Per element, Garner's algorithm turns the N residues into mixed-radix digits (int32 arithmetic), whose
-//    Horner sum in FP64 is A'B' to within FP64 rounding, and C = 2^-(sa[m] + sb[n]) A'B'.
+// 3. Per element, the Chinese remainder sum is formed from pairs of residues in exact FP64 limbs and reduced modulo P,
+//    which gives A'B' to within FP64 rounding, and C = 2^-(sa[m] + sb[n]) A'B'.
 //
 // The only approximation is step 1: each entry of op(A) (op(B)) is carried with `bits` bits relative to
 // the largest entry of its row (column); with N = 16 moduli and K <= 2^17 that is the full 53-bit FP64
 // mantissa.  The tensor-core work is N int8 GEMMs (B200: 4.5 dense int8 POPS against ~35 TFLOP/s of FP64
 // DGEMM).
 //
-// Kernels: ozaki_rowscale_kernel (exponents), ozaki_residue_kernel (int8 residue planes, K-major,
+// Kernels: ozaki_rowscale_kernel and ozaki_colscale_kernel (exponents), ozaki_residue_kernel (int8 residue planes, K-major,
 // zero-padded), ozaki_mma_kernel (persistent tcgen05 GEMM over (M tile, N tile, modulus), TMA operand ring,
-// double-buffered TMEM accumulators, residue epilogue), ozaki_crt_kernel (Garner + Horner + scaling).
+// double-buffered TMEM accumulators, residue epilogue), ozaki_crt_kernel (reconstruction and scaling).
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -44,142 +45,228 @@ constexpr int kModuli[MAXMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 22
 constexpr int KMAX = 131071;                // 128 * 128 * K < 2^31: exact int32 accumulation
 constexpr int SCALE_NONFINITE = -(1 << 20);  // row/column exponent marking an Inf or NaN entry
 
+// Per modulus p; residues are symmetric (|r| <= p / 2) and formed in FP32, see symres().
 struct Tables {
-    int p[MAXMOD];
-    double invp[MAXMOD];
-    int D[MAXMOD][MAXMOD];  // D[j][i] = (p_0 ... p_{i-1}) mod p_j, i < j
-    int Binv[MAXMOD];       // (p_0 ... p_{j-1})^-1 mod p_j
-    uint32_t mb[MAXMOD];    // Barrett multiplier floor(2^32 / p) + 1
-    int bias[MAXMOD];       // p 2^20, a multiple of p above 2^27
-    double q3[MAXMOD / 3 + 1];  // p_3k p_3k+1 p_3k+2, the radix of digit triple k
-    int c18[MAXMOD], c36[MAXMOD];  // 2^18 and 2^36 modulo p
+    float2 np[MAXMOD], invp[MAXMOD];    // -p and 1 / p, twice: the FP32 pair operands
+    uint32_t blo[MAXMOD], bhi[MAXMOD];  // int8 weights 2^(8 j) mod p of the bytes j = 0..3 and 4..7
+    int rinit[MAXMOD];                  // kMagicBits + (-2^54 mod p): undoes the offset that makes the bytes unsigned
+    int c16[MAXMOD];                    // 2^16 mod p, |c16| <= 85
 };
 
-// symmetric residue of t (|t| < 2^27) modulo p without float conversions: u = t + p 2^20 is in
-// [0, 2^29), floor(u mb / 2^32) is floor(u / p) or one more (the multiplier's excess over 2^32 / p is
-// below 1, so u mb / 2^32 exceeds u / p by less than 1/8), and the remainder is corrected once.
-__device__ __forceinline__ int symmod_b(int t, int p, uint32_t mb, int bias) {
-    const uint32_t u = (uint32_t)(t + bias);
-    const uint32_t q = __umulhi(u, mb);
-    int r = (int)(u - q * (uint32_t)p);
-    if (r < 0) r += p;
-    if (r > ((p - 1) >> 1)) r -= p;
-    return r;
+// Reconstruction from the first NM moduli, two at a time: with P_k = p_a p_b and W_k = P / P_k,
+//   X = sum_k W_k u_k mod P,  u_k = r_a A_a + r_b A_b,  A_a = p_b ((P / p_a)^-1 mod p_a) mod P_k
+// (int16 coefficients; |u_k| < 2^23).  W_k and P are held as balanced 28-bit limbs in FP64.
+struct CrtTables {
+    int a[MAXMOD / 2];           // A_a | A_b << 16
+    double w[MAXMOD / 2][4];     // limbs of W_k
+    double p[4];                 // limbs of P
+    double qscale;               // 2^(28 (limbs - 1)) / P
+};
+
+constexpr int kMagicBits = 0x4B400000;     // 1.5 2^23: adding it to an integer |t| < 2^22 gives the float 1.5 2^23 + t
+constexpr float kMagic = 12582912.0f;
+
+// FP32 pair arithmetic: one instruction slot for two operations (the residue and epilogue loops are issue-bound)
+__device__ __forceinline__ uint64_t f32x2(float a, float b) {
+    return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// Two words whose low bytes are the symmetric residues of t modulo p, from the bits of the floats 1.5 2^23 + t,
+// |t| < 2^22: t / p is rounded to an integer q with an error below 2^-11 (FP32 product against 1.5 2^23, whose ulp
+// is 1), so t - p q is within p / 2 + 0.1 of zero, exact, and for odd p the canonical residue (for p = 256, +-128
+// are one byte).
+__device__ __forceinline__ void symres2(int tm0, int tm1, uint64_t np, uint64_t invp, uint32_t &r0, uint32_t &r1) {
+    const uint64_t magic = f32x2(kMagic, kMagic), nmagic = f32x2(-kMagic, -kMagic);
+    const uint64_t tm = (uint64_t)(uint32_t)tm0 | (uint64_t)(uint32_t)tm1 << 32;
+    const uint64_t q = add2(fma2(add2(tm, nmagic), invp, magic), nmagic);
+    const uint64_t r = fma2(np, q, tm);
+    r0 = (uint32_t)r;
+    r1 = (uint32_t)(r >> 32);
+}
+
+__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
+__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {  // unsigned bytes of a, signed bytes of b
+    int d;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// 2^e as a double, |e| <= 1022
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+// x 2^e for any e (exact unless the result leaves the normal range)
+__device__ __forceinline__ double scale2(double x, int e) {
+    return (unsigned)(e + 1000) <= 2000u ? x * pow2(e) : ldexp(x, e);
 }
 
 // ---------------------------------------------------------------------------- scaling and residues
 
-// Y(r, k) = trans ? X[k * ldx + r] : X[r * ldx + k]; s[r] = bits - 1 - ilogb(max_k |Y(r, k)|) so that
+// Y(r, k) = X[r * ldx + k]; s[r] = bits - 1 - ilogb(max_k |Y(r, k)|) so that
 // |Y(r, k)| 2^s[r] < 2^bits (0 for a zero row, SCALE_NONFINITE for a row holding Inf or NaN); rows in
 // [rows, rpad) get 0.
-__global__ void ozaki_rowscale_kernel(int rows, int rpad, int K, const double *X, long long ldx, int trans, int bits,
-                                      int *s) {
-    if (!trans) {
-        const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-        if (warp >= rpad) return;
-        double m = 0.0;
-        bool bad = false;
-        if (warp < rows) {
-            const double *x = X + (long long)warp * ldx;
-            int k = lane;
-            for (; k + 96 < K; k += 128) {
-                // four independent loads in flight per lane
-                const double a0 = fabs(x[k]), a1 = fabs(x[k + 32]), a2 = fabs(x[k + 64]), a3 = fabs(x[k + 96]);
-                bad |= !(a0 <= 1.7976931348623157e308 && a1 <= 1.7976931348623157e308 &&
-                         a2 <= 1.7976931348623157e308 && a3 <= 1.7976931348623157e308);
-                m = fmax(fmax(m, fmax(a0, a1)), fmax(a2, a3));
-            }
-            for (; k < K; k += 32) {
-                const double a = fabs(x[k]);
-                bad |= !(a <= 1.7976931348623157e308);
-                m = fmax(m, a);
-            }
+__global__ void ozaki_rowscale_kernel(int rows, int rpad, int K, const double *X, long long ldx, int bits, int *s) {
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (warp >= rpad) return;
+    double m = 0.0;
+    bool bad = false;
+    if (warp < rows) {
+        const double *x = X + (long long)warp * ldx;
+        int k = lane;
+        for (; k + 96 < K; k += 128) {
+            // four independent loads in flight per lane
+            const double a0 = fabs(x[k]), a1 = fabs(x[k + 32]), a2 = fabs(x[k + 64]), a3 = fabs(x[k + 96]);
+            bad |= !(a0 <= 1.7976931348623157e308 && a1 <= 1.7976931348623157e308 &&
+                     a2 <= 1.7976931348623157e308 && a3 <= 1.7976931348623157e308);
+            m = fmax(fmax(m, fmax(a0, a1)), fmax(a2, a3));
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-            bad |= __shfl_xor_sync(0xffffffffu, (int)bad, o) != 0;
-        }
-        if (lane == 0) s[warp] = bad ? SCALE_NONFINITE : (m > 0.0 ? bits - 1 - ilogb(m) : 0);
-    } else {
-        // 32 rows per block (threadIdx.x, consecutive in memory), 32 phases of k (threadIdx.y)
-        __shared__ double sm[32][32];
-        __shared__ int sbad[32][32];
-        const int r = blockIdx.x * 32 + threadIdx.x;
-        double m = 0.0;
-        int bad = 0;
-        if (r < rows) {
-            for (int k = threadIdx.y; k < K; k += 32) {
-                const double a = fabs(X[(long long)k * ldx + r]);
-                bad |= !(a <= 1.7976931348623157e308);
-                m = fmax(m, a);
-            }
-        }
-        sm[threadIdx.y][threadIdx.x] = m;
-        sbad[threadIdx.y][threadIdx.x] = bad;
-        __syncthreads();
-        if (threadIdx.y == 0 && r < rpad) {
-            for (int y = 1; y < 32; ++y) {
-                m = fmax(m, sm[y][threadIdx.x]);
-                bad |= sbad[y][threadIdx.x];
-            }
-            s[r] = bad ? SCALE_NONFINITE : (m > 0.0 ? bits - 1 - ilogb(m) : 0);
+        for (; k < K; k += 32) {
+            const double a = fabs(x[k]);
+            bad |= !(a <= 1.7976931348623157e308);
+            m = fmax(m, a);
         }
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        bad |= __shfl_xor_sync(0xffffffffu, (int)bad, o) != 0;
+    }
+    if (lane == 0) s[warp] = bad ? SCALE_NONFINITE : (m > 0.0 ? bits - 1 - ilogb(m) : 0);
+}
+
+// The same for rows that are strided in memory (Y(r, k) = X[k * ldx + r]): a cluster of RC_SPLIT CTAs takes 32 rows
+// (consecutive in memory), each CTA a range of k with 16 phases, and the first CTA joins their maxima.
+// Split because 4146 rows are 130 blocks, too few loads in flight for one pass over 137 MB: 42 -> 39 us for 4146 x 4146,
+// and 96 us before with 32 phases in one block.
+constexpr int RC_SPLIT = 8, RC_PHASES = 8;
+__global__ void __cluster_dims__(1, RC_SPLIT, 1) __launch_bounds__(32 * RC_PHASES)
+    ozaki_colscale_kernel(int rows, int rpad, int K, const double *X, long long ldx, int bits, int *s) {
+    __shared__ double sm[RC_PHASES][32];
+    __shared__ double best[32];  // this CTA's maximum per row; infinite for a row holding Inf or NaN
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tx = threadIdx.x, ty = threadIdx.y, r = blockIdx.x * 32 + tx;
+    const int kper = (K + RC_SPLIT - 1) / RC_SPLIT;
+    const int k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    double m = 0.0;
+    if (r < rows) {
+        int k = k0 + ty;
+        for (; k + 7 * RC_PHASES < k1; k += 8 * RC_PHASES) {
+            double a[8];
+            const double *x = X + (long long)k * ldx + r;
+#pragma unroll
+            for (int u = 0; u < 8; ++u, x += RC_PHASES * ldx) a[u] = fabs(*x);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) m = a[u] <= m ? m : (a[u] < inf ? a[u] : inf);  // NaN fails both: infinite
+        }
+        for (; k < k1; k += RC_PHASES) {
+            const double a = fabs(X[(long long)k * ldx + r]);
+            m = a <= m ? m : (a < inf ? a : inf);
+        }
+    }
+    sm[ty][tx] = m;
+    __syncthreads();
+    if (ty == 0) {
+#pragma unroll
+        for (int y = 1; y < RC_PHASES; ++y) m = fmax(m, sm[y][tx]);
+        best[tx] = m;
+    }
+    cluster.sync();
+    if (cluster.block_rank() == 0 && ty == 0 && r < rpad) {
+        for (int c = 1; c < RC_SPLIT; ++c) m = fmax(m, *cluster.map_shared_rank(&best[tx], c));
+        s[r] = m == inf ? SCALE_NONFINITE : (m > 0.0 ? bits - 1 - ilogb(m) : 0);
+    }
+    cluster.sync();  // the other CTAs' shared memory stays until it has been read
 }
 
 constexpr int RT_ROWS = 32, RT_K = 128;
 
 // Residue planes R[i][r][k] (i < nmod, r < rows_write, k < kpad; zero outside rows x K) of the scaled,
-// rounded Y(r, k) 2^s[r].  One block per 32 x 128 tile of Y, staged through shared memory so that both the
-// FP64 reads (along k, or along r when transposed) and the int8 writes (4 consecutive k per thread) coalesce.
-template <int NM>
+// rounded Y(r, k) 2^s[r].  One block per 32 x 128 tile of Y; a warp takes four rows, a lane four consecutive k of each,
+// so the int8 writes are 128 contiguous bytes.  Rows that are contiguous in memory are read straight into registers;
+// strided ones (TRANS) are read along r and turned in shared memory, in 16-byte slots swizzled by the row.  Bound by
+// instruction issue, then by DRAM: about 6 instructions per entry and modulus (two dp4a, two FP32 pair operations for
+// two entries, packing).  B200, 4146 x 4146, 16 moduli (430 MB): 187 -> 90 us (rows contiguous) and 95 us (strided).
+template <int NM, bool TRANS>
 __global__ void __launch_bounds__(256) ozaki_residue_kernel(int rows, int rows_write, int K, const double *X,
-                                                            long long ldx, int trans, const int *s,
+                                                            long long ldx, const int *s,
                                                             const __grid_constant__ Tables tb, int8_t *R,
                                                             long long plane, int kpad) {
-    __shared__ double tile[RT_ROWS][RT_K + 1];
+    __shared__ __align__(16) double tile[TRANS ? RT_ROWS * RT_K : 2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r0 = blockIdx.y * RT_ROWS, k0 = blockIdx.x * RT_K;
-    for (int idx = threadIdx.x; idx < RT_ROWS * RT_K; idx += blockDim.x) {
-        int rr, kk;
-        if (trans) {
-            rr = idx % RT_ROWS;
-            kk = idx / RT_ROWS;
-        } else {
-            rr = idx / RT_K;
-            kk = idx % RT_K;
+    const int k = k0 + 4 * lane;
+    double x[4][4];
+    if (TRANS) {
+        const double *p = X + (long long)(k0 + warp) * ldx + r0 + lane;
+        const bool in = r0 + lane < rows;
+        double v[RT_K / 8];
+#pragma unroll
+        for (int j = 0; j < RT_K / 8; ++j, p += 8 * ldx) v[j] = (in && k0 + warp + 8 * j < K) ? *p : 0.0;
+#pragma unroll
+        for (int j = 0; j < RT_K / 8; ++j) {
+            const int kk = warp + 8 * j;
+            tile[lane * RT_K + (((kk >> 1) ^ (lane & 7)) << 1) + (kk & 1)] = v[j];
         }
-        const int r = r0 + rr, k = k0 + kk;
-        double v = 0.0;
-        if (r < rows && k < K) v = trans ? X[(long long)k * ldx + r] : X[(long long)r * ldx + k];
-        tile[rr][kk] = v;
+        __syncthreads();
+    } else {
+        const bool vec = ((ldx & 1) | (reinterpret_cast<uintptr_t>(X) & 8)) == 0 && k + 3 < K;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = r0 + warp + 8 * j;
+            const double *p = X + (long long)r * ldx + k;
+            if (r < rows && vec) {
+                const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+                x[j][0] = a.x, x[j][1] = a.y, x[j][2] = b.x, x[j][3] = b.y;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[j][e] = (r < rows && k + e < K) ? p[e] : 0.0;
+            }
+        }
     }
-    __syncthreads();
-    for (int item = threadIdx.x; item < RT_ROWS * (RT_K / 4); item += blockDim.x) {
-        const int rr = item / (RT_K / 4), kq = (item % (RT_K / 4)) * 4;
-        const int r = r0 + rr, k = k0 + kq;
-        if (k >= kpad || r >= rows_write) continue;
-        const int sr = (r < rows) ? s[r] : 0;
-        // the scaled, rounded entries (at most 53 bits) as h 2^36 + m 2^18 + l, |h| <= 2^17, 0 <= m, l < 2^18
-        int h[4], md[4], l[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int rr = warp + 8 * j, r = r0 + rr;
+        if (r >= rows_write) break;
+        if (TRANS) {
+            const double2 a = *reinterpret_cast<const double2 *>(tile + rr * RT_K + (((2 * lane) ^ (rr & 7)) << 1));
+            const double2 b = *reinterpret_cast<const double2 *>(tile + rr * RT_K + (((2 * lane + 1) ^ (rr & 7)) << 1));
+            x[j][0] = a.x, x[j][1] = a.y, x[j][2] = b.x, x[j][3] = b.y;
+        }
+        const int sr = r < rows ? s[r] : SCALE_NONFINITE;
+        // the scaled, rounded entries (at most 53 bits) plus 2^54, as seven unsigned bytes
+        uint32_t lo[4], hi[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const long long ai =
-                (sr == SCALE_NONFINITE || r >= rows) ? 0ll : __double2ll_rn(ldexp(tile[rr][kq + e], sr));
-            h[e] = (int)(ai >> 36);
-            md[e] = (int)((ai >> 18) & 0x3FFFF);
-            l[e] = (int)(ai & 0x3FFFF);
+            const long long ai = sr == SCALE_NONFINITE ? 0ll : __double2ll_rn(scale2(x[j][e], sr));
+            const unsigned long long u = (unsigned long long)(ai + (1ll << 54));
+            lo[e] = (uint32_t)u;
+            hi[e] = (uint32_t)(u >> 32);
         }
+        int8_t *out = R + (long long)r * kpad + k;
 #pragma unroll
-        for (int i = 0; i < NM; ++i) {
-            uint32_t w = 0;
+        for (int i = 0; i < NM; ++i, out += plane) {
+            const uint64_t np = f32x2(tb.np[i].x, tb.np[i].y), invp = f32x2(tb.invp[i].x, tb.invp[i].y);
+            int t[4];
+            uint32_t rd[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                // |h c36 + m c18 + l| < 2^25 + 2^26 + 2^18 < 2^27
-                const int t = h[e] * tb.c36[i] + md[e] * tb.c18[i] + l[e];
-                const int rd = symmod_b(t, tb.p[i], tb.mb[i], tb.bias[i]);
-                w |= ((uint32_t)(uint8_t)(int8_t)rd) << (8 * e);
-            }
-            *reinterpret_cast<uint32_t *>(R + i * plane + (long long)r * kpad + k) = w;
+            for (int e = 0; e < 4; ++e)  // seven products below 255 127: |t| < 2^18
+                t[e] = dp4a_us(lo[e], tb.blo[i], dp4a_us(hi[e], tb.bhi[i], tb.rinit[i]));
+            symres2(t[0], t[1], np, invp, rd[0], rd[1]);
+            symres2(t[2], t[3], np, invp, rd[2], rd[3]);
+            *reinterpret_cast<uint32_t *>(out) = pack4(rd[0], rd[1], rd[2], rd[3]);
         }
     }
 }
@@ -227,7 +314,9 @@ struct MmaParams {
 //                   (128-byte swizzle);
 //   warp 1 lane 0 : tcgen05.mma kind::i8 issuer (M = 128, N = 256, K = 32 per instruction) into one of two
 //                   256-column int32 TMEM accumulators (tile j uses accumulator j % 2);
-//   warps 2..5    : epilogue of tile j under the MMAs of tile j + 1: int32 -> residue mod p -> int8.
+//   warps 2..5    : epilogue of tile j under the MMAs of tile j + 1: int32 -> residue mod p -> int8.  It must take less
+//                   than a tile's MMAs (7k cycles at K = 1225): in FP64 it did not (8292 x 8292 x 1225, 14 moduli:
+//                   1.49 ms), in FP32 pairs it does (1.06 ms).
 // Every wait is bounded; on timeout the kernel records an error code, stops issuing, drains its copies
 // and releases TMEM.
 __global__ void __launch_bounds__(192, 1) ozaki_mma_kernel(const __grid_constant__ Maps maps, const MmaParams p,
@@ -348,8 +437,8 @@ __global__ void __launch_bounds__(192, 1) ozaki_mma_kernel(const __grid_constant
             const int mi = t % mt, ni = (t / mt) % nt, mod = t / (mt * nt);
             const int acc = j & 1;
             const int row = mi * BM + rloc, n0 = ni * BN;
-            const int pm = tb.p[mod];
-            const double invpd = tb.invp[mod];
+            const uint64_t np = f32x2(tb.np[mod].x, tb.np[mod].y), invp = f32x2(tb.invp[mod].x, tb.invp[mod].y);
+            const int c16 = tb.c16[mod];
             const bool ok = __all_sync(0xffffffffu, mbar_wait(&tfull[acc], (j >> 1) & 1) ? 1 : 0) != 0;
             if (!ok && lane == 0) atomicExch(p.err, 3);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -362,18 +451,17 @@ __global__ void __launch_bounds__(192, 1) ozaki_mma_kernel(const __grid_constant
                     uint32_t w[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        uint32_t word = 0;
+                        // a = ah 2^16 + al: |ah c16 + al| <= 2^15 85 + 2^16 < 2^22
+                        int t[4];
+                        uint32_t rd[4];
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            // |a| < 2^31 is exact in FP64, so q is round(a / p) or one off near a tie
                             const int a = (int)v[4 * q + e];
-                            const long long qq = (long long)rint((double)a * invpd);
-                            int r = (int)((long long)a - qq * pm);
-                            if (r > ((pm - 1) >> 1)) r -= pm;
-                            if (r < -(pm >> 1)) r += pm;
-                            word |= ((uint32_t)(uint8_t)(int8_t)r) << (8 * e);
+                            t[e] = (a >> 16) * c16 + ((a & 0xffff) | kMagicBits);
                         }
-                        w[q] = word;
+                        symres2(t[0], t[1], np, invp, rd[0], rd[1]);
+                        symres2(t[2], t[3], np, invp, rd[2], rd[3]);
+                        w[q] = pack4(rd[0], rd[1], rd[2], rd[3]);
                     }
                     uint4 *dst = reinterpret_cast<uint4 *>(p.RC + mod * p.planeC + (long long)row * p.ldr + col0);
                     dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -394,56 +482,68 @@ __global__ void __launch_bounds__(192, 1) ozaki_mma_kernel(const __grid_constant
 
 // ---------------------------------------------------------------------------- reconstruction
 
-// C[m][n] = alpha G[m][n] 2^-(sa[m] + sb[n]) X + beta C[m][n] (G optional), X the integer with residues RC[i][m][n] (Garner's
-// mixed-radix digits v_j, symmetric, X = v_0 + p_0 (v_1 + p_1 (v_2 + ...)) evaluated in FP64).  Four
-// consecutive columns per thread (one 32-bit word per residue plane); NM moduli.
+constexpr __host__ __device__ int crt_limbs(int nmod) { return nmod >= 13 ? 4 : (nmod >= 9 ? 3 : 2); }
+
+// C[m][n] = alpha G[m][n] 2^-(sa[m] + sb[n]) X + beta C[m][n] (G optional), X the integer with residues RC[i][m][n]:
+// the limbs S_l = sum_k u_k W_k,l are exact in FP64 (|u_k| < 2^23, |W_k,l| <= 2^27, 8 terms), Q = round(S / P) from the
+// three highest, and X = sum_l (S_l - Q P_l) 2^(28 l), rounded at most once per limb below the first that exceeds 53 bits.
+// Four consecutive columns per thread (one 32-bit word per residue plane); NM moduli.  Per entry it costs 8 PRMT, 8 dp2a
+// and ~55 FP64 operations, where the mixed-radix (Garner) form took 120 multiply-adds and 15 reductions: B200, 4146 x
+// 4146 from 16 planes (413 MB) 282 -> 99 us, 8292 x 8292 from 14 planes 1080 -> 360 us.
 template <int NM>
 __global__ void __launch_bounds__(256) ozaki_crt_kernel(int M, int N, const int8_t *RC, long long planeC, int ldr,
                                                         const int *sa, const int *sb, double alpha, const double *G,
                                                         long long ldg, double beta, double *C, long long ldc,
-                                                        const __grid_constant__ Tables tb) {
+                                                        const __grid_constant__ CrtTables tb) {
+    constexpr int NP = (NM + 1) / 2, NL = crt_limbs(NM), NW = (NM + 3) / 4;
     const int nq = (N + 3) / 4;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)M * nq) return;
     const int m = (int)(idx / nq), n0 = (int)(idx % nq) * 4;
-    uint32_t wd[NM];
+    uint32_t wd[4 * NW];
 #pragma unroll
-    for (int i = 0; i < NM; ++i)
-        wd[i] = *reinterpret_cast<const uint32_t *>(RC + i * planeC + (long long)m * ldr + n0);
+    for (int i = 0; i < 4 * NW; ++i)
+        wd[i] = i < NM ? *reinterpret_cast<const uint32_t *>(RC + i * planeC + (long long)m * ldr + n0) : 0u;
+    // 4 x 4 byte transposes: word 4 g + e then holds the residues modulo p_4g .. p_4g+3 of column e
+#pragma unroll
+    for (int g = 0; g < NW; ++g) {
+        uint32_t *w = wd + 4 * g;
+        const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+        const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+        w[0] = __byte_perm(a, b, 0x5410);
+        w[1] = __byte_perm(a, b, 0x7632);
+        w[2] = __byte_perm(c, d, 0x5410);
+        w[3] = __byte_perm(c, d, 0x7632);
+    }
     const int sm = sa[m];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const int n = n0 + e;
         if (n >= N) break;
-        int v[NM];
-        v[0] = (int)(int8_t)(uint8_t)(wd[0] >> (8 * e));
+        double S[NL];
 #pragma unroll
-        for (int jj = 1; jj < NM; ++jj) {
-            // |r - sum_i v_i D| <= 128 + 15 * 128 * 255 < 2^19 and Binv <= 255: the product stays below 2^27
-            int acc = (int)(int8_t)(uint8_t)(wd[jj] >> (8 * e));
+        for (int l = 0; l < NL; ++l) S[l] = 0.0;
 #pragma unroll
-            for (int i = 0; i < jj; ++i) acc -= v[i] * tb.D[jj][i];
-            v[jj] = symmod_b(acc * tb.Binv[jj], tb.p[jj], tb.mb[jj], tb.bias[jj]);
+        for (int k = 0; k < NP; ++k) {
+            const int r = (int)wd[4 * (k / 2) + e];
+            // u + 2^24 > 0 in the low word of 2^52 + (u + 2^24)
+            const int u = (k & 1) ? __dp2a_hi(tb.a[k], r, 1 << 24) : __dp2a_lo(tb.a[k], r, 1 << 24);
+            const double ud = __hiloint2double(0x43300000, u) - (4503599627370496.0 + 16777216.0);
+#pragma unroll
+            for (int l = 0; l < NL; ++l) S[l] = fma(ud, tb.w[k][l], S[l]);
         }
-        // Horner over digit triples: each triple v_a + p_a (v_b + p_b v_c) is an exact int32 (< 2^24)
-        constexpr int NG = (NM + 2) / 3;
-        double x = 0.0;
+        double q = fma(S[NL - 2], 0x1p-28, S[NL - 1]);
+        if (NL > 2) q = fma(S[NL > 2 ? NL - 3 : 0], 0x1p-56, q);
+        q = __dsub_rn(fma(q, tb.qscale, 6755399441055744.0), 6755399441055744.0);  // rounded: 1.5 2^52 has ulp 1
+        double x = fma(-q, tb.p[NL - 1], S[NL - 1]);
 #pragma unroll
-        for (int g = NG - 1; g >= 0; --g) {
-            const int a = 3 * g;
-            int t = v[a];
-            if (a + 2 < NM)
-                t += tb.p[a] * (v[a + 1] + tb.p[a + 1] * v[a + 2]);
-            else if (a + 1 < NM)
-                t += tb.p[a] * v[a + 1];
-            x = (g == NG - 1) ? (double)t : fma(x, tb.q3[g], (double)t);
-        }
+        for (int l = NL - 2; l >= 0; --l) x = fma(x, 0x1p28, fma(-q, tb.p[l], S[l]));
         const int sn = sb[n];
         double out;
         if (sm == SCALE_NONFINITE || sn == SCALE_NONFINITE)
             out = __longlong_as_double(0x7ff8000000000000ll);  // NaN
         else
-            out = alpha * ldexp(x, -(sm + sn));
+            out = alpha * scale2(x, -(sm + sn));
         if (G) out *= G[(long long)m * ldg + n];
         double *c = C + (long long)m * ldc + n;
         *c = beta == 0.0 ? out : out + beta * *c;
@@ -452,7 +552,7 @@ __global__ void __launch_bounds__(256) ozaki_crt_kernel(int M, int N, const int8
 
 template <int NM>
 void launch_crt(int M, int N, const int8_t *RC, long long planeC, int ldr, const int *sa, const int *sb, double alpha,
-                const double *G, long long ldg, double beta, double *C, long long ldc, const Tables &tb,
+                const double *G, long long ldg, double beta, double *C, long long ldc, const CrtTables &tb,
                 cudaStream_t st) {
     const long long nthreads = (long long)M * ((N + 3) / 4);
     ozaki_crt_kernel<NM><<<(unsigned)((nthreads + 255) / 256), 256, 0, st>>>(M, N, RC, planeC, ldr, sa, sb, alpha,
@@ -464,7 +564,51 @@ thread_local char g_err[256] = "";
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 std::mutex g_mutex;
 Tables g_tables;
+CrtTables g_crt[MAXMOD + 1];
 bool g_tables_ready = false;
+
+using u128 = unsigned __int128;
+
+// balanced 28-bit limbs of v, the highest unreduced
+void limbs28(u128 v, int n, double *out) {
+    for (int l = 0; l < n - 1; ++l) {
+        long long d = (long long)(v & ((1u << 28) - 1));
+        v >>= 28;
+        if (d >= (1 << 27)) {
+            d -= 1 << 28;
+            v += 1;
+        }
+        out[l] = (double)d;
+    }
+    out[n - 1] = (double)(unsigned long long)v;
+}
+
+void init_crt(CrtTables &t, int nmod) {
+    const int nl = crt_limbs(nmod);
+    u128 P = 1;
+    for (int i = 0; i < nmod; ++i) P *= (u128)kModuli[i];  // below 2^126
+    limbs28(P, nl, t.p);
+    double Pd = 0.0;
+    for (int l = nl - 1; l >= 0; --l) Pd = Pd * 268435456.0 + t.p[l];
+    t.qscale = ldexp(1.0, 28 * (nl - 1)) / Pd;
+    for (int k = 0; 2 * k < nmod; ++k) {
+        const int pa = kModuli[2 * k], pb = 2 * k + 1 < nmod ? kModuli[2 * k + 1] : 1;
+        const int pk = pa * pb;
+        limbs28(P / (u128)pk, nl, t.w[k]);
+        int A[2] = {0, 0};
+        for (int h = 0; h < 2; ++h) {
+            const int p = h == 0 ? pa : pb, other = h == 0 ? pb : pa;
+            if (p == 1) continue;
+            const int rest = (int)((P / (u128)p) % (u128)p);
+            int inv = 1;
+            while ((long long)rest * inv % p != 1) ++inv;
+            int c = (int)((long long)other * inv % pk);
+            if (c > pk / 2) c -= pk;
+            A[h] = c;
+        }
+        t.a[k] = (int)(((uint32_t)A[0] & 0xffffu) | ((uint32_t)A[1] << 16));
+    }
+}
 
 int init_host() {
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -482,34 +626,21 @@ int init_host() {
     if (!g_tables_ready) {
         Tables &t = g_tables;
         for (int i = 0; i < MAXMOD; ++i) {
-            t.p[i] = kModuli[i];
-            t.invp[i] = 1.0 / (double)kModuli[i];
+            const int p = kModuli[i];
+            auto sym = [p](long long v) {
+                const int r = (int)(((v % p) + p) % p);
+                return r > p / 2 ? r - p : r;
+            };
+            t.np[i] = make_float2(-(float)p, -(float)p);
+            t.invp[i] = make_float2(1.0f / (float)p, 1.0f / (float)p);
+            uint32_t w[2] = {0, 0};
+            for (int j = 0; j < 7; ++j) w[j >> 2] |= (uint32_t)(uint8_t)(int8_t)sym(1ll << (8 * j)) << (8 * (j & 3));
+            t.blo[i] = w[0];
+            t.bhi[i] = w[1];
+            t.rinit[i] = kMagicBits + sym(-(1ll << 54));
+            t.c16[i] = sym(1ll << 16);
         }
-        for (int j = 0; j < MAXMOD; ++j) {
-            const int pj = kModuli[j];
-            long long prod = 1;  // p_0 ... p_{i-1} mod p_j
-            for (int i = 0; i < MAXMOD; ++i) {
-                t.D[j][i] = (i < j) ? (int)prod : 0;
-                if (i < j) prod = (prod * kModuli[i]) % pj;
-            }
-            // prod = p_0 ... p_{j-1} mod p_j; its inverse by search (p_j <= 256)
-            int inv = 0;
-            for (int x = 1; x < pj && j > 0; ++x)
-                if ((prod * x) % pj == 1) {
-                    inv = x;
-                    break;
-                }
-            t.Binv[j] = (j == 0) ? 1 : inv;
-            t.mb[j] = (uint32_t)((1ull << 32) / (unsigned long long)pj + 1ull);
-            t.bias[j] = pj << 20;
-            t.c18[j] = (int)((1ull << 18) % (unsigned long long)pj);
-            t.c36[j] = (int)((1ull << 36) % (unsigned long long)pj);
-        }
-        for (int g = 0; 3 * g < MAXMOD; ++g) {
-            double q = 1.0;
-            for (int i = 3 * g; i < 3 * g + 3 && i < MAXMOD; ++i) q *= (double)kModuli[i];
-            t.q3[g] = q;
-        }
+        for (int nmod = 8; nmod <= MAXMOD; ++nmod) init_crt(g_crt[nmod], nmod);
         g_tables_ready = true;
     }
     return 0;
@@ -585,18 +716,21 @@ int prepare(int trans, int rows, int k, const double *X, long long ldx, int nmod
     int8_t *R = reinterpret_cast<int8_t *>(op + L.off_res) + (long long)row0 * L.kpad;
     if (!trans) {
         const long long threads = (long long)rows_write * 32;
-        ozaki_rowscale_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(rows, rows_write, k, X, ldx, 0, bits,
-                                                                                 s);
+        ozaki_rowscale_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(rows, rows_write, k, X, ldx, bits, s);
     } else {
-        ozaki_rowscale_kernel<<<(unsigned)((rows_write + 31) / 32), dim3(32, 32), 0, st>>>(rows, rows_write, k, X, ldx,
-                                                                                         1, bits, s);
+        ozaki_colscale_kernel<<<dim3((unsigned)((rows_write + 31) / 32), RC_SPLIT), dim3(32, RC_PHASES), 0, st>>>(
+            rows, rows_write, k, X, ldx, bits, s);
     }
     dim3 g((unsigned)(L.kpad / RT_K), (unsigned)((rows_write + RT_ROWS - 1) / RT_ROWS));
     switch (nmod) {
 #define OZK_RES(NMV)                                                                                            \
     case NMV:                                                                                                   \
-        ozaki_residue_kernel<NMV><<<g, 256, 0, st>>>(rows, rows_write, k, X, ldx, trans, s, g_tables, R, L.plane, \
-                                                     (int)L.kpad);                                              \
+        if (trans)                                                                                              \
+            ozaki_residue_kernel<NMV, true><<<g, 256, 0, st>>>(rows, rows_write, k, X, ldx, s, g_tables, R,     \
+                                                               L.plane, (int)L.kpad);                           \
+        else                                                                                                    \
+            ozaki_residue_kernel<NMV, false><<<g, 256, 0, st>>>(rows, rows_write, k, X, ldx, s, g_tables, R,    \
+                                                                L.plane, (int)L.kpad);                          \
         break;
         OZK_RES(8)
         OZK_RES(9)
@@ -655,7 +789,7 @@ int product(int m, int n, int k, int nmod, const uint8_t *A, int rows_a, const u
     switch (nmod) {
 #define OZK_CRT(NMV)                                                                                              \
     case NMV:                                                                                                     \
-        launch_crt<NMV>(m, n, RC, p.planeC, p.ldr, sa, sb, alpha, G, ldg, beta, C, ldc, g_tables, st); \
+        launch_crt<NMV>(m, n, RC, p.planeC, p.ldr, sa, sb, alpha, G, ldg, beta, C, ldc, g_crt[nmod], st); \
         break;
         OZK_CRT(8)
         OZK_CRT(9)
