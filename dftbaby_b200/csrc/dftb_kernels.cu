@@ -13,6 +13,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "dftbaby_b200.h"
 
@@ -240,129 +241,205 @@ __global__ void monopoles_kernel(int norb, int nat, const double *P, const doubl
 }
 
 // ----------------------------------------------------------------------------
-// FP64 tiled GEMM engine.  C(m,n) = alpha * sum_k A(m,k) B(k,n) [+ beta C]
-// with arbitrary element strides, a two-level batch index and optional split-K
-// (atomic accumulation).  64x64x16 tiles, 256 threads, 4x4 outputs per thread.
+// FP64 GEMM engine on the FP64 tensor tiles (mma.m8n8k4):
+//   C(m,n) = alpha * sum_k A(m,k) B(k,n) [+ beta C]
+// with arbitrary element strides, a batch index, optional split-K (atomic accumulation) and two-level indices: k in A
+// as (k / K2, k % K2), n in B and C as (n / N2, n % N2), so that a sum over (atom, orbital) pairs or an output of
+// (orbital, vector) columns is one product without reordering its operands.
+// A CTA of four warps takes a 64 x 64 tile (a warp 32 x 32) in 16-deep stages of a three-deep cp.async ring.  Each
+// operand is staged in the order in which it is contiguous in memory, with a pitch of 4 (mod 16) doubles either way,
+// so copies and fragment reads are both conflict-free; tiles of 8 rows beyond M are skipped.  Bound by the FP64 pipe:
+// 30 TFLOP/s at 4096^3 on B200 (the 4 x 4 register-tile form it replaces ran at 9 to 13; cuBLAS 35).
 // ----------------------------------------------------------------------------
 enum { EPI_STORE = 0, EPI_ATOMIC = 1 };
 
 struct GemmP {
     int M, N, K;
     const double *A;
-    long long sam, sak, sa1, sa2;
+    long long sam, sak, sak1, sa1;  // strides of m, k % K2, k / K2, batch
+    int K2;                         // two-level k needs sak == 1 (else K2 = K)
     const double *B;
-    long long sbk, sbn, sb1, sb2;
+    long long sbk, sbn, sbn1, sb1;  // strides of k, n % N2, n / N2, batch
     double *C;
-    long long scm, scn, sc1, sc2;
+    long long scm, scn, scn1, sc1;
+    int N2;
     double alpha, beta;
-    int nb2;     // batch index z_b -> (z_b / nb2, z_b % nb2)
     int ksplit;  // gridDim.z = nbatch * ksplit
+    int mstep;   // rows per CTA, a multiple of 8 and at most BM: the 8-row tiles of M dealt evenly to the CTAs
 };
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int BM = 64, BN = 64, BK = 16, GEMM_STAGES = 3, GEMM_THREADS = 128;
+constexpr int PITCH_K = BK + 4, PITCH_MN = BM + 4;  // operand tiles [m or n][k] and [k][m or n]
 
-template <int EPI>
-__global__ void __launch_bounds__(256) dgemm_kernel(GemmP p) {
-    __shared__ double As[BK][BM + 1];
-    __shared__ double Bs[BK][BN + 1];
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    const int bm = blockIdx.y * BM, bn = blockIdx.x * BN;
+// AK: A is contiguous along k (else staged along m); BNC: B is contiguous along n (else staged along k)
+template <int EPI, bool AK, bool BNC>
+__global__ void __launch_bounds__(GEMM_THREADS) dgemm_kernel(const GemmP p) {
+    constexpr int A_ELEMS = AK ? BM * PITCH_K : BK * PITCH_MN, B_ELEMS = BNC ? BK * PITCH_MN : BN * PITCH_K;
+    extern __shared__ __align__(16) double gemm_sm[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int bm = blockIdx.y * p.mstep, bn = blockIdx.x * BN, M = min(p.M, bm + p.mstep);
     const int zb = blockIdx.z / p.ksplit, zk = blockIdx.z % p.ksplit;
-    const int z1 = zb / p.nb2, z2 = zb % p.nb2;
-    const double *A = p.A + z1 * p.sa1 + z2 * p.sa2;
-    const double *B = p.B + z1 * p.sb1 + z2 * p.sb2;
-    double *C = p.C + z1 * p.sc1 + z2 * p.sc2;
+    const double *A = p.A + zb * p.sa1, *B = p.B + zb * p.sb1;
+    double *C = p.C + zb * p.sc1;
     const int kchunk = ((p.K + p.ksplit - 1) / p.ksplit + BK - 1) / BK * BK;
     const int k0 = zk * kchunk, k1 = min(p.K, k0 + kchunk);
-    double acc[4][4];
+    const int niter = k1 > k0 ? (k1 - k0 + BK - 1) / BK : 0;
+    auto noff = [&](int n, long long s1, long long s2) { return (n / p.N2) * s1 + (n % p.N2) * s2; };
+
+    // this thread's part of a stage: eight elements of each operand, along its contiguous index from thread to thread
+    const int ka = AK ? tid & 15 : tid >> 6, ma = AK ? tid >> 4 : tid & 63;
+    const int kb = BNC ? tid >> 6 : tid & 15, nb = BNC ? tid & 63 : tid >> 4;
+    int kq = (k0 + ka) / p.K2, kr = (k0 + ka) % p.K2;  // two-level k of A (AK)
+    const double *bcol = B + (BNC && bn + nb < p.N ? noff(bn + nb, p.sbn1, p.sbn) : 0);
+    long long boff[8];
+    if (!BNC) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) boff[i] = bn + nb + 8 * i < p.N ? noff(bn + nb + 8 * i, p.sbn1, p.sbn) : -1;
+    }
+    auto stage = [&](int it) {
+        if (it < niter) {
+            double *as = gemm_sm + (it % GEMM_STAGES) * (A_ELEMS + B_ELEMS), *bs = as + A_ELEMS;
+            const int kt = k0 + it * BK;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int mm = AK ? ma + 8 * i : ma, kk = AK ? ka : ka + 2 * i;
+                const bool v = bm + mm < M && kt + kk < k1;
+                const long long ko = AK ? kq * p.sak1 + kr * p.sak : (long long)(kt + kk) * p.sak;
+                cp_async8(as + (AK ? mm * PITCH_K + kk : kk * PITCH_MN + mm),
+                          v ? A + ((long long)(bm + mm) * p.sam + ko) : A, v);
+            }
+            if (AK) {
+                kr += BK;
+                while (kr >= p.K2) {
+                    kr -= p.K2;
+                    ++kq;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int nn = BNC ? nb : nb + 8 * i, kk = BNC ? kb + 2 * i : kb;
+                const bool v = bn + nn < p.N && kt + kk < k1;
+                const double *src = (BNC ? bcol : B + (v ? boff[BNC ? 0 : i] : 0)) + (v ? (kt + kk) * p.sbk : 0);
+                cp_async8(bs + (BNC ? kk * PITCH_MN + nn : nn * PITCH_K + kk), v ? src : B, v);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    double acc[4][4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    const bool a_k_contig = (p.sak == 1);
-    const bool b_n_contig = (p.sbn == 1);
-    for (int kt = k0; kt < k1; kt += BK) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int e = tid + 256 * r;
-            int mm, kk;
-            if (a_k_contig) {
-                kk = e % BK;
-                mm = e / BK;
-            } else {
-                mm = e % BM;
-                kk = e / BM;
-            }
-            const int gm = bm + mm, gk = kt + kk;
-            As[kk][mm] = (gm < p.M && gk < k1) ? A[gm * p.sam + (long long)gk * p.sak] : 0.0;
-            int nn, kb;
-            if (b_n_contig) {
-                nn = e % BN;
-                kb = e / BN;
-            } else {
-                kb = e % BK;
-                nn = e / BK;
-            }
-            const int gn = bn + nn, gkb = kt + kb;
-            double bv = 0.0;
-            if (gn < p.N && gkb < k1) {
-                bv = B[(long long)gkb * p.sbk + gn * p.sbn];
-            }
-            Bs[kb][nn] = bv;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
+        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    // neighbouring CTAs swap the upper and lower warps, so that short tiles do not all fall to the same SM quarters
+    const int wm = 32 * ((warp ^ blockIdx.x) & 1), wn = 32 * (warp >> 1);
+    const int mtiles = min(4, max(0, (M - bm - wm + 7) / 8)), ntiles = min(4, max(0, (p.N - bn - wn + 7) / 8));
+    const int arow = wm + (lane >> 2), acol = lane & 3, bcol_l = wn + (lane >> 2);
+    for (int s = 0; s < GEMM_STAGES - 1; ++s) stage(s);
+    for (int it = 0; it < niter; ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GEMM_STAGES - 2) : "memory");
+        __syncthreads();  // stage it has landed, and every warp has left stage it - 1
+        stage(it + GEMM_STAGES - 1);
+        const double *as = gemm_sm + (it % GEMM_STAGES) * (A_ELEMS + B_ELEMS), *bs = as + A_ELEMS;
+        auto step = [&](int ks, auto full) {
             double a[4], b[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+            for (int i = 0; i < 4; ++i)
+                a[i] = AK ? as[(arow + 8 * i) * PITCH_K + ks + acol] : as[(ks + acol) * PITCH_MN + arow + 8 * i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+            for (int j = 0; j < 4; ++j)
+                b[j] = BNC ? bs[(ks + acol) * PITCH_MN + bcol_l + 8 * j] : bs[(bcol_l + 8 * j) * PITCH_K + ks + acol];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
+                if (decltype(full)::value || i < mtiles) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                    for (int j = 0; j < 4; ++j) dmma884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                }
+        };
+        if (ntiles == 0) continue;
+        if (mtiles == 4) {  // without branches between the MMAs
+#pragma unroll
+            for (int ks = 0; ks < BK; ks += 4) step(ks, std::true_type());
+        } else {
+#pragma unroll
+            for (int ks = 0; ks < BK; ks += 4) step(ks, std::false_type());
         }
-        __syncthreads();
     }
+    if (EPI == EPI_ATOMIC && niter == 0) return;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = bm + ty + 16 * i;
-        if (m >= p.M) continue;
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = bn + tx + 16 * j;
+        for (int e = 0; e < 2; ++e) {
+            const int n = bn + wn + 8 * j + 2 * (lane & 3) + e;
             if (n >= p.N) continue;
-            double *c = C + m * p.scm + n * p.scn;
-            const double val = p.alpha * acc[i][j];
-            if (EPI == EPI_STORE) {
-                *c = (p.beta == 0.0) ? val : val + p.beta * (*c);
-            } else {
-                atomicAdd(c, val);
+            double *col = C + noff(n, p.scn1, p.scn);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int m = bm + arow + 8 * i;
+                if (m >= M) continue;
+                double *c = col + m * p.scm;
+                const double val = p.alpha * acc[i][j][e];
+                if (EPI == EPI_STORE)
+                    *c = (p.beta == 0.0) ? val : val + p.beta * (*c);
+                else
+                    atomicAdd(c, val);
             }
         }
-    }
 }
 
 GemmP gemm_defaults() {
     GemmP p;
     memset(&p, 0, sizeof(p));
     p.alpha = 1.0;
-    p.nb2 = 1;
     p.ksplit = 1;
     return p;
+}
+
+template <int EPI, bool AK, bool BNC>
+int launch_gemm_as(const GemmP &p, dim3 grid, cudaStream_t st) {
+    constexpr int smem =
+        GEMM_STAGES * (int)sizeof(double) * ((AK ? BM * PITCH_K : BK * PITCH_MN) + (BNC ? BK * PITCH_MN : BN * PITCH_K));
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        if (cudaFuncSetAttribute(dgemm_kernel<EPI, AK, BNC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess)
+            return fail(DFTB_ERR_CUDA, "gemm: shared memory");
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    dgemm_kernel<EPI, AK, BNC><<<grid, GEMM_THREADS, smem, st>>>(p);
+    return check_launch("dgemm_kernel");
 }
 
 int launch_gemm(GemmP p, int epi, int nbatch, cudaStream_t st) {
     if (p.M <= 0 || p.N <= 0 || nbatch <= 0) return DFTB_OK;
     if (p.K <= 0) return fail(DFTB_ERR_BAD_SIZE, "gemm: K <= 0");
-    dim3 grid(cdiv(p.N, BN), cdiv(p.M, BM), (unsigned)(nbatch * p.ksplit));
+    if (p.K2 == 0) p.K2 = p.K;
+    if (p.N2 == 0) p.N2 = p.N;
+    const int mblocks = (int)cdiv(p.M, BM);
+    p.mstep = 8 * (int)cdiv(cdiv(p.M, 8), mblocks);
+    dim3 grid(cdiv(p.N, BN), mblocks, (unsigned)(nbatch * p.ksplit));
     if (grid.y > 65535u || grid.z > 65535u) return fail(DFTB_ERR_BAD_SIZE, "gemm: grid too large");
+    const bool ak = p.sak == 1, bn = p.sbn == 1;
+    if (p.K2 != p.K && !ak) return fail(DFTB_ERR_BAD_SIZE, "gemm: two-level k");
     if (epi == EPI_STORE)
-        dgemm_kernel<EPI_STORE><<<grid, 256, 0, st>>>(p);
-    else
-        dgemm_kernel<EPI_ATOMIC><<<grid, 256, 0, st>>>(p);
-    return check_launch("dgemm_kernel");
+        return ak ? (bn ? launch_gemm_as<EPI_STORE, true, true>(p, grid, st)
+                        : launch_gemm_as<EPI_STORE, true, false>(p, grid, st))
+                  : (bn ? launch_gemm_as<EPI_STORE, false, true>(p, grid, st)
+                        : launch_gemm_as<EPI_STORE, false, false>(p, grid, st));
+    return ak ? (bn ? launch_gemm_as<EPI_ATOMIC, true, true>(p, grid, st)
+                    : launch_gemm_as<EPI_ATOMIC, true, false>(p, grid, st))
+              : (bn ? launch_gemm_as<EPI_ATOMIC, false, true>(p, grid, st)
+                    : launch_gemm_as<EPI_ATOMIC, false, false>(p, grid, st));
+}
+
+// K ranges so that about two CTAs per SM are in flight, at least four stages each (C40H42's 32 tiles of K = 8282: two
+// CTAs 76 us, four 80 us a product; C20H22's five tiles of K = 2142: four stages 9 us, sixteen 21 us)
+int pick_ksplit(int M, int N, int K) {
+    const long long tiles = (long long)cdiv(M, BM) * cdiv(N, BN);
+    const long long want = (148LL * 2) / tiles, most = K / (4 * BK);
+    return (int)(want < 1 || most < 1 ? 1 : (want < most ? want : most));
 }
 
 // ----------------------------------------------------------------------------
@@ -807,14 +884,17 @@ int coulomb_product(int nat, int nov, int nvec, const double *gamma, const doubl
 
 // Exchange terms in the transition-charge form, accumulated into us:
 //   us += sK1 * K1 v + sK2 * K2 v
+// Each term is a batched product per atom, laid out so that the sum over atoms and one orbital index is then a single
+// product of that length with whole (orbital, vector) rows (a product per atom and vector, added into us with atomics,
+// ran at 7 TFLOP/s).  B200, C40H42 (82 atoms, 101 x 101 orbitals), 10 vectors, (A+B).V and (A-B).V: 1820 -> 840 us.
 int exchange_products(int nat, int nocc, int nvirt, int nvec, const double *g_lr, const double *q_oo,
                       const double *q_ov, const double *q_vv, const double *vs, double *us, double sK1, double sK2,
                       double *work, cudaStream_t st) {
     const long long no = nocc, nv = nvirt, m = nvec;
     int rc;
-    // ---- K1: us[i][a][c] += sK1 * sum_B sum_b (sum_j Z[B][i][j] v[j][b][c]) q_vv[B][a][b],
-    //          Z[B][i][j] = sum_A g_lr[A][B] q_oo[A][i][j]
-    double *Z = work, *T = work + nat * no * no;
+    // ---- K1: us(i; a,c) += sK1 sum_{B,j} Z[B](i,j) Y[B][j](a,c),
+    //          Z[B](i,j) = sum_A g_lr[A][B] q_oo[A](i,j),  Y[B][j](a,c) = sum_b q_vv[B](a,b) v(j,b,c)
+    double *Z = work, *Y = work + nat * no * no;
     GemmP p = gemm_defaults();
     p.M = nat;
     p.N = (int)(no * no);
@@ -830,45 +910,44 @@ int exchange_products(int nat, int nocc, int nvirt, int nvec, const double *g_lr
     p.scn = 1;
     if ((rc = launch_gemm(p, EPI_STORE, 1, st))) return rc;
     p = gemm_defaults();
-    p.M = (int)no;
-    p.N = (int)(nv * m);
-    p.K = (int)no;
-    p.A = Z;
-    p.sam = no;
+    p.M = (int)nv;  // a
+    p.N = (int)(no * m);  // (j, c)
+    p.N2 = (int)m;
+    p.K = (int)nv;  // b
+    p.A = q_vv;
+    p.sam = nv;
     p.sak = 1;
-    p.sa1 = no * no;
+    p.sa1 = nv * nv;
     p.B = vs;
-    p.sbk = nv * m;
+    p.sbk = m;
+    p.sbn1 = nv * m;
     p.sbn = 1;
-    p.C = T;
-    p.scm = nv * m;
+    p.C = Y;
+    p.scm = m;
+    p.scn1 = nv * m;
     p.scn = 1;
     p.sc1 = no * nv * m;
     if ((rc = launch_gemm(p, EPI_STORE, nat, st))) return rc;
     p = gemm_defaults();
-    p.M = (int)no;
-    p.N = (int)nv;
-    p.K = (int)nv;
-    p.A = T;  // (i, b) of batch (B, c): T[B][i][b][c]
-    p.sam = nv * m;
-    p.sak = m;
-    p.sa1 = no * nv * m;
-    p.sa2 = 1;
-    p.B = q_vv;  // (b, a) = q_vv[B][a][b]
-    p.sbk = 1;
-    p.sbn = nv;
-    p.sb1 = nv * nv;
-    p.sb2 = 0;
-    p.C = us;  // (i, a) of column c
+    p.M = (int)no;  // i
+    p.N = (int)(nv * m);  // (a, c)
+    p.K = (int)(nat * no);  // (B, j)
+    p.K2 = (int)no;
+    p.A = Z;
+    p.sam = no;
+    p.sak1 = no * no;
+    p.sak = 1;
+    p.B = Y;
+    p.sbk = nv * m;
+    p.sbn = 1;
+    p.C = us;
     p.scm = nv * m;
-    p.scn = m;
-    p.sc1 = 0;
-    p.sc2 = 1;
-    p.nb2 = (int)m;
+    p.scn = 1;
     p.alpha = sK1;
-    if ((rc = launch_gemm(p, EPI_ATOMIC, (int)(nat * m), st))) return rc;
-    // ---- K2: us[i][a][c] += sK2 * sum_A sum_b q_ov[A][i][b] W[A][a][b][c],
-    //          W[A][a][b][c] = sum_j Z2[A][j][a] v[j][b][c],  Z2 = g_lr . q_ov
+    p.ksplit = pick_ksplit(p.M, p.N, p.K);
+    if ((rc = launch_gemm(p, EPI_ATOMIC, 1, st))) return rc;
+    // ---- K2: us(i; a,c) += sK2 sum_{A,b} q_ov[A](i,b) W[A][b](a,c),
+    //          Z2[A](j,a) = sum_B g_lr[A][B] q_ov[B](j,a),  W[A][b](a,c) = sum_j Z2[A](j,a) v(j,b,c)
     double *Z2 = work, *W = work + nat * no * nv;
     p = gemm_defaults();
     p.M = nat;
@@ -885,41 +964,42 @@ int exchange_products(int nat, int nocc, int nvirt, int nvec, const double *g_lr
     p.scn = 1;
     if ((rc = launch_gemm(p, EPI_STORE, 1, st))) return rc;
     p = gemm_defaults();
-    p.M = (int)nv;
-    p.N = (int)(nv * m);
-    p.K = (int)no;
-    p.A = Z2;  // (a, j) = Z2[A][j][a]
+    p.M = (int)nv;  // a
+    p.N = (int)(nv * m);  // (b, c)
+    p.N2 = (int)m;
+    p.K = (int)no;  // j
+    p.A = Z2;
     p.sam = 1;
     p.sak = nv;
     p.sa1 = no * nv;
     p.B = vs;
     p.sbk = nv * m;
+    p.sbn1 = m;
     p.sbn = 1;
     p.C = W;
-    p.scm = nv * m;
+    p.scm = m;
+    p.scn1 = nv * m;
     p.scn = 1;
     p.sc1 = nv * nv * m;
     if ((rc = launch_gemm(p, EPI_STORE, nat, st))) return rc;
     p = gemm_defaults();
-    p.M = (int)no;
-    p.N = (int)nv;
-    p.K = (int)nv;
-    p.A = q_ov;  // (i, b) = q_ov[A][i][b]
+    p.M = (int)no;  // i
+    p.N = (int)(nv * m);  // (a, c)
+    p.K = (int)(nat * nv);  // (A, b)
+    p.K2 = (int)nv;
+    p.A = q_ov;
     p.sam = nv;
+    p.sak1 = no * nv;
     p.sak = 1;
-    p.sa1 = no * nv;
-    p.B = W;  // (b, a) = W[A][a][b][c]
-    p.sbk = m;
-    p.sbn = nv * m;
-    p.sb1 = nv * nv * m;
-    p.sb2 = 1;
+    p.B = W;
+    p.sbk = nv * m;
+    p.sbn = 1;
     p.C = us;
     p.scm = nv * m;
-    p.scn = m;
-    p.sc2 = 1;
-    p.nb2 = (int)m;
+    p.scn = 1;
     p.alpha = sK2;
-    return launch_gemm(p, EPI_ATOMIC, (int)(nat * m), st);
+    p.ksplit = pick_ksplit(p.M, p.N, p.K);
+    return launch_gemm(p, EPI_ATOMIC, 1, st);
 }
 
 int check_products(int nat, int nocc, int nvirt, int nvec, int lc, const double *g, const double *g_lr,
