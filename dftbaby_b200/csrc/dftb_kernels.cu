@@ -41,84 +41,235 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 #include "sk_device.cuh"
 #include "coulomb.cuh"
 
-// One thread per matrix element (mu, nu); the value is the reference's
-// lower-triangle element for (max, min), so both triangles are written
-// directly and coalesced.  slako.f90:77-231.
-__global__ void h0_and_s_kernel(int norb, int nat, OrbTables O, const double *r, const double *x, const double *y,
-                                const double *z, const int *mprox, const double *orben, SkTables TS, SkTables TH,
-                                double *S, double *H0) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = blockIdx.y;
-    if (col >= norb || row >= norb) return;
-    const int mu = row > col ? row : col, nu = row > col ? col : row;
-    const size_t o = (size_t)row * norb + col;
-    const int i = O.ind[mu], j = O.ind[nu];
-    double s = 0.0, h = 0.0;
-    if (mprox[(size_t)i * nat + j] != 0) {
-        if (mu == nu) {
-            s = 1.0;
-            h = orben[mu];
-        } else if (i != j) {
-            const int l1 = O.ls[mu], m1 = O.ms[mu], l2 = O.ls[nu], m2 = O.ms[nu];
-            if (l1 > 1 || l2 > 1) {
-                s = h = __longlong_as_double(0x7ff8000000000000ULL);
-            } else {
-                const int typi = O.typ[mu], typj = O.typ[nu];
-                const int tmin = min(typi, typj), tmax = max(typi, typj);
-                const int ipair = tmax * (tmax + 1) / 2 + tmin;
-                double rij, e[3];
-                pair_dir(nat, r, x, y, z, i, j, rij, e);
-                if (typi <= typj) {
-                    s = sk_rule(TS, ipair, rij, e, l1, m1, l2, m2);
-                    h = sk_rule(TH, ipair, rij, e, l1, m1, l2, m2);
-                } else {
-                    const double me[3] = {-e[0], -e[1], -e[2]};
-                    s = sk_rule(TS, ipair, rij, me, l2, m2, l1, m1);
-                    h = sk_rule(TH, ipair, rij, me, l2, m2, l1, m1);
-                }
-            }
-        }
-    }
-    S[o] = s;
-    H0[o] = h;
+// ----------------------------------------------------------------------------
+// S, H0 and dipoles (slako.f90:77-394).  A block takes the orbitals of 8 row atoms x 32 column atoms.  Its 256 threads
+// first evaluate the splines of one atom pair each (an element's own evaluation took up to four splines, 50 per
+// carbon pair, with six divisions each), then write the elements from them, a warp along each row.  The value is the
+// reference's lower-triangle element for (max, min), so both triangles are written directly.  Four blocks per SM: the
+// phases are short chains of loads between barriers, and 64 registers with a few spills (125 us, below) beat 80 without
+// (136 us).  B200, C1014H90 (4146 orbitals): S and H0 846 -> 125 us (275 MB written, 42 us), D 879 -> 167 us (412 MB);
+// C20H22: 19 -> 15 us each.
+// ----------------------------------------------------------------------------
+constexpr int SK_TA = 8, SK_TB = 32, SK_PAIRS = SK_TA * SK_TB;
+constexpr int SK_ROWS = 64, SK_COLS = 160;  // orbitals of a tile with their (atom, l, axis) in shared memory
+
+struct SkTile {
+    int first[SK_TA + SK_TB + 2];  // orbital ranges of the row atoms (0 .. SK_TA) and of the column atoms (SK_TA + 1 ..)
+    int rinfo[SK_ROWS], cinfo[SK_COLS];
+    unsigned present, mask[SK_SHARED_PAIRS];
+    unsigned char flags[SK_PAIRS];  // 1: proximate, 2: read as (later atom, earlier atom)
+};
+
+// an atom pair: r and the direction from the first to the second centre in the order in which its tables are read
+struct SkPair {
+    double r, e[3];
+    int i, j, ipair;
+    bool near;
+};
+
+__device__ __forceinline__ int orb_info(const OrbTables &O, int mu, int atom0) {
+    return (O.ind[mu] - atom0) | O.ls[mu] << 8 | axis_of_m(O.ms[mu]) << 16;
 }
 
-// slako.f90:238-394; D planes (3, norb, norb).
-__global__ void dipole_kernel(int norb, int nat, OrbTables O, const double *r, const double *x, const double *y,
-                              const double *z, const double *pos, const int *mprox, const double *Smat,
-                              SkTables TD, double *D) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = blockIdx.y;
-    if (col >= norb || row >= norb) return;
-    const int mu = row > col ? row : col, nu = row > col ? col : row;
-    const size_t o = (size_t)row * norb + col, plane = (size_t)norb * norb;
-    const int i = O.ind[mu], j = O.ind[nu];
-    double d[3] = {0.0, 0.0, 0.0};
-    if (mprox[(size_t)i * nat + j] != 0) {
-        const int l1 = O.ls[mu], m1 = O.ms[mu], l2 = O.ls[nu], m2 = O.ms[nu];
-        if (l1 > 1 || l2 > 1) {
-            d[0] = d[1] = d[2] = __longlong_as_double(0x7ff8000000000000ULL);
-        } else {
-            const int typi = O.typ[mu], typj = O.typ[nu];
-            const int tmin = min(typi, typj), tmax = max(typi, typj);
-            const int ipair = tmax * (tmax + 1) / 2 + tmin;
-            double rij, e[3];
-            pair_dir(nat, r, x, y, z, i, j, rij, e);
-            const double s = Smat[(size_t)mu * norb + nu];
-            if (typi <= typj) {
-                sk_dipole_rule(TD, ipair, rij, e, l1, m1, l2, m2, d);
+// ranges, orbital tables, the thread's atom pair and the type pairs of the tile
+__device__ __forceinline__ SkPair sk_tile_setup(SkTile &t, const OrbTables &O, int norb, int nat, const double *r,
+                                                const double *x, const double *y, const double *z, const int *mprox,
+                                                int A0, int B0) {
+    const int tid = threadIdx.x;
+    if (tid <= SK_TA) t.first[tid] = first_orbital(O.ind, norb, min(nat, A0 + tid));
+    else if (tid <= SK_TA + 1 + SK_TB) t.first[tid] = first_orbital(O.ind, norb, min(nat, B0 + tid - SK_TA - 1));
+    else if (tid < 64) {
+        if (tid == 48) t.present = 0u;
+        if (tid > 48 && tid <= 48 + SK_SHARED_PAIRS) t.mask[tid - 49] = 0u;
+    }
+    const int ia = tid / SK_TB, ib = tid % SK_TB, A = A0 + ia, B = B0 + ib;
+    const bool in = A < nat && B < nat;
+    SkPair p;
+    p.i = max(A, B);
+    p.j = min(A, B);
+    p.r = p.e[0] = p.e[1] = p.e[2] = 0.0;
+    p.near = in && mprox[(size_t)p.i * nat + p.j] != 0;
+    if (in) pair_dir(nat, r, x, y, z, p.i, p.j, p.r, p.e);
+    __syncthreads();
+    const int row0 = t.first[0], row1 = t.first[SK_TA], col0 = t.first[SK_TA + 1], col1 = t.first[SK_TA + 1 + SK_TB];
+    if (tid < SK_ROWS && row0 + tid < row1) t.rinfo[tid] = orb_info(O, row0 + tid, A0);
+    const int c = tid - (SK_PAIRS - SK_COLS);
+    if (c >= 0 && col0 + c < col1) t.cinfo[c] = orb_info(O, col0 + c, B0);
+    const int fa = t.first[ia], fb = t.first[SK_TA + 1 + ib];
+    bool straight = true;
+    p.ipair = 0;
+    p.near = p.near && fa < t.first[ia + 1] && fb < t.first[SK_TA + 2 + ib];
+    if (p.near) {
+        const int ta = O.typ[fa], tb = O.typ[fb], tmin = min(ta, tb), tmax = max(ta, tb);
+        p.ipair = tmax * (tmax + 1) / 2 + tmin;
+        straight = A >= B ? ta <= tb : tb <= ta;  // type of the later atom <= type of the earlier one
+        if (!straight)
+            for (int k = 0; k < 3; ++k) p.e[k] = -p.e[k];
+    }
+    t.flags[tid] = (p.near ? 1 : 0) | (straight ? 2 : 0);
+    const unsigned here = __reduce_or_sync(0xffffffffu, p.near && p.ipair < SK_SHARED_PAIRS ? 1u << p.ipair : 0u);
+    if ((tid & 31) == 0 && here) atomicOr(&t.present, here);
+    __syncthreads();
+    return p;
+}
+
+// filled and shared bits of a pair's tables; pairs beyond SK_SHARED_PAIRS look their own tables up
+template <int NT>
+__device__ __forceinline__ unsigned sk_pair_mask(const SkTile &t, const SkTables &TA, const SkTables *TB, int ipair,
+                                                 const int (&tabs)[NT]) {
+    if (ipair < SK_SHARED_PAIRS) return t.mask[ipair];
+    unsigned m = 0;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) d[c] += pos[3 * j + c] * s;
-            } else {
-                const double me[3] = {-e[0], -e[1], -e[2]};
-                sk_dipole_rule(TD, ipair, rij, me, l2, m2, l1, m1, d);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) d[c] += pos[3 * i + c] * s;
+    for (int q = 0; q < NT; ++q) {
+        if (tabs[q] < TA.nsk && TA.filled[ipair * TA.nsk + tabs[q]] == 1) m |= 1u << q;
+        if (TB && tabs[q] < TB->nsk && TB->filled[ipair * TB->nsk + tabs[q]] == 1) m |= 1u << (NT + q);
+    }
+    return m;
+}
+
+__global__ void __launch_bounds__(SK_PAIRS, 4) h0_and_s_kernel(int norb, int nat, OrbTables O, const double *r,
+                                                               const double *x, const double *y, const double *z,
+                                                               const int *mprox, const double *orben, SkTables TS,
+                                                               SkTables TH, double *S, double *H0) {
+    constexpr int tabs[5] = {0, 2, 4, 5, 6};  // ss, sp, ps, pp-pi, pp-sigma
+    __shared__ double vals[13][SK_PAIRS];     // S tables, H tables, direction
+    __shared__ SkTile t;
+    const int A0 = blockIdx.y * SK_TA, B0 = blockIdx.x * SK_TB, tid = threadIdx.x;
+    {
+        const SkPair p = sk_tile_setup(t, O, norb, nat, r, x, y, z, mprox, A0, B0);
+        sk_shared_tables(TS, &TH, tabs, t.present, t.mask);
+        __syncthreads();
+        if (p.near && p.i != p.j) {
+            const unsigned m = sk_pair_mask(t, TS, &TH, p.ipair, tabs);
+            SkBasis b = {};
+            if (m >> 16)
+                b = sk_basis(TS.knots + ((size_t)p.ipair * TS.nsk + sk_first_filled(TS, p.ipair, tabs)) * TS.npts,
+                             TS.npts, p.r);
+            sk_values(TS, p.ipair, tabs, p.r, b, m & 31u, m >> 16 & 31u, &vals[0][tid], SK_PAIRS);
+            sk_values(TH, p.ipair, tabs, p.r, b, m >> 5 & 31u, m >> 21 & 31u, &vals[5][tid], SK_PAIRS);
+        }
+        for (int c = 0; c < 3; ++c) vals[10 + c][tid] = p.e[c];
+    }
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31;
+    const int row0 = t.first[0], row1 = t.first[SK_TA], col0 = t.first[SK_TA + 1], col1 = t.first[SK_TA + 1 + SK_TB];
+    const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+    for (int col = col0 + lane; col < col1; col += 32) {
+        const int ci = col - col0 < SK_COLS ? t.cinfo[col - col0] : orb_info(O, col, B0);
+        const int ib = ci & 255, lc = ci >> 8 & 255, ac = ci >> 16;
+        for (int row = row0 + warp; row < row1; row += SK_PAIRS / 32) {
+            const int ri = row - row0 < SK_ROWS ? t.rinfo[row - row0] : orb_info(O, row, A0);
+            const int ia = ri & 255, lr = ri >> 8 & 255, ar = ri >> 16;
+            const int q = ia * SK_TB + ib, f = t.flags[q];
+            const double *v = &vals[0][q];
+            double s = 0.0, h = 0.0;
+            if (A0 + ia == B0 + ib) {
+                if (row == col && (f & 1)) {
+                    s = 1.0;
+                    h = orben[row];
+                }
+            } else if (f & 1) {
+                const bool rf = (row > col) == ((f & 2) != 0);  // the row's orbital is the first one
+                const double ang = (lr ? v[(10 + ar) * SK_PAIRS] : 1.0) * (lc ? v[(10 + ac) * SK_PAIRS] : 1.0);
+                const int k = lr + lc < 2 ? (lr == lc ? 0 : ((lr == 1) == rf ? 2 : 1)) : 4;  // ss, ps, sp, pp-sigma
+                s = v[k * SK_PAIRS];
+                h = v[(5 + k) * SK_PAIRS];
+                if (k == 4) {
+                    const double spi = v[3 * SK_PAIRS], hpi = v[8 * SK_PAIRS], on = ar == ac ? 1.0 : 0.0;
+                    s = on * spi + ang * (s - spi);
+                    h = on * hpi + ang * (h - hpi);
+                } else {
+                    s *= ang;
+                    h *= ang;
+                }
+                if (max(lr, lc) > 1) s = h = nan;
             }
+            const size_t o = (size_t)row * norb + col;
+            S[o] = s;
+            H0[o] = h;
         }
     }
+}
+
+// D planes (3, norb, norb)
+__global__ void __launch_bounds__(SK_PAIRS, 4) dipole_kernel(int norb, int nat, OrbTables O, const double *r,
+                                                             const double *x, const double *y, const double *z,
+                                                             const double *pos, const int *mprox, const double *Smat,
+                                                             SkTables TD, double *D) {
+    constexpr int tabs[8] = {3, 1, 4, 6, 13, 7, 8, 14};  // ss; sp pi, sigma; ps pi, sigma; pp
+    __shared__ double vals[11][SK_PAIRS];                 // tables, direction
+    __shared__ double centre[SK_TA + SK_TB][3];
+    __shared__ SkTile t;
+    const int A0 = blockIdx.y * SK_TA, B0 = blockIdx.x * SK_TB, tid = threadIdx.x;
+    if (tid < 3 * (SK_TA + SK_TB)) {
+        const int k = tid / 3, atom = k < SK_TA ? A0 + k : B0 + k - SK_TA;
+        centre[k][tid % 3] = atom < nat ? pos[3 * atom + tid % 3] : 0.0;
+    }
+    {
+        const SkPair p = sk_tile_setup(t, O, norb, nat, r, x, y, z, mprox, A0, B0);
+        sk_shared_tables(TD, nullptr, tabs, t.present, t.mask);
+        __syncthreads();
+        if (p.near) {
+            const unsigned m = sk_pair_mask(t, TD, nullptr, p.ipair, tabs);
+            SkBasis b = {};
+            if (m >> 16)
+                b = sk_basis(TD.knots + ((size_t)p.ipair * TD.nsk + sk_first_filled(TD, p.ipair, tabs)) * TD.npts,
+                             TD.npts, p.r);
+            sk_values(TD, p.ipair, tabs, p.r, b, m & 255u, m >> 16 & 255u, &vals[0][tid], SK_PAIRS);
+        }
+        for (int c = 0; c < 3; ++c) vals[8 + c][tid] = p.e[c];
+    }
+    __syncthreads();
+    const size_t plane = (size_t)norb * norb;
+    const int warp = tid >> 5, lane = tid & 31;
+    const int row0 = t.first[0], row1 = t.first[SK_TA], col0 = t.first[SK_TA + 1], col1 = t.first[SK_TA + 1 + SK_TB];
+    for (int col = col0 + lane; col < col1; col += 32) {
+        const int ci = col - col0 < SK_COLS ? t.cinfo[col - col0] : orb_info(O, col, B0);
+        const int ib = ci & 255, lc = ci >> 8 & 255, ac = ci >> 16;
+        for (int row = row0 + warp; row < row1; row += SK_PAIRS / 32) {
+            const int ri = row - row0 < SK_ROWS ? t.rinfo[row - row0] : orb_info(O, row, A0);
+            const int ia = ri & 255, lr = ri >> 8 & 255, ar = ri >> 16;
+            const int q = ia * SK_TB + ib, f = t.flags[q];
+            const double *v = &vals[0][q];
+            double d[3] = {0.0, 0.0, 0.0};
+            if (f & 1) {
+                const bool lower = row >= col, st = (f & 2) != 0, rf = lower == st;
+                const double s = Smat[lower ? (size_t)row * norb + col : (size_t)col * norb + row];
+                // the second centre: the earlier atom where straight
+                const double *o = centre[st == (A0 + ia >= B0 + ib) ? SK_TA + ib : ia];
+                const int a1 = rf ? ar : ac, a2 = rf ? ac : ar;
+                if (max(lr, lc) > 1) {
+                    d[0] = d[1] = d[2] = __longlong_as_double(0x7ff8000000000000ULL);
+                } else if (lr + lc == 0) {
+                    const double d3 = v[0];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) D[c * plane + o] = d[c];
+                    for (int c = 0; c < 3; ++c) d[c] = v[(8 + c) * SK_PAIRS] * d3;
+                } else if (lr + lc == 1) {
+                    const int b = lr == 1 ? ar : ac, tb = (lr == 1) == rf ? 3 : 1;  // ps or sp
+                    const double dpi = v[tb * SK_PAIRS], w = v[(8 + b) * SK_PAIRS] * (v[(tb + 1) * SK_PAIRS] - dpi);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) d[c] = (c == b ? dpi : 0.0) + v[(8 + c) * SK_PAIRS] * w;
+                } else {
+                    const double d7 = v[5 * SK_PAIRS], d8 = v[6 * SK_PAIRS], cub = v[7 * SK_PAIRS] - d7 - 2.0 * d8;
+                    const double ea = v[(8 + a1) * SK_PAIRS], eb = v[(8 + a2) * SK_PAIRS], w = ea * eb * cub;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const double ec = v[(8 + c) * SK_PAIRS];
+                        double u = ec * w;
+                        if (a1 == c) u += eb * d7;
+                        if (c == a2) u += ea * d8;
+                        if (a1 == a2) u += ec * d8;
+                        d[c] = u;
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) d[c] += o[c] * s;
+            }
+            const size_t out = (size_t)row * norb + col;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) D[c * plane + out] = d[c];
+        }
+    }
 }
 
 __global__ void dircos_kernel(int nat, const double *pos, double *r, double *x, double *y, double *z) {
@@ -162,11 +313,17 @@ __global__ void gamma_kernel(int nat, const double *r, const double *sigma, doub
     }
 }
 
+// rows per thread of the element-wise (norb, norb) kernels: enough loads and stores in flight to reach HBM speed
+constexpr int AO_ROWS = 8;
+
 __global__ void ao_expand_kernel(int norb, int nat, const int *ind, const double *g, double *G) {
     const int nu = blockIdx.x * blockDim.x + threadIdx.x;
-    const int mu = blockIdx.y;
-    if (nu >= norb || mu >= norb) return;
-    G[(size_t)mu * norb + nu] = g[(size_t)ind[mu] * nat + ind[nu]];
+    if (nu >= norb) return;
+    const double *col = g + ind[nu];
+    const int mu0 = blockIdx.y * AO_ROWS, mu1 = min(norb, mu0 + AO_ROWS);
+#pragma unroll
+    for (int mu = mu0; mu < mu0 + AO_ROWS; ++mu)
+        if (mu < mu1) G[(size_t)mu * norb + nu] = col[(size_t)ind[mu] * nat];
 }
 
 // estat[A] = sum_B gamma[A][B] dq[B]; one warp per atom
@@ -184,11 +341,16 @@ __global__ void estat_kernel(int nat, const double *gamma, const double *dq, dou
 __global__ void scc_h_kernel(int norb, const int *ind, const double *H0, const double *Smat, const double *estat,
                              double *H) {
     const int nu = blockIdx.x * blockDim.x + threadIdx.x;
-    const int mu = blockIdx.y;
-    if (nu >= norb || mu >= norb) return;
-    const size_t o = (size_t)mu * norb + nu;
-    const double h1 = 0.5 * (estat[ind[mu]] + estat[ind[nu]]);
-    H[o] = H0[o] + h1 * Smat[o];
+    if (nu >= norb) return;
+    const double en = estat[ind[nu]];
+    const int mu0 = blockIdx.y * AO_ROWS, mu1 = min(norb, mu0 + AO_ROWS);
+#pragma unroll
+    for (int mu = mu0; mu < mu0 + AO_ROWS; ++mu)
+        if (mu < mu1) {
+            const size_t o = (size_t)mu * norb + nu;
+            const double h1 = 0.5 * (estat[ind[mu]] + en);
+            H[o] = H0[o] + h1 * Smat[o];
+        }
 }
 
 // Mulliken monopoles: one block per atom, reduction over its rows.
@@ -1090,8 +1252,9 @@ int dftb_h0_and_s(int norb, int nat, const int *ind, const int *typ, const int *
     OrbTables O{ind, typ, ls, ms};
     SkTables TS{tab_filled, S_knots, S_coefs, nsk, npts};
     SkTables TH{tab_filled, H_knots, H_coefs, nsk, npts};
-    dim3 grid(cdiv(norb, 128), norb);
-    h0_and_s_kernel<<<grid, 128, 0, S(stream)>>>(norb, nat, O, r, x, y, z, mprox, orben, TS, TH, Sm, H0);
+    dim3 grid(cdiv(nat, SK_TB), cdiv(nat, SK_TA));
+    if (grid.y > 65535u) return fail(DFTB_ERR_BAD_SIZE, "h0_and_s: more than 524280 atoms");
+    h0_and_s_kernel<<<grid, SK_PAIRS, 0, S(stream)>>>(norb, nat, O, r, x, y, z, mprox, orben, TS, TH, Sm, H0);
     return check_launch("h0_and_s_kernel");
 }
 
@@ -1107,8 +1270,9 @@ int dftb_dipole_matrix(int norb, int nat, const int *ind, const int *typ, const 
         return fail(DFTB_ERR_NULL, "dipole_matrix: null");
     OrbTables O{ind, typ, ls, ms};
     SkTables TD{tab_filled_D, D_knots, D_coefs, nskd, npts};
-    dim3 grid(cdiv(norb, 128), norb);
-    dipole_kernel<<<grid, 128, 0, S(stream)>>>(norb, nat, O, r, x, y, z, pos, mprox, Sm, TD, D);
+    dim3 grid(cdiv(nat, SK_TB), cdiv(nat, SK_TA));
+    if (grid.y > 65535u) return fail(DFTB_ERR_BAD_SIZE, "dipole_matrix: more than 524280 atoms");
+    dipole_kernel<<<grid, SK_PAIRS, 0, S(stream)>>>(norb, nat, O, r, x, y, z, pos, mprox, Sm, TD, D);
     return check_launch("dipole_kernel");
 }
 
@@ -1124,7 +1288,7 @@ int dftb_gamma_matrices(int nat, const double *r, const double *sigma, double r_
 int dftb_ao_expand(int norb, int nat, const int *ind, const double *g, double *G, void *stream) {
     if (norb <= 0 || nat <= 0) return fail(DFTB_ERR_BAD_SIZE, "ao_expand: sizes");
     if (!ind || !g || !G) return fail(DFTB_ERR_NULL, "ao_expand: null");
-    dim3 grid(cdiv(norb, 128), norb);
+    dim3 grid(cdiv(norb, 128), cdiv(norb, AO_ROWS));
     ao_expand_kernel<<<grid, 128, 0, S(stream)>>>(norb, nat, ind, g, G);
     return check_launch("ao_expand_kernel");
 }
@@ -1136,7 +1300,7 @@ int dftb_scc_hamiltonian(int norb, int nat, const int *ind, const double *H0, co
     estat_kernel<<<cdiv(nat, 8), 256, 0, S(stream)>>>(nat, gamma, dq, estat);
     int rc = check_launch("estat_kernel");
     if (rc) return rc;
-    dim3 grid(cdiv(norb, 128), norb);
+    dim3 grid(cdiv(norb, 128), cdiv(norb, AO_ROWS));
     scc_h_kernel<<<grid, 128, 0, S(stream)>>>(norb, ind, H0, Sm, estat, H);
     return check_launch("scc_h_kernel");
 }

@@ -159,16 +159,6 @@ __device__ void pair_sk_gradient(int nat, const OrbTables &O, const double *r, c
     }
 }
 
-// First orbital of atom j in the sorted, contiguous orbital -> atom table.
-__device__ __forceinline__ int first_orbital(const int *ind, int norb, int j) {
-    int lo = 0, hi = norb;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (ind[mid] < j) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -127,3 +127,124 @@ __device__ __forceinline__ void pair_dir(int nat, const double *r, const double 
     e[2] = z[o];
 }
 
+// First orbital of atom j in the sorted, contiguous orbital -> atom table.
+__device__ __forceinline__ int first_orbital(const int *ind, int norb, int j) {
+    int lo = 0, hi = norb;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ind[mid] < j) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// ----------------------------------------------------------------------------
+// Tables of one type pair that share their knots: the B-splines of an argument are then the same for all of them and
+// are formed once (they take six divisions; a table's value from them takes four multiply-adds).  Whether they do is
+// found per block by comparing the knots themselves.
+// ----------------------------------------------------------------------------
+constexpr int SK_SHARED_PAIRS = 6;  // type pairs looked at (three elements); tables of further pairs stand alone
+
+// the B-splines on the interval of splev_uniform's rule; l is 1-based
+struct SkBasis {
+    double h[4];
+    int l;
+};
+
+__device__ __forceinline__ SkBasis sk_basis(const double *__restrict__ t, int n, double x) {
+    const int k = 3, k1 = 4, nk1 = n - k1;
+    const double tb = t[k1 - 1], te = t[nk1];
+    SkBasis b;
+    double arg;
+    if (x <= tb) {
+        arg = tb;
+        b.l = k1;
+    } else if (x >= te) {
+        arg = te;
+        b.l = nk1;
+    } else {
+        arg = x;
+        b.l = (int)((x - t[0]) / (t[k1 + 1] - t[k1])) + 1;
+    }
+    if (b.l < k) b.l = k1;
+    double hh[3];
+    b.h[0] = 1.0;
+#pragma unroll
+    for (int j = 1; j <= k; ++j) {
+#pragma unroll
+        for (int i = 1; i <= j; ++i) hh[i - 1] = b.h[i - 1];
+        b.h[0] = 0.0;
+#pragma unroll
+        for (int i = 1; i <= j; ++i) {
+            const int li = b.l + i, lj = li - j;
+            const double f = hh[i - 1] / (t[li - 1] - t[lj - 1]);
+            b.h[i - 1] = b.h[i - 1] + f * (t[li - 1] - arg);
+            b.h[i] = f * (arg - t[lj - 1]);
+        }
+    }
+    return b;
+}
+
+// (a coefficient index below 1, reachable only on interval 3, contributes zero)
+__device__ __forceinline__ double sk_dot(const SkBasis &b, const double *__restrict__ c) {
+    const double *q = c + (b.l - 4);
+    double sp = b.l > 3 ? q[0] * b.h[0] : 0.0;
+#pragma unroll
+    for (int j = 1; j < 4; ++j) sp += q[j] * b.h[j];
+    return sp;
+}
+
+// For each type pair p of `present`, by the whole block between two barriers: mask[p] gets bit q where table tabs[q] of
+// TA is filled and bit 16 + q where it also has the knots of TR's first filled table tabs[ref(p)], likewise bits
+// NT + q and 16 + NT + q for TB (unless it is NULL).  A warp takes one table at a time.
+template <int NT>
+__device__ __forceinline__ int sk_first_filled(const SkTables &T, int p, const int (&tabs)[NT]) {
+    int ref = -1;
+#pragma unroll
+    for (int q = NT - 1; q >= 0; --q)
+        if (tabs[q] < T.nsk && T.filled[p * T.nsk + tabs[q]] == 1) ref = tabs[q];
+    return ref;
+}
+
+template <int NT>
+__device__ __forceinline__ void sk_shared_tables(const SkTables &TA, const SkTables *TB, const int (&tabs)[NT],
+                                                 unsigned present, unsigned *mask) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int n = TB ? 2 * NT : NT;
+    for (int p = 0; p < SK_SHARED_PAIRS; ++p) {
+        if (!(present >> p & 1)) continue;
+        const int ref = sk_first_filled(TA, p, tabs);
+        for (int q = warp; q < n; q += nw) {
+            const SkTables T = q < NT ? TA : *TB;
+            int tab = 0;  // tabs[q % NT], without an array in local memory
+#pragma unroll
+            for (int k = 0; k < NT; ++k)
+                if (k == q || k + NT == q) tab = tabs[k];
+            if (tab >= T.nsk || T.filled[p * T.nsk + tab] != 1) continue;
+            bool same = ref >= 0;
+            if (same) {
+                const double *a = TA.knots + ((size_t)p * TA.nsk + ref) * TA.npts;
+                const double *b = T.knots + ((size_t)p * T.nsk + tab) * T.npts;
+#pragma unroll 8
+                for (int i = lane; i < T.npts; i += 32) same &= a[i] == b[i];
+            }
+            same = __all_sync(0xffffffffu, same);
+            if (lane == 0) atomicOr(mask + p, (1u << q) | (same ? 1u << (16 + q) : 0u));
+        }
+    }
+}
+
+// values of the tables tabs[] at r (0 where not filled) into v[q * stride]; filled and shared: bit q
+template <int NT>
+__device__ __forceinline__ void sk_values(const SkTables &T, int ipair, const int (&tabs)[NT], double r,
+                                          const SkBasis &b, unsigned filled, unsigned shared, double *v, int stride) {
+    const size_t o = (size_t)ipair * T.nsk * T.npts;
+#pragma unroll
+    for (int q = 0; q < NT; ++q) {
+        double x = 0.0;
+        if (shared >> q & 1)
+            x = sk_dot(b, T.coefs + o + tabs[q] * T.npts);
+        else if (filled >> q & 1)
+            x = sk_dot(sk_basis(T.knots + o + tabs[q] * T.npts, T.npts, r), T.coefs + o + tabs[q] * T.npts);
+        v[q * stride] = x;
+    }
+}
