@@ -89,34 +89,15 @@ __device__ __forceinline__ void store_row16(float *dst, int n, const float v[16]
     }
 }
 
-__device__ __forceinline__ void store_row16_bf16(__nv_bfloat16 *dst, int n, const __nv_bfloat16 v[16]) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(dst);
-    uint32_t w[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const __nv_bfloat162 pr = __halves2bfloat162(v[2 * q], v[2 * q + 1]);
-        w[q] = *reinterpret_cast<const uint32_t *>(&pr);
-    }
-    if (n == 16 && (a & 15) == 0) {
-        uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-        d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    } else if (n == 16 && (a & 3) == 0) {
-        uint32_t *d = reinterpret_cast<uint32_t *>(dst);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) d[q] = w[q];
-    } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (j < n) dst[j] = v[j];
-    }
-}
-
-// Transposed-output staging: per epilogue warp a [32 tile columns][32 tile rows] BF16 block for hi
-// and for lo, rows padded to 40 elements (80 B, a multiple of 16 B for the 16-byte reads).
-constexpr int EPI_THREADS = 128;
+// Eight epilogue warps, two per TMEM lane quarter with every other 32-column chunk each: the epilogues with a Hadamard
+// factor or a transposed output are instruction-bound, and with four warps they outlasted the next tile's MMAs (a dense
+// layer of 65536 x 256: 50 us with four warps, 32 us with eight).
+constexpr int EPI_WARPS = 8, EPI_THREADS = 32 * EPI_WARPS, THREADS = 64 + EPI_THREADS;
+// BF16 output staging: per epilogue warp a 32 x 32 block (row-major or transposed, hi, then lo), rows padded to 40
+// elements (80 B, a multiple of 16 B for the 16-byte reads), so that a store instruction writes eight whole 64-byte
+// pieces instead of 16 bytes of 32 rows (the exchange's W 83 -> 77 us, N 556 -> 522 us).
 constexpr int TPITCH = 40;
-constexpr int TSTAGE_BYTES = 4 * 2 * 32 * TPITCH * 2;
+constexpr int TSTAGE_BYTES = EPI_WARPS * 32 * TPITCH * 2;
 
 template <bool SPLIT, bool WIDE = false> struct Cfg {
     // 128 x 128 output tiles with 64-element K blocks (128-byte swizzle); WIDE (split mode only): 128 x 256
@@ -153,7 +134,29 @@ struct Params {
     __nv_bfloat16 *Thi, *Tlo;  // transposed hi/lo output: T(n, m) (ld = ldt)
     long long ldt;
     int *err;  // device error word (0 = ok)
+    // dense layer (MLP): relu(v + bias) or v o (mask > 0), rounded to Ohi and Thi; colsum += column sums of the
+    // unrounded values
+    const float *bias;
+    const __nv_bfloat16 *mask;
+    long long ldm;
+    float *colsum;
 };
+
+// Sums over the warp's 32 lanes of 32 values per lane: lane q returns the sum of every lane's v[q] (halving the values
+// with each exchange: 31 shuffles, where 32 separate reductions take 160).
+__device__ __forceinline__ float warp_column_sums(float v[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+        const bool up = (lane & half) != 0;
+#pragma unroll
+        for (int q = 0; q < half; ++q) {
+            const float send = up ? v[q] : v[q + half], keep = up ? v[q + half] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+        }
+    }
+    return v[0];
+}
 
 // UMMA shared-memory descriptor for K-major rows of 64 B with 64-byte swizzle: 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t smem_desc_k64(uint32_t saddr) {
@@ -224,12 +227,15 @@ __device__ __forceinline__ TileCoords tile_coords(int t, int mt, int nt, int bnx
 //   warp 0 lane 0 : TMA producer over the operand ring (continues across tiles);
 //   warp 1 lane 0 : tcgen05.mma issuer into one of two 128-column TMEM accumulators
 //                   (tile j uses accumulator j % 2);
-//   warps 2..5    : epilogue of tile j while the MMAs of tile j + 1 run; warp w reads TMEM
-//                   lanes 32 (w % 4) .. 32 (w % 4) + 31.
+//   warps 2..9    : epilogue of tile j while the MMAs of tile j + 1 run; warp w reads TMEM
+//                   lanes 32 (w % 4) .. 32 (w % 4) + 31, every other 32-column chunk.
 // Barriers: full/empty per ring slot, tfull (MMA -> epilogue, tcgen05.commit) and tempty
-// (epilogue -> MMA, 128 arrivals) per accumulator.  Every wait is bounded.
-template <bool SPLIT, bool WIDE>
-__global__ void __launch_bounds__(192, 1) gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
+// (epilogue -> MMA, 256 arrivals) per accumulator.  Every wait is bounded.
+// MLP (segment mode): the epilogue of a dense layer of the pair-scoring network, forward (bias and ReLU) or backward
+// (ReLU mask and bias gradient), instead of an FP32 result that another kernel would read again.  B200, 65536 samples x
+// 256 units: product and bias_relu 32 + 46 us, product and relu_backward 32 + 80 us; here 25 to 40 us.
+template <bool SPLIT, bool WIDE, bool MLP = false>
+__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
     using C = Cfg<SPLIT, WIDE>;
     constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES;
     constexpr int BNX = C::BNX, TILE_BX = C::TILE_BX, TILE_AX = C::TILE_AX, BKX = C::BKX;
@@ -372,12 +378,50 @@ __global__ void __launch_bounds__(192, 1) gemm_kernel(const __grid_constant__ Ma
             }
         }
     } else {
-        // ---------------- epilogue (warps 2..5, 128 threads)
+        // ---------------- epilogue (warps 2..9, 256 threads)
         const int rq = warp & 3;  // TMEM lane quarter this warp may access
         const int rloc = rq * 32 + lane;
-        const bool stage_t = p.Thi != nullptr && p.ksplit == 1;
-        __nv_bfloat16 *sh = tstage + (warp - 2) * (2 * 32 * TPITCH);
-        __nv_bfloat16 *sl = sh + 32 * TPITCH;
+        const int chunk0 = 32 * ((warp - 2) >> 2);  // this warp's chunks start here, 64 columns apart
+        __nv_bfloat16 *sh = tstage + (warp - 2) * (32 * TPITCH);
+        // writes the staged 32 x 32 block to D rows r0 .., columns c0 .. (inside rows x cols)
+        auto write_block = [&](__nv_bfloat16 *D, long long ld, int r0, int c0, int rows, int cols) {
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int rl = q * 8 + (lane >> 2), part = lane & 3;
+                const int r = r0 + rl, c = c0 + part * 8, nv = min(8, cols - c);
+                if (r < rows && nv > 0) {
+                    const __nv_bfloat16 *src = sh + rl * TPITCH + part * 8;
+                    __nv_bfloat16 *dst = D + (long long)r * ld + c;
+                    if (nv == 8 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0)
+                        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(src);
+                    else
+                        for (int e = 0; e < nv; ++e) dst[e] = src[e];
+                }
+            }
+            __syncwarp();
+        };
+        // this warp's block of BF16 values (a row per lane) to the row-major output O and the transposed one T
+        auto write_bf16 = [&](const __nv_bfloat16 *x, __nv_bfloat16 *O, __nv_bfloat16 *T, int row0, int col0) {
+            if (O) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const __nv_bfloat162 pr = __halves2bfloat162(x[8 * q + 2 * e], x[8 * q + 2 * e + 1]);
+                        w[e] = *reinterpret_cast<const uint32_t *>(&pr);
+                    }
+                    *reinterpret_cast<uint4 *>(sh + lane * TPITCH + 8 * q) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+                write_block(O, p.ldo, row0, col0, p.M, p.N);
+            }
+            if (T) {
+#pragma unroll
+                for (int q = 0; q < 32; ++q) sh[q * TPITCH + lane] = x[q];
+                write_block(T, p.ldt, col0, row0, p.N, p.M);
+            }
+        };
         int j = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++j) {
             const TileCoords tc = tile_coords(t, mt, nt, BNX, kblocks_all, kper);
@@ -389,22 +433,73 @@ __global__ void __launch_bounds__(192, 1) gemm_kernel(const __grid_constant__ Ma
                 // pull this tile's G row into L2 while its MMAs run (128-byte lines, inside the matrix)
                 const float *g = p.G + (long long)row * p.ldg + n0;
                 const int ncols = min(BNX, p.N - n0);
-                for (int c = 0; c < ncols; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + c));
+                for (int c = chunk0; c < ncols; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + c));
             }
+            const float *bias_s = MLP && p.bias ? p.bias + n0 : nullptr;
             const bool ok = __all_sync(0xffffffffu, mbar_wait(&tfull[acc], (j >> 1) & 1) ? 1 : 0) != 0;
             if (!ok && lane == 0) atomicExch(p.err, 3);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool live = ok && !*(volatile int *)abort_flag && total > 0;  // warp-uniform
-            for (int c0 = 0; c0 < BNX; c0 += 32) {
+            for (int c0 = chunk0; c0 < BNX; c0 += 64) {
                 float v[32];
                 tmem_ld32(tmem + ((uint32_t)(rq * 32) << 16) + (uint32_t)(acc * BNX + c0), v);
                 const int col0 = n0 + c0;
+                if constexpr (MLP) {
+                    const int ncol = min(32, p.N - col0);
+                    const bool in = live && row < p.M && ncol > 0;
+                    if (p.bias) {
+                        // lane q holds the bias of column q; one shuffle each instead of one load each
+                        const float bl = lane < ncol ? __ldg(bias_s + c0 + lane) : 0.0f;
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) v[q] = fmaxf(v[q] + __shfl_sync(0xffffffffu, bl, q), 0.0f);
+                        if (!in || ncol < 32) {
+#pragma unroll
+                            for (int q = 0; q < 32; ++q)
+                                if (!in || q >= ncol) v[q] = 0.0f;
+                        }
+                    } else {
+                        const __nv_bfloat16 *mk = p.mask + (long long)row * p.ldm + col0;
+                        if (in && ncol == 32 && (reinterpret_cast<uintptr_t>(mk) & 15) == 0) {
+                            uint32_t m[16];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                *reinterpret_cast<uint4 *>(m + 4 * q) = reinterpret_cast<const uint4 *>(mk)[q];
+#pragma unroll
+                            for (int q = 0; q < 16; ++q) {  // a bf16 is above zero if its sign is clear and it is not zero
+                                if ((int16_t)(m[q] & 0xffff) <= 0) v[2 * q] = 0.0f;
+                                if ((int16_t)(m[q] >> 16) <= 0) v[2 * q + 1] = 0.0f;
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 32; ++q)
+                                if (!(in && q < ncol && __bfloat162float(mk[q]) > 0.0f)) v[q] = 0.0f;
+                        }
+                    }
+                    __nv_bfloat16 hi[32];
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) hi[q] = __float2bfloat16_rn(v[q]);
+                    if (live && ncol > 0) write_bf16(hi, p.Ohi, p.Thi, m0 + rq * 32, col0);
+                    if (p.colsum) {
+                        const float sum = warp_column_sums(v);
+                        if (live && lane < ncol) atomicAdd(p.colsum + col0 + lane, sum);
+                    }
+                    continue;
+                }
                 if (live && row < p.M && col0 < p.N) {
                     const int ncol = min(32, p.N - col0);
                     if (p.ksplit > 1) {  // partial sums over this tile's K range
+                        float *c = &p.C[(long long)row * p.ldc + col0];
+                        if (ncol == 32 && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
 #pragma unroll
-                        for (int q = 0; q < 32; ++q)
-                            if (q < ncol) atomicAdd(&p.C[(long long)row * p.ldc + col0 + q], p.alpha * v[q]);
+                            for (int q = 0; q < 32; q += 4)  // four elements per reduction where the row is aligned
+                                atomicAdd(reinterpret_cast<float4 *>(c + q),
+                                          make_float4(p.alpha * v[q], p.alpha * v[q + 1], p.alpha * v[q + 2],
+                                                      p.alpha * v[q + 3]));
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 32; ++q)
+                                if (q < ncol) atomicAdd(c + q, p.alpha * v[q]);
+                        }
                     } else {
                         const int n1 = min(16, ncol), n2 = ncol - 16;  // the two 16-column halves (n2 <= 0: none)
 #pragma unroll
@@ -421,61 +516,16 @@ __global__ void __launch_bounds__(192, 1) gemm_kernel(const __grid_constant__ Ma
                             store_row16(p.C + (long long)row * p.ldc + col0, n1, v);
                             if (n2 > 0) store_row16(p.C + (long long)row * p.ldc + col0 + 16, n2, v + 16);
                         }
-                        if (p.Ohi || stage_t) {
-                            __nv_bfloat16 hi[32], lo[32];
-#pragma unroll
-                            for (int q = 0; q < 32; ++q) {
-                                hi[q] = __float2bfloat16_rn(v[q]);
-                                lo[q] = __float2bfloat16_rn(v[q] - __bfloat162float(hi[q]));
-                            }
-                            if (p.Ohi) {
-                                __nv_bfloat16 *oh = p.Ohi + (long long)row * p.ldo + col0;
-                                __nv_bfloat16 *ol = p.Olo + (long long)row * p.ldo + col0;
-                                store_row16_bf16(oh, n1, hi);
-                                store_row16_bf16(ol, n1, lo);
-                                if (n2 > 0) {
-                                    store_row16_bf16(oh + 16, n2, hi + 16);
-                                    store_row16_bf16(ol + 16, n2, lo + 16);
-                                }
-                            }
-                            if (stage_t) {
-                                // column c0+q of the tile: the warp's 32 lanes write 32 consecutive rows
-#pragma unroll
-                                for (int q = 0; q < 32; ++q) {
-                                    sh[q * TPITCH + lane] = hi[q];
-                                    sl[q * TPITCH + lane] = lo[q];
-                                }
-                            }
-                        }
                     }
                 }
-                if (stage_t) {
-                    __syncwarp();
-                    if (live && col0 < p.N) {
-                        // this warp's 32 x 32 block of T: T-rows col0 .. col0+31, T-columns m0+32rq .. +31
+                if ((p.Ohi || p.Thi) && p.ksplit == 1 && live && col0 < p.N) {  // rows beyond M are staged, not written
+                    __nv_bfloat16 x[32];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const int c = q * 8 + (lane >> 2), part = lane & 3;
-                            const int trow = col0 + c, tcol0 = m0 + rq * 32 + part * 8;
-                            const int nv = min(8, p.M - tcol0);
-                            if (trow < p.N && nv > 0) {
-                                const long long off = (long long)trow * p.ldt + tcol0;
-                                const __nv_bfloat16 *srh = sh + c * TPITCH + part * 8, *srl = sl + c * TPITCH + part * 8;
-                                __nv_bfloat16 *dh = p.Thi + off, *dl = p.Tlo + off;
-                                if (nv == 8 &&
-                                    ((reinterpret_cast<uintptr_t>(dh) | reinterpret_cast<uintptr_t>(dl)) & 15) == 0) {
-                                    *reinterpret_cast<uint4 *>(dh) = *reinterpret_cast<const uint4 *>(srh);
-                                    *reinterpret_cast<uint4 *>(dl) = *reinterpret_cast<const uint4 *>(srl);
-                                } else {
-                                    for (int e = 0; e < nv; ++e) {
-                                        dh[e] = srh[e];
-                                        dl[e] = srl[e];
-                                    }
-                                }
-                            }
-                        }
-                    }
-                    __syncwarp();
+                    for (int q = 0; q < 32; ++q) x[q] = __float2bfloat16_rn(v[q]);
+                    write_bf16(x, p.Ohi, p.Thi, m0 + rq * 32, col0);
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) x[q] = __float2bfloat16_rn(v[q] - __bfloat162float(x[q]));
+                    write_bf16(x, p.Olo, p.Tlo, m0 + rq * 32, col0);
                 }
             }
             // the accumulator has been read: hand it back to the MMA issuer
@@ -562,6 +612,44 @@ int make_map(CUtensorMap *map, const void *base, int rows, int cols, long long l
     return 0;
 }
 
+// mode: 0 segments, 1 split, 2 split with 128 x 256 tiles, 3 segments with a dense layer's epilogue
+int launch(const Maps &maps, const Params &p, int mode, void *stream) {
+    using Kernel = void (*)(const Maps, const Params);
+    static const Kernel kernels[4] = {gemm_kernel<false, false>, gemm_kernel<true, false>, gemm_kernel<true, true>,
+                                      gemm_kernel<false, false, true>};
+    static const int smem[4] = {Cfg<false>::SMEM_BYTES, Cfg<true>::SMEM_BYTES, Cfg<true, true>::SMEM_BYTES,
+                                Cfg<false>::SMEM_BYTES};
+    static bool attr_set[4][64] = {{false}};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[mode][dev]) {
+        if (cudaFuncSetAttribute(kernels[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, smem[mode]) != cudaSuccess) {
+            snprintf(g_err, sizeof(g_err), "bf16x3_gemm: cannot reserve %d bytes of shared memory", smem[mode]);
+            return DFTB_ERR_CUDA;
+        }
+        if (dev >= 0 && dev < 64) attr_set[mode][dev] = true;
+    }
+    const int bnx = mode == 2 ? Cfg<true, true>::BNX : Cfg<false>::BNX;
+    // persistent launch: one CTA per SM (the shared-memory footprint admits one), each walking tiles
+    const long long ntiles = (long long)((p.M + BM - 1) / BM) * ((p.N + bnx - 1) / bnx) * p.ksplit;
+    if (ntiles > (1LL << 30)) return DFTB_ERR_BAD_SIZE;
+    static int sm_count[64] = {0};
+    if (dev >= 0 && dev < 64 && sm_count[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        sm_count[dev] = n;
+    }
+    const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
+    kernels[mode]<<<(unsigned)(ntiles < sms ? ntiles : sms), THREADS, smem[mode], reinterpret_cast<cudaStream_t>(stream)>>>(
+        maps, p);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        snprintf(g_err, sizeof(g_err), "gemm_kernel: %s", cudaGetErrorString(e));
+        return DFTB_ERR_CUDA;
+    }
+    return DFTB_OK;
+}
+
 }  // namespace tcg
 
 extern "C" {
@@ -633,48 +721,53 @@ int dftb_bf16x3_gemm_ex(int M, int N, int K, int nseg, int shared_split, int ksp
     p.Tlo = reinterpret_cast<__nv_bfloat16 *>(Tlo);
     p.ldt = ldt;
     p.err = err;
-    static bool attr_set[3][64] = {{false}};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int mode = shared_split;  // 0 segments, 1 split, 2 split with 128 x 256 tiles
-    const int smem = mode == 2 ? Cfg<true, true>::SMEM_BYTES : (mode ? Cfg<true>::SMEM_BYTES : Cfg<false>::SMEM_BYTES);
-    if (dev >= 0 && dev < 64 && !attr_set[mode][dev]) {
-        cudaError_t e =
-            mode == 2 ? cudaFuncSetAttribute(gemm_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-            : mode    ? cudaFuncSetAttribute(gemm_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-                      : cudaFuncSetAttribute(gemm_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             smem);
-        if (e != cudaSuccess) {
-            snprintf(g_err, sizeof(g_err), "bf16x3_gemm: cannot reserve %d bytes of shared memory", smem);
-            return DFTB_ERR_CUDA;
-        }
-        attr_set[mode][dev] = true;
+    p.bias = nullptr;
+    p.mask = nullptr;
+    p.ldm = 0;
+    p.colsum = nullptr;
+    return tcg::launch(maps, p, shared_split, stream);
+}
+
+int dftb_mlp_dense(int ns, int nout, int nin, const void *X, int ldx, const void *W, int ldw, const float *bias,
+                   const void *mask, int ldm, void *H, int ldh, void *HT, int ldht, float *colsum, int *err,
+                   void *stream) {
+    using namespace tcg;
+    if (ns <= 0 || nout <= 0 || nin <= 0 || ldx % 8 || ldw % 8 || ldx < nin || ldw < nin || (H && ldh < nout) ||
+        (HT && ldht < ns) || (mask && ldm < nout)) {
+        snprintf(g_err, sizeof(g_err), "mlp_dense: sizes or leading dimensions");
+        return DFTB_ERR_BAD_SIZE;
     }
-    const int bnx = mode == 2 ? Cfg<true, true>::BNX : (mode ? Cfg<true>::BNX : Cfg<false>::BNX);
-    // persistent launch: one CTA per SM (the shared-memory footprint admits one), each walking tiles
-    const long long ntiles = (long long)((M + BM - 1) / BM) * ((N + bnx - 1) / bnx) * ksplit;
-    if (ntiles > (1LL << 30)) return DFTB_ERR_BAD_SIZE;
-    static int sm_count[64] = {0};
-    if (dev >= 0 && dev < 64 && sm_count[dev] == 0) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        sm_count[dev] = n;
+    if (!X || !W || !err || (!bias == !mask) || (!H && !HT)) {
+        snprintf(g_err, sizeof(g_err), "mlp_dense: operands, a bias or a mask, and an output");
+        return DFTB_ERR_NULL;
     }
-    const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
-    dim3 grid((unsigned)(ntiles < sms ? ntiles : sms));
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (mode == 2)
-        gemm_kernel<true, true><<<grid, 192, smem, st>>>(maps, p);
-    else if (mode == 1)
-        gemm_kernel<true, false><<<grid, 192, smem, st>>>(maps, p);
-    else
-        gemm_kernel<false, false><<<grid, 192, smem, st>>>(maps, p);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        snprintf(g_err, sizeof(g_err), "gemm_kernel: %s", cudaGetErrorString(e));
+    if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) {
+        snprintf(g_err, sizeof(g_err), "mlp_dense: operands must be 16-byte aligned");
+        return DFTB_ERR_BAD_SIZE;
+    }
+    if (get_encode()) return DFTB_ERR_CUDA;
+    Maps maps;
+    memset(&maps, 0, sizeof(maps));
+    if (make_map(&maps.a[0], X, ns, nin, ldx, BM, BK) || make_map(&maps.b[0], W, nout, nin, ldw, BN, BK))
         return DFTB_ERR_CUDA;
-    }
-    return DFTB_OK;
+    Params p;
+    memset(&p, 0, sizeof(p));
+    p.M = ns;
+    p.N = nout;
+    p.K = nin;
+    p.nseg = 1;
+    p.ksplit = 1;
+    p.alpha = 1.0f;
+    p.Ohi = reinterpret_cast<__nv_bfloat16 *>(H);
+    p.ldo = ldh;
+    p.Thi = reinterpret_cast<__nv_bfloat16 *>(HT);
+    p.ldt = ldht;
+    p.bias = bias;
+    p.mask = reinterpret_cast<const __nv_bfloat16 *>(mask);
+    p.ldm = ldm;
+    p.colsum = colsum;
+    p.err = err;
+    return launch(maps, p, 3, stream);
 }
 
 int dftb_split_bf16(int rows, int cols, const float *X, int ldx, int transpose, void *hi, void *lo, int ld,

@@ -47,12 +47,12 @@ def _bf16(rows, cols, dev):
     return torch.zeros((rows, cols), dtype=torch.bfloat16, device=dev)
 
 
-def _mm(A, B, M, N, K, C, ksplit=1):
-    """C (M x N, FP32) = A (M x K) . B (N x K)^T with BF16 K-major operands on the tensor cores."""
+def _mm(A, B, M, N, K, C, ksplit=1, zeroed=False):
+    """C (M x N, FP32) = A (M x K) . B (N x K)^T with BF16 K-major operands on the tensor cores (zeroed: C is zero)."""
     L = tcgemm._lib()
     Ap = (ctypes.c_void_p * 3)(A.data_ptr(), 0, 0)
     Bp = (ctypes.c_void_p * 3)(B.data_ptr(), 0, 0)
-    if ksplit > 1:
+    if ksplit > 1 and not zeroed:
         C.zero_()
     err = tcgemm._errword(A.device)
     rc = L.dftb_bf16x3_gemm_ex(M, N, K, 1, 0, int(ksplit), Ap, A.stride(0), Bp, B.stride(0), 1.0, None, 0,
@@ -64,8 +64,10 @@ def _mm(A, B, M, N, K, C, ksplit=1):
 
 
 def _ksplit(M, N, K):
+    # one round of CTAs: 256 x 256 x 65536 takes 24 us in 37 ranges (51 in 64:
+    # two rounds of CTAs and more atomics)
     tiles = ((M + 127) // 128) * ((N + 127) // 128)
-    return max(1, min(64, (2 * tcgemm.SMS) // tiles, K // 512))
+    return max(1, min(64, tcgemm.SMS // tiles, K // 512))
 
 
 class GuessNet:
@@ -102,40 +104,47 @@ class GuessNet:
         self.W3bT[:, :NOUT] = self.W3.T.to(torch.bfloat16)
 
     # ------------------------------------------------------------ data layout
-    def _inputs(self, feats):
-        """Standardised features -> X (Ns x 64) and X^T (64 x Ns), BF16, Ns padded to SPAD."""
+    def _inputs(self, feats, weights=None, msum=None):
+        """Standardised features -> X (Ns x 64), BF16, Ns padded to SPAD; for training (weights given) also X^T
+        (64 x Ns) and the sum of the weights, added to msum."""
         n = feats.shape[0]
         ns = (n + SPAD - 1) // SPAD * SPAD
-        X = _bf16(ns, FPAD, self.device)
-        X[:n, :NFEAT] = ((feats.float() - self.mean) / self.std).to(torch.bfloat16)
-        return X, ns
+        F = torch.broadcast_to(feats.float(), (n, NFEAT))
+        if F.stride(1) != 1 or F.stride(0) < F.shape[1]:
+            F = F.contiguous()
+        X = torch.empty((ns, FPAD), dtype=torch.bfloat16, device=self.device)
+        XT = torch.empty((FPAD, ns), dtype=torch.bfloat16, device=self.device) if weights is not None else None
+        P = native.ptr
+        native.call("dftb_mlp_inputs", n, ns, NFEAT, FPAD, P(F), max(NFEAT, F.stride(0)), P(self.mean), P(self.std),
+                    P(X), FPAD, P(XT), ns, P(weights), P(msum), native.stream())
+        return X, XT, ns
+
+    def _dense(self, X, W, nin, ns, bias=None, mask=None, out=True, out_t=False, colsum=None):
+        """One hidden layer (dftb_mlp_dense): relu(X W^T + bias), or (X W^T) o (mask > 0), as BF16 (row-major,
+        transposed)."""
+        dev, P = self.device, native.ptr
+        H = torch.empty((ns, HIDDEN), dtype=torch.bfloat16, device=dev) if out else None
+        HT = torch.empty((HIDDEN, ns), dtype=torch.bfloat16, device=dev) if out_t else None
+        native.call("dftb_mlp_dense", ns, HIDDEN, nin, P(X), X.stride(0), P(W), W.stride(0), P(bias), P(mask), HIDDEN,
+                    P(H), HIDDEN, P(HT), ns, P(colsum), P(tcgemm._errword(dev)), native.stream())
+        return H, HT
 
     def _forward(self, X, ns, keep=False):
-        dev, P, st = self.device, native.ptr, native.stream()
-        Z = torch.empty((ns, HIDDEN), dtype=torch.float32, device=dev)
-        H1 = _bf16(ns, HIDDEN, dev)
-        H1T = _bf16(HIDDEN, ns, dev) if keep else None
-        _mm(X, self.W1b, ns, HIDDEN, FPAD, Z)
-        native.call("dftb_mlp_bias_relu", ns, HIDDEN, P(Z), HIDDEN, P(self.b1), P(H1), HIDDEN, P(H1T), ns, st)
-        H2 = _bf16(ns, HIDDEN, dev)
-        H2T = _bf16(HIDDEN, ns, dev) if keep else None
-        _mm(H1, self.W2b, ns, HIDDEN, HIDDEN, Z)
-        native.call("dftb_mlp_bias_relu", ns, HIDDEN, P(Z), HIDDEN, P(self.b2), P(H2), HIDDEN, P(H2T), ns, st)
-        Z3 = torch.empty((ns, OPAD), dtype=torch.float32, device=dev)
-        _mm(H2, self.W3b, ns, OPAD, HIDDEN, Z3)
-        return Z3, (H1, H1T, H2, H2T)
+        H1, H1T = self._dense(X, self.W1b, FPAD, ns, bias=self.b1, out_t=keep)
+        H2, _ = self._dense(H1, self.W2b, HIDDEN, ns, bias=self.b2)
+        return H1, H1T, H2
 
     # ------------------------------------------------------------ inference
     @torch.no_grad()
     def predict(self, feats):
         """(score, shift) per pair in the units of the targets (shift in Hartree)."""
         n = feats.shape[0]
-        X, ns = self._inputs(feats)
-        Z3, _ = self._forward(X, ns)
+        X, _, ns = self._inputs(feats)
+        _, _, H2 = self._forward(X, ns)
         Y = torch.empty((ns, NOUT), dtype=torch.float32, device=self.device)
         P = native.ptr
-        native.call("dftb_mlp_output", ns, NOUT, P(Z3), OPAD, P(self.b3), None, None, None, 0.0, P(Y), None, 0,
-                    None, 0, None, None, native.stream())
+        native.call("dftb_mlp_head", ns, 0, HIDDEN, P(H2), HIDDEN, P(self.W3b), HIDDEN, P(self.b3), None, None, None,
+                    0.0, 0.0, None, P(Y), None, 0, None, 0, None, None, None, None, native.stream())
         Y = Y[:n] / self.target_scale
         return Y[:, 0], Y[:, 1]
 
@@ -147,38 +156,25 @@ class GuessNet:
         against the CPU oracle."""
         dev, P, st = self.device, native.ptr, native.stream()
         n = feats.shape[0]
-        X, ns = self._inputs(feats)
-        XT = X.T.contiguous()
-        Z3, (H1, H1T, H2, H2T) = self._forward(X, ns, keep=True)
-        T = torch.zeros((ns, NOUT), dtype=torch.float32, device=dev)
-        T[:n] = targets.float() * self.target_scale
-        m = torch.zeros(ns, dtype=torch.float32, device=dev)
-        m[:n] = weights.float()
-        wout = torch.tensor(out_weights, dtype=torch.float32, device=dev)
-        inv_norm = 1.0 / max(float(m.sum()), 1e-30)
-        Y = torch.empty((ns, NOUT), dtype=torch.float32, device=dev)
-        dYp = _bf16(ns, FPAD, dev)
-        dYT = _bf16(OPAD, ns, dev)
-        grads = [torch.zeros_like(p) for p in self.params]
+        m = torch.broadcast_to(weights.float().to(dev), (n,)).contiguous()
+        # one zeroed buffer for everything that is summed into (each gradient on a 16-byte boundary); the forward pass
+        # is launched before its views are made
+        sizes = [(p.numel() + 3) // 4 * 4 for p in self.params]
+        flat = torch.zeros(sum(sizes) + 4, dtype=torch.float32, device=dev)
+        loss, msum = flat[-4:].view(torch.float64).split(1)
+        X, XT, ns = self._inputs(feats, m, msum)
+        H1, H1T, H2 = self._forward(X, ns, keep=True)
+        T = torch.broadcast_to(targets.float(), (n, NOUT)).contiguous()
+        grads = [f[:p.numel()].view(p.shape) for f, p in zip(flat[:-4].split(sizes), self.params)]
         dW1, db1, dW2, db2, dW3, db3 = grads
-        loss = torch.zeros(1, dtype=torch.float64, device=dev)
-        native.call("dftb_mlp_output", ns, NOUT, P(Z3), OPAD, P(self.b3), P(T), P(m), P(wout), float(inv_norm), P(Y),
-                    P(dYp), FPAD, P(dYT), ns, P(db3), P(loss), st)
-        dW3full = torch.empty((OPAD, HIDDEN), dtype=torch.float32, device=dev)
-        _mm(dYT, H2T, OPAD, HIDDEN, ns, dW3full, _ksplit(OPAD, HIDDEN, ns))
-        dW3.copy_(dW3full[:NOUT])
-        G = torch.empty((ns, HIDDEN), dtype=torch.float32, device=dev)
-        _mm(dYp, self.W3bT, ns, HIDDEN, FPAD, G)
-        dZ2 = _bf16(ns, HIDDEN, dev)
-        dZ2T = _bf16(HIDDEN, ns, dev)
-        native.call("dftb_mlp_relu_backward", ns, HIDDEN, P(G), HIDDEN, P(H2), HIDDEN, P(dZ2), HIDDEN, P(dZ2T), ns,
-                    P(db2), st)
-        _mm(dZ2T, H1T, HIDDEN, HIDDEN, ns, dW2, _ksplit(HIDDEN, HIDDEN, ns))
-        _mm(dZ2, self.W2bT, ns, HIDDEN, HIDDEN, G)
-        dZ1T = _bf16(HIDDEN, ns, dev)
-        native.call("dftb_mlp_relu_backward", ns, HIDDEN, P(G), HIDDEN, P(H1), HIDDEN, None, 0, P(dZ1T), ns,
-                    P(db1), st)
-        _mm(dZ1T, XT, HIDDEN, FPAD, ns, dW1, _ksplit(HIDDEN, FPAD, ns))
+        dZ2 = torch.empty((ns, HIDDEN), dtype=torch.bfloat16, device=dev)
+        dZ2T = torch.empty((HIDDEN, ns), dtype=torch.bfloat16, device=dev)
+        native.call("dftb_mlp_head", ns, n, HIDDEN, P(H2), HIDDEN, P(self.W3b), HIDDEN, P(self.b3), P(T),
+                    P(self.target_scale), P(m), float(out_weights[0]), float(out_weights[1]), P(msum), None, P(dZ2),
+                    HIDDEN, P(dZ2T), ns, P(dW3), P(db3), P(db2), P(loss), st)
+        _mm(dZ2T, H1T, HIDDEN, HIDDEN, ns, dW2, _ksplit(HIDDEN, HIDDEN, ns), zeroed=True)
+        _, dZ1T = self._dense(dZ2, self.W2bT, HIDDEN, ns, mask=H1, out=False, out_t=True, colsum=db1)
+        _mm(dZ1T, XT, HIDDEN, FPAD, ns, dW1, _ksplit(HIDDEN, FPAD, ns), zeroed=True)
         return float(loss.item()), grads
 
     def train_step(self, feats, targets, weights, lr=1e-3, weight_decay=0.0):

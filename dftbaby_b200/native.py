@@ -81,6 +81,10 @@ _SIGNATURES = {
     "dftb_mlp_output": (_I, [_I, _I, _P, _I, _P, _P, _P, _P, ctypes.c_float, _P, _P, _I, _P, _I, _P, _P, _P]),
     "dftb_mlp_adam": (_I, [_I, _I, _P, _P, _P, _P, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                            _I, ctypes.c_float, _P, _I, _P, _I, _P]),
+    "dftb_mlp_inputs": (_I, [_I, _I, _I, _I, _P, _I, _P, _P, _P, _I, _P, _I, _P, _P, _P]),
+    "dftb_mlp_dense": (_I, [_I, _I, _I, _P, _I, _P, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P]),
+    "dftb_mlp_head": (_I, [_I, _I, _I, _P, _I, _P, _I, _P, _P, _P, _P, ctypes.c_float, ctypes.c_float, _P, _P, _P, _I, _P,
+                           _I, _P, _P, _P, _P, _P]),
     "dftb_mlp_last_error": (ctypes.c_char_p, []),
     "dftb_batched_eigh_workspace_size": (_I, [_I, _I, ctypes.POINTER(_Z)]),
     "dftb_batched_eigh": (_I, [_I, _I, _P, _P, _P, _Z, _P, _P]),
@@ -149,7 +153,8 @@ def check(rc, what):
         msg = ""
         if _lib is not None:
             msg = (_lib.dftb_last_error().decode() or _lib.dftb_grad_last_error().decode()
-                   or _lib.dftb_mlp_last_error().decode() or _lib.dftb_eigh_last_error().decode()
+                   or _lib.dftb_mlp_last_error().decode() or _lib.dftb_tc_last_error().decode()
+                   or _lib.dftb_eigh_last_error().decode()
                    or _lib.dftb_solver_last_error().decode() or _lib.dftb_ozaki_last_error().decode())
         raise NativeError("%s failed (%s): %s" % (what, _ERRORS.get(rc, rc), msg))
 
@@ -162,7 +167,7 @@ KERNELS_PER_CALL = {
     "dftb_davidson_precondition": 1, "dftb_davidson_residual": 2, "dftb_dgemm": 1,
     "dftb_gradients_h0_and_s": 3, "dftb_sk_gradient_contract": 1, "dftb_pair_gradients": 1,
     "dftb_repulsive_energy": 1, "dftb_mlp_bias_relu": 1, "dftb_mlp_relu_backward": 1, "dftb_mlp_output": 1,
-    "dftb_mlp_adam": 1, "dftb_ozaki_dgemm": 6, "dftb_ozaki_prepare": 2, "dftb_ozaki_product": 2,
+    "dftb_mlp_adam": 1, "dftb_mlp_inputs": 1, "dftb_mlp_dense": 1, "dftb_mlp_head": 1, "dftb_ozaki_dgemm": 6, "dftb_ozaki_prepare": 2, "dftb_ozaki_product": 2,
 }
 
 

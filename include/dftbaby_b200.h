@@ -377,6 +377,25 @@ int dftb_mlp_output(int ns, int no, const float *Z, int ldz, const float *b, con
 int dftb_mlp_adam(int rows, int cols, float *W, const float *G, float *m1, float *m2, float lr, float beta1,
                   float beta2, float eps, int step, float weight_decay, void *Wb, int ldwb, void *WbT, int ldwbt,
                   void *stream);
+/* The fused layers that training and inference run on.
+ * dftb_mlp_inputs: X (ns x fpad, BF16) = (F - mean) / std of n x nf FP32 features, zero-padded, and, unless XT is NULL,
+ * its transpose; with sample weights m (n), msum (device, FP64) is increased by their sum.
+ * dftb_mlp_dense: V = X W^T on the tensor cores (X: ns x nin, W: nout x nin, BF16, leading dimensions multiples of 8,
+ * 16-byte aligned; FP32 accumulation) with the layer's epilogue: relu(V + bias), or V o (mask > 0) for the backward pass
+ * (exactly one of bias and mask is given).  The result goes to H (BF16, row-major) and/or HT (transposed); colsum, unless
+ * NULL, is increased by its column sums (before rounding).  err as for dftb_bf16x3_gemm.
+ * dftb_mlp_head: the output layer of two units, y = H W^T + b (H: ns x nh, nh <= 256).  Inference (T NULL): Y (ns x 2).
+ * Training: with targets T (n x 2, times tscale), sample weights m (n), their sum msum (device) and output weights wout0, wout1,
+ * the loss (FP64, increased) and gradients of the first n samples: dW (2 x nh), db (2) and dbz (nh) are increased,
+ * dZ = (dY W) o (H > 0) is written row-major and transposed (zero for the samples beyond n); Y may be NULL. */
+int dftb_mlp_inputs(int n, int ns, int nf, int fpad, const float *F, int ldf, const float *mean, const float *std,
+                    void *X, int ldx, void *XT, int ldxt, const float *m, double *msum, void *stream);
+int dftb_mlp_dense(int ns, int nout, int nin, const void *X, int ldx, const void *W, int ldw, const float *bias,
+                   const void *mask, int ldm, void *H, int ldh, void *HT, int ldht, float *colsum, int *err,
+                   void *stream);
+int dftb_mlp_head(int ns, int n, int nh, const void *H, int ldh, const void *W, int ldw, const float *b, const float *T,
+                  const float *tscale, const float *m, float wout0, float wout1, const double *msum, float *Y, void *dZ,
+                  int lddz, void *dZT, int lddzt, float *dW, float *db, float *dbz, double *loss, void *stream);
 const char *dftb_mlp_last_error(void);
 
 /* ---- batched symmetric eigensolver --------------------------------------------
