@@ -165,8 +165,7 @@ def batched_gradients(G, lc, scc, exc, state, par, r_lr):
     out = []
     for b, m in enumerate(G.mols):
         n = m.norb
-        g = contract(m, par, r_lr, XS[b, :n, :n].contiguous(), XH[b, :n, :n].contiguous(),
-                     Yg[b, :n, :n].contiguous(), Ylr[b, :n, :n].contiguous() if lc else None, True)
+        g = contract(m, par, r_lr, XS[b, :n, :n], XH[b, :n, :n], Yg[b, :n, :n], Ylr[b, :n, :n] if lc else None, True)
         out.append(g)
     return [g.cpu().numpy() for g in out]
 

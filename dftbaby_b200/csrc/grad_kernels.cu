@@ -306,6 +306,236 @@ __global__ void __launch_bounds__(kGradThreads) vrep_energy_kernel(int nat, cons
     if (threadIdx.x == 0) e[i] = 0.5 * s;
 }
 
+// ----------------------------------------------------------------------------
+// The whole contraction of one molecule in one launch.  A block per atom J; two warps each take the S, the H0, the gamma
+// (with the repulsive potential) and the gamma^lr terms, a thread an atom I at a time.  The adjoints are symmetrised and
+// summed as they are read.  The SK rules are linear in the adjoint, so an atom pair's orbital block enters as one scalar
+// (s-s), two vectors (s-p, p-s) and a 3 x 3 matrix (p-p) against ten spline values and derivatives, instead of 16 rules
+// with their own splines; tables with the same knots share their B-splines.  Bound by latency for small molecules (one
+// pass of a block is a chain of about ten loads), by the FP64 pipe for large ones.  B200: C40H42 21 us (the separate
+// kernels 54 + 7 us, and 50 us of torch kernels for the symmetrised adjoints and block sums), C294H42 139 us.
+// ----------------------------------------------------------------------------
+constexpr int GC_ROLE = 64, GC_THREADS = 4 * GC_ROLE;
+constexpr int GC_SMEM = 24 << 10;  // a molecule's orbital tables go to shared memory up to this size (3000 carbons)
+
+struct GradP {
+    int norb, nat, npair;
+    OrbTables O;
+    const double *r, *x, *y, *z;
+    const int *mprox;
+    SkTables T[2];           // S, H0
+    const double *X[2];      // XS, XH
+    long long ldx[2];
+    const double *pos, *sigma;
+    const int *atype;
+    double r_lr;
+    const double *Y[2];      // Yg, Ylr
+    long long ldy[2];
+    VrepTables V;
+    int use_vrep, use_smem;
+    double *out;
+};
+
+// B-splines of the value (splev_uniform's interval) and of the derivative (FITPACK's interval), with the derivative's
+// coefficient factors 3 / (t(i+4) - t(i+1)) (negative: the degenerate case, in which the coefficient itself counts)
+struct GradBasis {
+    SkBasis v;
+    double h[3], w[3];
+    int l;
+};
+
+__device__ GradBasis grad_basis(const double *__restrict__ t, int n, double r) {
+    GradBasis b;
+    b.v = sk_basis(t, n, r);
+    const double tb = t[3], te = t[n - 4], arg = r < tb ? tb : (r > te ? te : r);
+    b.l = knot_interval(t, n, arg);
+    double hh[2];
+    b.h[0] = 1.0;
+#pragma unroll
+    for (int j = 1; j <= 2; ++j) {
+#pragma unroll
+        for (int i = 1; i <= j; ++i) hh[i - 1] = b.h[i - 1];
+        b.h[0] = 0.0;
+#pragma unroll
+        for (int i = 1; i <= j; ++i) {
+            const double hi = t[b.l + i - 1], lo = t[b.l + i - j - 1];
+            const double f = hh[i - 1] / (hi - lo);
+            b.h[i - 1] = b.h[i - 1] + f * (hi - arg);
+            b.h[i] = f * (arg - lo);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int ll = b.l - 3 + j;  // 1-based coefficient
+        const double fac = t[ll + 3] - t[ll];
+        b.w[j] = fac > 0.0 ? 3.0 / fac : -1.0;
+    }
+    return b;
+}
+
+__device__ __forceinline__ void grad_eval(const GradBasis &b, const double *__restrict__ c, double &v, double &d) {
+    v = sk_dot(b.v, c);
+    d = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const double *q = c + (b.l - 4 + j);
+        d += (b.w[j] > 0.0 ? b.w[j] * (q[1] - q[0]) : q[0]) * b.h[j];
+    }
+}
+
+__global__ void __launch_bounds__(GC_THREADS) gradient_kernel(const GradP p) {
+    constexpr int tabs[5] = {0, 2, 4, 5, 6};  // ss, sp, ps, pp-pi, pp-sigma
+    extern __shared__ int gc_sm[];
+    __shared__ double red[GC_THREADS / 32];
+    __shared__ unsigned mask[SK_SHARED_PAIRS];
+    __shared__ int range[2];
+    int *first = gc_sm;                                                                   // nat + 1
+    unsigned char *kind = reinterpret_cast<unsigned char *>(gc_sm + p.nat + 1);           // norb
+    const int J = blockIdx.x, tid = threadIdx.x, role = tid / GC_ROLE, lane64 = tid % GC_ROLE;
+    const OrbTables &O = p.O;
+    const bool sk = p.X[0] || p.X[1];
+    auto kind_of = [&](int mu) { return O.ls[mu] == 0 ? 0 : (O.ls[mu] == 1 ? 1 + axis_of_m(O.ms[mu]) : 255); };
+    if (tid < SK_SHARED_PAIRS) mask[tid] = 0u;
+    if (p.use_smem) {
+        for (int mu = tid; mu < p.norb; mu += GC_THREADS) {
+            const int a = O.ind[mu], before = mu ? O.ind[mu - 1] : -1;
+            for (int k = before + 1; k <= min(a, p.nat); ++k) first[k] = mu;
+            if (mu == p.norb - 1)
+                for (int k = a + 1; k <= p.nat; ++k) first[k] = p.norb;
+            kind[mu] = (unsigned char)kind_of(mu);
+        }
+    } else if (tid < 2) {
+        range[tid] = first_orbital(O.ind, p.norb, J + tid);
+    }
+    __syncthreads();
+    const int f0 = p.use_smem ? first[J] : range[0], f1 = p.use_smem ? first[J + 1] : range[1];
+    int typj = 0;
+    if (sk && f0 < f1) {
+        // the type pairs of this atom's type
+        typj = O.typ[f0];
+        unsigned present = 0;
+        for (int t = 0; t < SK_SHARED_PAIRS; ++t) {
+            const int hi = max(t, typj), q = hi * (hi + 1) / 2 + min(t, typj);
+            if (q < p.npair && q < SK_SHARED_PAIRS) present |= 1u << q;
+        }
+        sk_shared_tables(p.T[0], &p.T[1], tabs, present, mask);
+    }
+    __syncthreads();
+    double acc[3] = {0.0, 0.0, 0.0};
+    if (role < 2 && p.X[role] && f0 < f1) {
+        const SkTables T = p.T[role];
+        const double *X = p.X[role];
+        const long long ld = p.ldx[role];
+        for (int I = lane64; I < p.nat; I += GC_ROLE) {
+            if (I == J || p.mprox[(size_t)I * p.nat + J] == 0) continue;
+            const int g0 = p.use_smem ? first[I] : first_orbital(O.ind, p.norb, I);
+            const int g1 = p.use_smem ? first[I + 1] : first_orbital(O.ind, p.norb, I + 1);
+            if (g0 >= g1) continue;
+            double rij, e[3];
+            pair_dir(p.nat, p.r, p.x, p.y, p.z, I, J, rij, e);
+            const int typi = O.typ[g0], tmax = max(typi, typj), ipair = tmax * (tmax + 1) / 2 + min(typi, typj);
+            const bool straight = typi <= typj;
+            const double sgn = straight ? 1.0 : -1.0;
+            for (int k = 0; k < 3; ++k) e[k] *= sgn;
+            // the symmetrised block by kinds of the (first, second) orbital
+            double ss = 0.0, sp[3] = {0.0, 0.0, 0.0}, ps[3] = {0.0, 0.0, 0.0}, pp[3][3] = {};
+            for (int nu = f0; nu < f1; ++nu) {
+                const int kn = p.use_smem ? kind[nu] : kind_of(nu);
+                for (int mu = g0; mu < g1; ++mu) {
+                    const int km = p.use_smem ? kind[mu] : kind_of(mu);
+                    if (max(kn, km) > 3) continue;  // l > 1
+                    const double v = X[(long long)mu * ld + nu] + X[(long long)nu * ld + mu];
+                    const int k1 = straight ? km : kn, k2 = straight ? kn : km;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        if (k1 == 0 && k2 == a + 1) sp[a] += v;
+                        if (k1 == a + 1 && k2 == 0) ps[a] += v;
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+                            if (k1 == a + 1 && k2 == c + 1) pp[a][c] += v;
+                    }
+                    if (k1 + k2 == 0) ss += v;
+                }
+            }
+            // spline values and derivatives
+            unsigned filled = 0, shared = 0;
+            if (ipair < SK_SHARED_PAIRS) {
+                filled = mask[ipair] >> (5 * role) & 31u;
+                shared = mask[ipair] >> (16 + 5 * role) & 31u;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    if (tabs[q] < T.nsk && T.filled[ipair * T.nsk + tabs[q]] == 1) filled |= 1u << q;
+            }
+            const size_t o = (size_t)ipair * T.nsk * T.npts;
+            GradBasis b = {};
+            if (shared)
+                b = grad_basis(p.T[0].knots + ((size_t)ipair * p.T[0].nsk + sk_first_filled(p.T[0], ipair, tabs)) *
+                                                  p.T[0].npts,
+                               p.T[0].npts, rij);
+            double v[5], d[5];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                v[q] = d[q] = 0.0;
+                if (shared >> q & 1)
+                    grad_eval(b, T.coefs + o + tabs[q] * T.npts, v[q], d[q]);
+                else if (filled >> q & 1)
+                    grad_eval(grad_basis(T.knots + o + tabs[q] * T.npts, T.npts, rij), T.coefs + o + tabs[q] * T.npts,
+                              v[q], d[q]);
+            }
+            // d/d(r e): e_k along the bond, (delta_ak - e_a e_k) / r across it (slako_transformations_grad_lmax2.f90)
+            const double ri = 1.0 / rij;
+            double spe = 0.0, pse = 0.0, tr = 0.0, Me[3], qe = 0.0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                spe += sp[a] * e[a];
+                pse += ps[a] * e[a];
+                tr += pp[a][a];
+                Me[a] = 0.0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) Me[a] += (pp[a][c] + pp[c][a]) * e[c];
+                qe += 0.5 * Me[a] * e[a];
+            }
+            const double along = ss * d[0] + spe * (d[1] - v[1] * ri) + pse * (d[2] - v[2] * ri) + tr * d[3] +
+                                 qe * (d[4] - d[3] - 2.0 * (v[4] - v[3]) * ri);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                acc[k] += sgn * (along * e[k] + ri * (v[1] * sp[k] + v[2] * ps[k] + (v[4] - v[3]) * Me[k]));
+        }
+    } else if (role >= 2 && (p.Y[role - 2] || (role == 2 && p.use_vrep))) {
+        const double *Y = p.Y[role - 2];
+        const long long ld = p.ldy[role - 2];
+        const double extra = role == 3 ? 0.5 * p.r_lr * p.r_lr : 0.0;
+        for (int I = lane64; I < p.nat; I += GC_ROLE) {
+            if (I == J) continue;
+            const double dx = p.pos[3 * J] - p.pos[3 * I], dy = p.pos[3 * J + 1] - p.pos[3 * I + 1],
+                         dz = p.pos[3 * J + 2] - p.pos[3 * I + 2];
+            const double R = sqrt(dx * dx + dy * dy + dz * dz);
+            double w = 0.0;
+            if (Y) {
+                const int g0 = p.use_smem ? first[I] : first_orbital(O.ind, p.norb, I);
+                const int g1 = p.use_smem ? first[I + 1] : first_orbital(O.ind, p.norb, I + 1);
+                double sum = 0.0;
+                for (int nu = f0; nu < f1; ++nu)
+                    for (int mu = g0; mu < g1; ++mu) sum += Y[(long long)mu * ld + nu] + Y[(long long)nu * ld + mu];
+                const double s2 = p.sigma[J] * p.sigma[J] + p.sigma[I] * p.sigma[I];
+                w = gauss_gamma_deriv(1.0 / sqrt(2.0 * (s2 + extra)), R) * sum;
+            }
+            if (role == 2 && p.use_vrep) {
+                const int ta = p.atype[J], tb = p.atype[I], tmax = max(ta, tb);
+                w += vrep_eval(p.V, tmax * (tmax + 1) / 2 + min(ta, tb), R, 1);
+            }
+            acc[0] += w * dx / R;
+            acc[1] += w * dy / R;
+            acc[2] += w * dz / R;
+        }
+    }
+    for (int c = 0; c < 3; ++c) {
+        const double s = block_sum<GC_THREADS>(acc[c], red);
+        if (tid == 0) p.out[3 * J + c] = s;
+    }
+}
+
 int fail_grad(int code, const char *what) {
     snprintf(g_last_error_grad, sizeof(g_last_error_grad), "%s", what);
     return code;
@@ -383,6 +613,58 @@ int dftb_repulsive_energy(int nat, const double *pos, const int *atype, const do
     VrepTables V{vrep_knots, vrep_coefs, vrep_dmax, nknots};
     vrep_energy_kernel<<<nat, kGradThreads, 0, S(stream)>>>(nat, pos, atype, V, e_atom);
     return check_launch("vrep_energy_kernel");
+}
+
+int dftb_gradient_contract(int norb, int nat, const int *ind, const int *typ, const int *ls, const int *ms,
+                           const double *r, const double *x, const double *y, const double *z, const int *mprox,
+                           int deg, const int *tab_filled, const double *S_knots, const double *S_coefs,
+                           const double *H_knots, const double *H_coefs, int npair, int nsk, int npts,
+                           const double *pos, const int *atype, const double *sigma, double r_lr, const double *XS,
+                           int ldxs, const double *XH, int ldxh, const double *Yg, int ldyg, const double *Ylr,
+                           int ldylr, const double *vrep_knots, const double *vrep_coefs, const double *vrep_dmax,
+                           int nknots, double *grad, void *stream) {
+    if (norb <= 0 || nat <= 0 || npair <= 0 || nsk <= 0 || npts < 8)
+        return fail_grad(DFTB_ERR_BAD_SIZE, "gradient_contract: sizes");
+    if (deg != 3) return fail_grad(DFTB_ERR_UNSUPPORTED, "gradient_contract: only cubic splines");
+    const int use_vrep = vrep_knots != nullptr;
+    if (use_vrep && (nknots < 8 || !vrep_coefs || !vrep_dmax))
+        return fail_grad(DFTB_ERR_BAD_SIZE, "gradient_contract: repulsive-potential tables");
+    if ((XS && ldxs < norb) || (XH && ldxh < norb) || (Yg && ldyg < norb) || (Ylr && ldylr < norb))
+        return fail_grad(DFTB_ERR_BAD_SIZE, "gradient_contract: leading dimensions");
+    if (!ind || !typ || !ls || !ms || !r || !x || !y || !z || !mprox || !tab_filled || !S_knots || !S_coefs ||
+        !H_knots || !H_coefs || !pos || !grad || ((Yg || Ylr) && !sigma) || (use_vrep && !atype))
+        return fail_grad(DFTB_ERR_NULL, "gradient_contract: null");
+    GradP p;
+    p.norb = norb;
+    p.nat = nat;
+    p.npair = npair;
+    p.O = OrbTables{ind, typ, ls, ms};
+    p.r = r;
+    p.x = x;
+    p.y = y;
+    p.z = z;
+    p.mprox = mprox;
+    p.T[0] = SkTables{tab_filled, S_knots, S_coefs, nsk, npts};
+    p.T[1] = SkTables{tab_filled, H_knots, H_coefs, nsk, npts};
+    p.X[0] = XS;
+    p.X[1] = XH;
+    p.ldx[0] = ldxs;
+    p.ldx[1] = ldxh;
+    p.pos = pos;
+    p.sigma = sigma;
+    p.atype = atype;
+    p.r_lr = r_lr;
+    p.Y[0] = Yg;
+    p.Y[1] = Ylr;
+    p.ldy[0] = ldyg;
+    p.ldy[1] = ldylr;
+    p.V = VrepTables{vrep_knots, vrep_coefs, vrep_dmax, nknots};
+    p.use_vrep = use_vrep;
+    p.out = grad;
+    const size_t smem = sizeof(int) * ((size_t)nat + 1) + (size_t)norb;
+    p.use_smem = smem <= (size_t)GC_SMEM;
+    gradient_kernel<<<nat, GC_THREADS, p.use_smem ? smem : 0, S(stream)>>>(p);
+    return check_launch("gradient_kernel");
 }
 
 }  // extern "C"

@@ -69,34 +69,27 @@ def _Flr_adjoint(S, g, v, W):
 
 def contract(geo, par, r_lr, XS, XH, Yg, Ylr, vrep):
     """3 Nat gradient of one molecule from adjoints: SK pair derivatives against XS, XH (Norb x Norb);
-    gamma and gamma^lr derivatives against the orbital adjoints Yg, Ylr (summed per atom block here);
-    plus the repulsive potential when vrep is set.
+    gamma and gamma^lr derivatives against the orbital adjoints Yg, Ylr; plus the repulsive potential when vrep is
+    set.  The kernel symmetrises the adjoints and sums the gamma ones per atom block (dftb_gradient_contract).
 
     ``geo`` carries the molecule's device tables: ind, typ, ls, ms (orbital tables), dircos (r, x, y, z),
     mprox, pos, atype, sigma."""
     nat, norb = geo.pos.shape[0], geo.ind.shape[0]
     dev = geo.pos.device
-    P, st = native.ptr, native.stream()
+    if XS is None and XH is None and Yg is None and Ylr is None and not vrep:
+        return torch.zeros(3 * nat, dtype=torch.float64, device=dev)
+    P = native.ptr
     t = par.device_tables(dev)
     r, x, y, z = geo.dircos
-    out = torch.zeros(3 * nat, dtype=torch.float64, device=dev)
-    if XS is not None or XH is not None:
-        XSs = (XS + XS.T).contiguous() if XS is not None else None
-        XHs = (XH + XH.T).contiguous() if XH is not None else None
-        g = torch.empty(3 * nat, dtype=torch.float64, device=dev)
-        native.call("dftb_sk_gradient_contract", norb, nat, P(geo.ind), P(geo.typ), P(geo.ls), P(geo.ms), P(r),
-                    P(x), P(y), P(z), P(geo.mprox), par.deg, P(t["tab_filled_SH0"]), P(t["S_knots"]),
-                    P(t["S_coefs"]), P(t["H_knots"]), P(t["H_coefs"]), par.npair, par.nsk, par.npts, P(XSs), P(XHs),
-                    P(g), st)
-        out += g
-    if Yg is not None or Ylr is not None or vrep:
-        Ygs = _block_sum(Yg + Yg.T, geo.ind, nat).contiguous() if Yg is not None else None
-        Ylrs = _block_sum(Ylr + Ylr.T, geo.ind, nat).contiguous() if Ylr is not None else None
-        g = torch.empty(3 * nat, dtype=torch.float64, device=dev)
-        native.call("dftb_pair_gradients", nat, P(geo.pos), P(geo.atype), P(geo.sigma), float(r_lr), P(Ygs),
-                    P(Ylrs), P(t["vrep_knots"]) if vrep else None, P(t["vrep_coefs"]), P(t["vrep_dmax"]),
-                    par.vrep_nknots, P(g), st)
-        out += g
+    rows = lambda A: A if A is None or (A.stride(1) == 1 and A.stride(0) >= norb) else A.contiguous()
+    ld = lambda A: 0 if A is None else max(norb, A.stride(0))
+    XS, XH, Yg, Ylr = rows(XS), rows(XH), rows(Yg), rows(Ylr)
+    out = torch.empty(3 * nat, dtype=torch.float64, device=dev)
+    native.call("dftb_gradient_contract", norb, nat, P(geo.ind), P(geo.typ), P(geo.ls), P(geo.ms), P(r), P(x), P(y), P(z),
+                P(geo.mprox), par.deg, P(t["tab_filled_SH0"]), P(t["S_knots"]), P(t["S_coefs"]), P(t["H_knots"]),
+                P(t["H_coefs"]), par.npair, par.nsk, par.npts, P(geo.pos), P(geo.atype), P(geo.sigma), float(r_lr), P(XS),
+                ld(XS), P(XH), ld(XH), P(Yg), ld(Yg), P(Ylr), ld(Ylr), P(t["vrep_knots"]) if vrep else None,
+                P(t["vrep_coefs"]), P(t["vrep_dmax"]), par.vrep_nknots, P(out), native.stream())
     return out
 
 

@@ -74,6 +74,8 @@ _SIGNATURES = {
     "dftb_sk_gradient_contract": (_I, [_I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I,
                                        _I, _P, _P, _P, _P]),
     "dftb_pair_gradients": (_I, [_I, _P, _P, _P, _D, _P, _P, _P, _P, _P, _I, _P, _P]),
+    "dftb_gradient_contract": (_I, [_I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P,
+                                    _P, _P, _D, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _P, _P]),
     "dftb_repulsive_energy": (_I, [_I, _P, _P, _P, _P, _P, _I, _P, _P]),
     "dftb_grad_last_error": (ctypes.c_char_p, []),
     "dftb_mlp_bias_relu": (_I, [_I, _I, _P, _I, _P, _P, _I, _P, _I, _P]),
@@ -165,7 +167,7 @@ KERNELS_PER_CALL = {
     "dftb_ao_expand": 1, "dftb_scc_hamiltonian": 2, "dftb_monopoles": 1, "dftb_trans_charges": 4,
     "dftb_trans_charges_diag": 3, "dftb_trans_charges_noalloc": 6, "dftb_hermitian_rv": 3, "dftb_apbv": 2, "dftb_ambv": 1,
     "dftb_davidson_precondition": 1, "dftb_davidson_residual": 2, "dftb_dgemm": 1,
-    "dftb_gradients_h0_and_s": 3, "dftb_sk_gradient_contract": 1, "dftb_pair_gradients": 1,
+    "dftb_gradients_h0_and_s": 3, "dftb_sk_gradient_contract": 1, "dftb_pair_gradients": 1, "dftb_gradient_contract": 1,
     "dftb_repulsive_energy": 1, "dftb_mlp_bias_relu": 1, "dftb_mlp_relu_backward": 1, "dftb_mlp_output": 1,
     "dftb_mlp_adam": 1, "dftb_mlp_inputs": 1, "dftb_mlp_dense": 1, "dftb_mlp_head": 1, "dftb_ozaki_dgemm": 6, "dftb_ozaki_prepare": 2, "dftb_ozaki_product": 2,
 }

@@ -340,6 +340,20 @@ int dftb_pair_gradients(int nat, const double *pos, const int *atype, const doub
                         const double *Yg, const double *Ylr, const double *vrep_knots, const double *vrep_coefs,
                         const double *vrep_dmax, int nknots, double *grad, void *stream);
 
+/* Both contractions for one molecule, from adjoints as they come (not symmetrised, gamma adjoints per orbital):
+ *   grad = dftb_sk_gradient_contract with XS + XS^T, XH + XH^T
+ *        + dftb_pair_gradients with the atom-block sums of Yg + Yg^T, Ylr + Ylr^T.
+ * XS, XH, Yg, Ylr: (norb, norb), row-major with leading dimensions of their own, or NULL each; vrep_knots = NULL
+ * skips the repulsive potential.  grad: (3 nat), overwritten. */
+int dftb_gradient_contract(int norb, int nat, const int *ind, const int *typ, const int *ls, const int *ms,
+                           const double *r, const double *x, const double *y, const double *z, const int *mprox,
+                           int deg, const int *tab_filled, const double *S_knots, const double *S_coefs,
+                           const double *H_knots, const double *H_coefs, int npair, int nsk, int npts,
+                           const double *pos, const int *atype, const double *sigma, double r_lr, const double *XS,
+                           int ldxs, const double *XH, int ldxh, const double *Yg, int ldyg, const double *Ylr,
+                           int ldylr, const double *vrep_knots, const double *vrep_coefs, const double *vrep_dmax,
+                           int nknots, double *grad, void *stream);
+
 /* Repulsive energy per atom, e_atom[i] = 1/2 sum_{j != i} Vrep(R_ij); the sum
  * over atoms is DFTB2.getRepulsiveEnergy (DFTB2.py:2339-2359).  Tables as in
  * dftb_pair_gradients. */
