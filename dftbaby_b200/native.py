@@ -135,8 +135,15 @@ def ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
+# the raw handle of the current stream without building a torch.cuda.Stream (3.4 us a call, a launch takes 2.5);
+# torch.cuda.current_stream() where this torch has no such function
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if _raw_stream is None or not torch.cuda.is_initialized():
+        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
 
 
 def transpose(X):
@@ -196,13 +203,20 @@ class Counters:
 counters = Counters()
 
 
+_functions = {}  # name -> entry point, from its first call (after load() has found a library and a device)
+
+
 def call(name, *args):
-    L = load()
+    f = _functions.get(name)
+    if f is None:
+        f = _functions[name] = getattr(load(), name)
     ev = None
     if counters.timed is not None and name in counters.timed:
         ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
         ev[0].record()
-    check(getattr(L, name)(*args), name)
+    rc = f(*args)
+    if rc != DFTB_OK:
+        check(rc, name)
     if ev is not None:
         ev[1].record()
         counters.timed[name].append(ev)
