@@ -607,166 +607,139 @@ int pick_ksplit(int M, int N, int K) {
 // ----------------------------------------------------------------------------
 // transition charges
 // ----------------------------------------------------------------------------
-__global__ void prefix_kernel(int nat, const int *opa, int *first) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int f = 0;
-        for (int A = 0; A < nat; ++A) {
-            first[A] = f;
-            f += opa[A];
+// first[A] = orbitals before atom A, first[nat] = all of them: one block scans (one thread did, 17 us at 336 atoms)
+constexpr int PREFIX_THREADS = 512;
+
+__global__ void __launch_bounds__(PREFIX_THREADS) prefix_kernel(int nat, const int *opa, int *first) {
+    __shared__ int wsum[PREFIX_THREADS / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int base = 0;
+    for (int A0 = 0; A0 < nat; A0 += PREFIX_THREADS) {
+        const int A = A0 + t, v = A < nat ? opa[A] : 0;
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        first[nat] = f;
-    }
-}
-
-// q[A][p][q] = 1/2 sum_{mu in A} (C1[mu][p] Sc2[mu][q] + C2[mu][q] Sc1[mu][p]).
-// The output (nat x n1 x n2 doubles) is the only large stream, so the kernel is built around writing it at
-// HBM speed: a CTA owns a TC_TP x TC_TQ tile of (p, q) for a run of TC_ATOMS atoms.  Per atom the rows mu of
-// C1, Sc1 (TC_TP wide) and C2, Sc2 (TC_TQ wide) are staged in shared memory by cp.async, one atom ahead
-// (three buffers, so one barrier per atom suffices), and the next atom's rows arrive while the current
-// atom's outputs are stored; every thread writes
-// adjacent pairs of q with 16-byte stores (each warp stores 512 contiguous bytes of one row p).  Atoms with up
-// to TC_MAXO orbitals (s and p shells) take the staged path; larger ones read their rows from global memory.
-constexpr int TC_TP = 64, TC_TQ = 128, TC_THREADS = 256, TC_MAXO = 4, TC_ATOMS = 8, TC_ROWS = 4;
-
-struct TcStage {
-    double c1[TC_MAXO][TC_TP], s1[TC_MAXO][TC_TP], c2[TC_MAXO][TC_TQ], s2[TC_MAXO][TC_TQ];
-};
-
-__device__ __forceinline__ void tc_stage(TcStage &b, int f0, int nA, int n1, int n2, int p0, int q0,
-                                         const double *C1, const double *Sc1, const double *C2,
-                                         const double *Sc2) {
-    for (int i = threadIdx.x; i < nA * TC_TP; i += TC_THREADS) {
-        const int j = i / TC_TP, pp = i % TC_TP, p = p0 + pp;
-        const bool v = p < n1;
-        const size_t o = v ? (size_t)(f0 + j) * n1 + p : 0;
-        cp_async8(&b.c1[j][pp], C1 + o, v);
-        cp_async8(&b.s1[j][pp], Sc1 + o, v);
-    }
-    for (int i = threadIdx.x; i < nA * TC_TQ; i += TC_THREADS) {
-        const int j = i / TC_TQ, qq = i % TC_TQ, qi = q0 + qq;
-        const bool v = qi < n2;
-        const size_t o = v ? (size_t)(f0 + j) * n2 + qi : 0;
-        cp_async8(&b.c2[j][qq], C2 + o, v);
-        cp_async8(&b.s2[j][qq], Sc2 + o, v);
-    }
-}
-
-template <bool VEC>
-__global__ void __launch_bounds__(TC_THREADS) tc_tile_kernel(int nat, int n1, int n2, const int *first,
-                                                             const double *__restrict__ C1,
-                                                             const double *__restrict__ Sc1,
-                                                             const double *__restrict__ C2,
-                                                             const double *__restrict__ Sc2, double *q) {
-    __shared__ __align__(16) TcStage buf[3];
-    const int tid = threadIdx.x;
-    const int qp = tid & 63, pg = tid >> 6;  // q pair within the tile; row group
-    const int q0 = blockIdx.x * TC_TQ, p0 = blockIdx.y * TC_TP;
-    const int qg = q0 + 2 * qp;
-    const int A0 = blockIdx.z * TC_ATOMS;
-    const int A1 = min(nat, A0 + TC_ATOMS);
-    // prologue: stage the first atom
-    {
-        const int f0 = first[A0], nA = first[A0 + 1] - f0;
-        if (nA <= TC_MAXO) tc_stage(buf[0], f0, nA, n1, n2, p0, q0, C1, Sc1, C2, Sc2);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    for (int A = A0; A < A1; ++A) {
-        const int k = A - A0;
-        const int f0 = first[A], nA = first[A + 1] - f0;
-        const bool staged = nA <= TC_MAXO;
-        if (A + 1 < A1) {
-            // next atom's rows into buffer (k + 1) % 3, last read in iteration k - 2: every thread has
-            // passed the barrier of iteration k - 1 since, so those reads are finished
-            const int g0 = first[A + 1], nB = first[A + 2] - g0;
-            if (nB <= TC_MAXO) tc_stage(buf[(k + 1) % 3], g0, nB, n1, n2, p0, q0, C1, Sc1, C2, Sc2);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        if (lane == 31) wsum[warp] = x;
         __syncthreads();
-        const TcStage &sb = buf[k % 3];
-        for (int batch = 0; batch < TC_TP / (4 * TC_ROWS); ++batch) {
-            double acc0[TC_ROWS], acc1[TC_ROWS];
+        int before = base, all = 0;
+        for (int w = 0; w < PREFIX_THREADS / 32; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (A < nat) first[A] = before + x - v;
+        base += all;
+        __syncthreads();
+    }
+    if (t == 0) first[nat] = base;
+}
+
+// q[A][p][q] = 1/2 sum_{mu in A} (C1[mu][p] Sc2[mu][q] + Sc1[mu][p] C2[mu][q]).
+// The output (nat x n1 x n2 doubles) is the only large stream and its rows start at any multiple of 8 bytes.  A warp
+// owns one atom and TC_Q columns, holds the atom's S c and c of those columns as B fragments of the FP64 tensor
+// instruction (K = up to four orbitals, twice) in registers, and walks over blocks of 8 rows p: two loads, 32
+// instructions, and the 8 x TC_Q block goes to the warp's own shared-memory buffer and from there to memory by one
+// asynchronous bulk copy per row, 16-byte aligned, with the odd element of a row's ends stored singly.  Two buffers a
+// warp; no barriers.  Bound by the writes.  (Outputs from registers, 16-byte stores through shuffles, two FP64 units'
+// worth of FMAs each: L1 80 % and FP64 67 % busy, 3.7 TB/s of writes.  B200, C294H42 with 609 x 609 orbitals, 3.0 GB:
+// 747 us so, 530 us here; filling the same memory takes 402 us.)
+constexpr int TC_Q = 128, TC_WARPS = 4, TC_THREADS = 32 * TC_WARPS, TC_BLOCKS = 8;
+// Row pitch of the staging buffer.  Rows that all start on a 16-byte boundary are staged by 16-byte stores, free of
+// bank conflicts at 136; rows of both alignments by 8-byte stores, free of them at 130.
+constexpr int TC_PITCH16 = 136, TC_PITCH8 = 130;
+constexpr int TC_BUF = 8 * TC_PITCH16;
+constexpr int TC_SMEM = TC_WARPS * 2 * TC_BUF * (int)sizeof(double);
+
+__global__ void __launch_bounds__(TC_THREADS, 3) tc_kernel(int n1, int n2, const int *first,
+                                                           const double *__restrict__ C1,
+                                                           const double *__restrict__ Sc1,
+                                                           const double *__restrict__ C2,
+                                                           const double *__restrict__ Sc2, double *q) {
+    extern __shared__ __align__(16) double tc_buf[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kk = lane & 3, rr = lane >> 2;
+    double *buf = tc_buf + warp * 2 * TC_BUF;
+    const int A = blockIdx.z, q0 = blockIdx.x * TC_Q, ncols = min(TC_Q, n2 - q0);
+    const int f0 = first[A], nA = first[A + 1] - f0;
+    const int nblocks = (n1 + 7) / 8, stride = gridDim.y * TC_WARPS;
+    double *qA = q + (size_t)A * n1 * n2 + q0;
+    const bool vec = (n2 & 1) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+    const int pitch = vec ? TC_PITCH16 : TC_PITCH8;
+    // one value of a (norb x n) matrix, zero outside
+    auto at = [&](const double *X, int n, int j, int c) {
+        return j < nA && c < n ? __ldg(X + (size_t)(f0 + j) * n + c) : 0.0;
+    };
+    double bs[TC_Q / 8], bc[TC_Q / 8];
 #pragma unroll
-            for (int r = 0; r < TC_ROWS; ++r) acc0[r] = acc1[r] = 0.0;
-            // this thread's rows: TC_ROWS consecutive ones, so that the staged C1 / Sc1 values of two rows
-            // come in one 16-byte shared-memory read (the same address for the whole warp: a broadcast)
-            const int pl0 = (batch * 4 + pg) * TC_ROWS;
-            if (staged) {
-                for (int j = 0; j < nA; ++j) {
-                    const double2 c2 = *reinterpret_cast<const double2 *>(&sb.c2[j][2 * qp]);
-                    const double2 s2 = *reinterpret_cast<const double2 *>(&sb.s2[j][2 * qp]);
+    for (int t = 0; t < TC_Q / 8; ++t) {
+        bs[t] = at(Sc2, n2, kk, q0 + 8 * t + rr);
+        bc[t] = at(C2, n2, kk, q0 + 8 * t + rr);
+    }
+    int pb = blockIdx.y * TC_WARPS + warp;
+    double ac = at(C1, n1, kk, 8 * pb + rr), as = at(Sc1, n1, kk, 8 * pb + rr);
+    for (int step = 0; pb < nblocks; pb += stride, ++step) {
+        double *out = buf + (step & 1) * TC_BUF;
+        const int p0 = 8 * pb;
+        const double ac0 = 0.5 * ac, as0 = 0.5 * as;
+        ac = at(C1, n1, kk, p0 + 8 * stride + rr);  // the next block's
+        as = at(Sc1, n1, kk, p0 + 8 * stride + rr);
+        // the copies issued two steps ago have read this buffer
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+        const int phase = (int)((reinterpret_cast<uintptr_t>(qA + (size_t)(p0 + rr) * n2) >> 3) & 1);
+        double *o = out + rr * pitch + phase + 2 * kk;
 #pragma unroll
-                    for (int r = 0; r < TC_ROWS; r += 2) {
-                        const double2 a1 = *reinterpret_cast<const double2 *>(&sb.c1[j][pl0 + r]);
-                        const double2 b1 = *reinterpret_cast<const double2 *>(&sb.s1[j][pl0 + r]);
-                        acc0[r] += a1.x * s2.x + c2.x * b1.x;
-                        acc1[r] += a1.x * s2.y + c2.y * b1.x;
-                        acc0[r + 1] += a1.y * s2.x + c2.x * b1.y;
-                        acc1[r + 1] += a1.y * s2.y + c2.y * b1.y;
-                    }
-                }
-            } else {
-                for (int j = 0; j < nA; ++j) {
-                    const size_t r2 = (size_t)(f0 + j) * n2;
-                    const double c2a = qg < n2 ? C2[r2 + qg] : 0.0, s2a = qg < n2 ? Sc2[r2 + qg] : 0.0;
-                    const double c2b = qg + 1 < n2 ? C2[r2 + qg + 1] : 0.0;
-                    const double s2b = qg + 1 < n2 ? Sc2[r2 + qg + 1] : 0.0;
-#pragma unroll
-                    for (int r = 0; r < TC_ROWS; ++r) {
-                        const int p = p0 + pl0 + r;
-                        const size_t r1 = (size_t)(f0 + j) * n1 + p;
-                        const double a1 = p < n1 ? C1[r1] : 0.0, b1 = p < n1 ? Sc1[r1] : 0.0;
-                        acc0[r] += a1 * s2a + c2a * b1;
-                        acc1[r] += a1 * s2b + c2b * b1;
-                    }
-                }
+        for (int t = 0; t < TC_Q / 8; ++t) {
+            if (8 * t >= ncols) break;
+            double d0 = 0.0, d1 = 0.0;
+            dmma884(d0, d1, ac0, bs[t]);
+            dmma884(d0, d1, as0, bc[t]);
+            for (int j = 4; j < nA; j += 4) {  // atoms with d shells: the further orbitals, four at a time
+                dmma884(d0, d1, 0.5 * at(C1, n1, j + kk, p0 + rr), at(Sc2, n2, j + kk, q0 + 8 * t + rr));
+                dmma884(d0, d1, 0.5 * at(Sc1, n1, j + kk, p0 + rr), at(C2, n2, j + kk, q0 + 8 * t + rr));
             }
-#pragma unroll
-            for (int r = 0; r < TC_ROWS; ++r) {
-                const int p = p0 + pl0 + r;  // the same for the whole warp
-                if (p >= n1) continue;
-                double *row = q + ((size_t)A * n1 + p) * n2;
-                if (VEC) {
-                    // 16-byte stores on every row: a row whose tile segment starts on an odd element (odd n2)
-                    // stores the pairs (qg + 1, qg + 2), the second value taken from the next lane; lane 0
-                    // stores its first column and lane 31 its second as single elements
-                    const int lane = tid & 31;
-                    const double nxt = __shfl_down_sync(0xffffffffu, acc0[r], 1);
-                    const bool odd = (reinterpret_cast<uintptr_t>(row + q0) & 15) != 0;  // warp-uniform
-                    if (!odd) {
-                        if (qg + 1 < n2)
-                            *reinterpret_cast<double2 *>(row + qg) = make_double2(0.5 * acc0[r], 0.5 * acc1[r]);
-                        else if (qg < n2)
-                            row[qg] = 0.5 * acc0[r];
-                    } else {
-                        if (lane == 0 && qg < n2) row[qg] = 0.5 * acc0[r];
-                        if (lane < 31 && qg + 2 < n2)
-                            *reinterpret_cast<double2 *>(row + qg + 1) = make_double2(0.5 * acc1[r], 0.5 * nxt);
-                        else if (qg + 1 < n2)
-                            row[qg + 1] = 0.5 * acc1[r];
-                    }
-                } else {
-                    if (qg >= n2) continue;
-                    row[qg] = 0.5 * acc0[r];
-                    if (qg + 1 < n2) row[qg + 1] = 0.5 * acc1[r];
-                }
+            if (vec) {
+                *reinterpret_cast<double2 *>(o + 8 * t) = make_double2(d0, d1);
+            } else {
+                o[8 * t] = d0;
+                o[8 * t + 1] = d1;
             }
         }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        // lanes 0..7: the 16-byte aligned part of row lane; 8..15 an odd first element, 16..23 an odd last one
+        const int r = lane & 7;
+        if (p0 + r < n1) {
+            double *dst = qA + (size_t)(p0 + r) * n2;
+            const int head = (int)((reinterpret_cast<uintptr_t>(dst) >> 3) & 1), body = (ncols - head) & ~1;
+            const double *src = out + r * pitch + head;
+            if (lane < 8) {
+                if (body > 0)
+                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + head),
+                                 "r"(static_cast<uint32_t>(__cvta_generic_to_shared(src + head))), "r"(body * 8)
+                                 : "memory");
+            } else if (lane < 16) {
+                if (head) dst[0] = src[0];
+            } else if (lane < 24) {
+                if (head + body < ncols) dst[ncols - 1] = src[ncols - 1];
+            }
+        }
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // one (n1 x n2) block of transition charges for all atoms
 int launch_tc(int nat, int n1, int n2, const int *first, const double *C1, const double *Sc1, const double *C2,
               const double *Sc2, double *out, cudaStream_t st, const char *where) {
-    dim3 grid(cdiv(n2, TC_TQ), cdiv(n1, TC_TP), cdiv(nat, TC_ATOMS));
+    // about TC_BLOCKS row blocks a warp: enough to pay for its B fragments, few enough to fill the GPU (609 x 609 orbitals,
+    // 336 atoms: 552, 530, 543 and 582 us with 4, 8, 16 and 32)
+    dim3 grid(cdiv(n2, TC_Q), cdiv(cdiv(n1, 8), TC_WARPS * TC_BLOCKS), nat);
     if (grid.y > 65535u || grid.z > 65535u) return fail(DFTB_ERR_BAD_SIZE, "trans_charges: grid too large");
-    // 16-byte stores need an aligned base; rows that start on an odd element shift their pairs by one
-    if (((uintptr_t)out & 15) == 0)
-        tc_tile_kernel<true><<<grid, TC_THREADS, 0, st>>>(nat, n1, n2, first, C1, Sc1, C2, Sc2, out);
-    else
-        tc_tile_kernel<false><<<grid, TC_THREADS, 0, st>>>(nat, n1, n2, first, C1, Sc1, C2, Sc2, out);
+    cudaError_t e = cudaFuncSetAttribute(tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+    if (e != cudaSuccess) return fail(DFTB_ERR_CUDA, "trans_charges: shared memory");
+    tc_kernel<<<grid, TC_THREADS, TC_SMEM, st>>>(n1, n2, first, C1, Sc1, C2, Sc2, out);
     return check_launch(where);
 }
 
@@ -844,7 +817,7 @@ int trans_charges_common(int norb, int nat, int nocc, int nvirt, const double *c
     *scv = (double *)w;
     w += align256(sizeof(double) * (size_t)norb * nvirt);
     *first = (int *)w;
-    prefix_kernel<<<1, 1, 0, st>>>(nat, opa, *first);
+    prefix_kernel<<<1, PREFIX_THREADS, 0, st>>>(nat, opa, *first);
     int rc = check_launch("prefix_kernel");
     if (rc) return rc;
     // Sc = S . C (S is symmetric)
@@ -1338,7 +1311,7 @@ int dftb_trans_charges(int norb, int nat, int nocc, int nvirt, const double *co,
                  {q_vv, cv, scv, cv, scv, nvirt, nvirt}};
     for (auto &b : blks) {
         if (!b.out || b.n1 == 0 || b.n2 == 0) continue;
-        if ((rc = launch_tc(nat, b.n1, b.n2, first, b.c1, b.s1, b.c2, b.s2, b.out, st, "tc_tile_kernel")))
+        if ((rc = launch_tc(nat, b.n1, b.n2, first, b.c1, b.s1, b.c2, b.s2, b.out, st, "tc_kernel")))
             return rc;
     }
     return DFTB_OK;
