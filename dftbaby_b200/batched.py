@@ -33,7 +33,7 @@ run on batched device tensors.
 import numpy as np
 import torch
 
-from . import native
+from . import eigen, native
 from .exceptions import ExcitedStatesError, ExcitedStatesNotConverged, SCFNotConverged
 from .params import Parametrization
 
@@ -79,18 +79,23 @@ def _native_batched_eigh(A):
 
 
 def batched_eigh(A, workers=16):
-    """Eigen-decomposition of a batch of symmetric matrices: one batched cuSOLVER call where the
-    library provides it, else torch.linalg.eigh spread over host threads with one CUDA stream each
+    """Eigen-decomposition of a batch of symmetric matrices: the library's own kernel for small ones, one batched
+    cuSOLVER call where that library provides it, else torch.linalg.eigh spread over host threads with one CUDA stream each
     (the dense solver runs one matrix at a time and is bound by launch and synchronisation latency at
     these sizes; independent streams let the solves of different matrices overlap)."""
     global _POOL
     B = A.shape[0]
+    if B > 1 and eigen.small(A):
+        w, V, info = eigen.small_eigh(A)
+        if bool(info.any()):
+            raise ExcitedStatesError("batched eigensolver did not converge for %d matrices" % int((info != 0).sum()))
+        return w, V
     if A.device.type == "cuda" and B > 1:
         out = _native_batched_eigh(A)
         if out is not None:
             return out
     if B < 2 * workers or A.device.type != "cuda":
-        return torch.linalg.eigh(A)
+        return eigen.eigh(A)
     from concurrent.futures import ThreadPoolExecutor
     if _POOL is None:
         # torch loads its eigensolver wrapper lazily; that must not race between the pool's threads

@@ -9,11 +9,7 @@
 // 1500625, 10 columns without the square roots: T 2.60 ms, G 5.8 us, us 2.33 ms (13.2 GB, 2.03 ms).
 #pragma once
 
-__device__ __forceinline__ void dmma884(double &c0, double &c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
+#include "dmma.cuh"
 
 __device__ __forceinline__ void cp_async8(void *dst, const double *src, bool valid) {
     // 8-byte asynchronous copy; with src-size 0 the destination is zero-filled and nothing is read

@@ -18,7 +18,7 @@ import re
 import numpy as np
 import torch
 
-from . import native
+from . import eigen, native
 from .exceptions import SCFChargeInconsistency, SCFNotConverged
 from .params import ELEMENT_NAMES, Parametrization, raw_params
 
@@ -508,14 +508,14 @@ class DFTB2(object):
                     Hm = mm(mm(B.T, Hk), B)
                     virt = torch.nonzero(self.f == 0.0).flatten()
                     Hm[virt, virt] += b
-                    self.orbe, Cp = torch.linalg.eigh(Hm)
+                    self.orbe, Cp = eigen.eigh(Hm)
                     self.orbs = mm(B, Cp)
                 else:
                     # L^-1 Hk L^-T and L^-T C' by triangular solves (n^3 FLOPs each instead of the
                     # 2 n^3 of a product with an explicit inverse); eigh reads the lower triangle
                     Y = torch.linalg.solve_triangular(self._L, Hk, upper=False)
                     Hp = torch.linalg.solve_triangular(self._L, Y.mT, upper=False).mT
-                    self.orbe, Cp = torch.linalg.eigh(Hp)
+                    self.orbe, Cp = eigen.eigh(Hp)
                     self.orbs = torch.linalg.solve_triangular(self._L.mT, Cp, upper=True)
                 have_orbe = True
                 self.f = self._occupation(self.orbe)

@@ -33,7 +33,7 @@ import os
 import numpy as np
 import torch
 
-from . import native, tcgemm
+from . import eigen, native, tcgemm
 
 NFEAT = 8
 FPAD = 64
@@ -359,7 +359,7 @@ def dense_start(net, td, nstates, block=24, extra=8, frontier=False):
     if d.long_range_correction == 1:
         A = A - torch.einsum("Aij,AB,Bab->iajb", q_oo, d.gamma_lr, q_vv).reshape(n, n)
     A = A + torch.diag(td.omega[oi][:, vi].reshape(-1))
-    Om, X = torch.linalg.eigh(0.5 * (A + A.T))
+    Om, X = eigen.eigh(0.5 * (A + A.T))
     Om = Om[:nstates].clamp_min(1e-6)
     T = torch.zeros((nstates, no, nv), dtype=torch.float64, device=d.device)
     T[:, oi[:, None], vi[None, :]] = X[:, :nstates].T.reshape(nstates, bo, bv)

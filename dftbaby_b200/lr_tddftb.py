@@ -26,7 +26,7 @@ q_vv.  The Coulomb term uses q_ov and the native product kernels.
 import numpy as np
 import torch
 
-from . import native
+from . import eigen, native
 from .dftb2 import DFTB2
 from .exceptions import ExcitedStatesError, ExcitedStatesNotConverged
 from .params import raw_params
@@ -643,12 +643,12 @@ class LR_TDDFTB:
         if offdiag < 1.0e-10:
             sq = torch.diag(torch.sqrt(torch.diag(AmB)))
         else:
-            lam, V = torch.linalg.eigh(0.5 * (AmB + AmB.T))
+            lam, V = eigen.eigh(0.5 * (AmB + AmB.T))
             sq = (V * torch.sqrt(lam)) @ V.T
         R = sq @ (A + B) @ sq
         if torch.linalg.norm(R - R.T).item() >= 1.0e-10:
             raise ExcitedStatesError("TD-DFTB matrix not hermitian")
-        O2, F = torch.linalg.eigh(R)
+        O2, F = eigen.eigh(R)
         Om = torch.sqrt(O2)
         XpY = (sq @ F) / torch.sqrt(Om)
         XmY = ((A + B) @ XpY) / Om

@@ -34,6 +34,7 @@ _P = ctypes.c_void_p
 _I = ctypes.c_int
 _D = ctypes.c_double
 _Z = ctypes.c_size_t
+_L = ctypes.c_longlong
 
 _SIGNATURES = {
     "dftb_version": (ctypes.c_char_p, []),
@@ -91,6 +92,7 @@ _SIGNATURES = {
     "dftb_batched_eigh_workspace_size": (_I, [_I, _I, ctypes.POINTER(_Z)]),
     "dftb_batched_eigh": (_I, [_I, _I, _P, _P, _P, _Z, _P, _P]),
     "dftb_eigh_last_error": (ctypes.c_char_p, []),
+    "dftb_small_eigh": (_I, [_I, _I, _P, _L, _L, _L, _P, _P, _P, _P]),
     "dftb_solver_workspace_size": (_Z, [_I, _I, _I, _I, _I]),
     "dftb_solver_create": (_I, [_I, _I, _I, _I, _I, _P, _Z, ctypes.POINTER(_P)]),
     "dftb_solver_solve_hermitian": (_I, [_P, _P, _P, _P, _D, _I, _I, _P, _P, _P, _P, ctypes.POINTER(_I), _P]),

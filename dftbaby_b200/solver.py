@@ -24,7 +24,7 @@ are FP64 on the device.
 import numpy as np
 import torch
 
-from . import native
+from . import eigen, native
 from .exceptions import ExcitedStatesError, ExcitedStatesNotConverged
 
 
@@ -231,7 +231,7 @@ def hermitian_davidson(rv, omega, nstates, ifact=1, conv=1.0e-14, maxiter=10, Xp
     for it in range(maxiter):
         bs, AB = B.bs, B.prod(0)
         Hb = B.M[0]
-        w2, Tb = torch.linalg.eigh(Hb)
+        w2, Tb = eigen.eigh(Hb)
         if L2_thresh > 0.0 and Oia is not None:
             T_all = bs @ Tb
             L2 = torch.sum(T_all * T_all * Oia.reshape(-1, 1), dim=0).cpu().numpy()
@@ -271,7 +271,7 @@ def hermitian_davidson(rv, omega, nstates, ifact=1, conv=1.0e-14, maxiter=10, Xp
 
 def _sqrtm_spd(M):
     """Principal square root of the symmetric positive definite subspace matrix."""
-    lam, V = torch.linalg.eigh(0.5 * (M + M.T))
+    lam, V = eigen.eigh(0.5 * (M + M.T))
     if bool((lam <= 0.0).any()):
         raise ExcitedStatesError("(A-B) projected onto the expansion space is not positive definite")
     return (V * torch.sqrt(lam)) @ V.T
@@ -288,7 +288,7 @@ def _ssf_cholesky(Mp, Mm):
         return None
     Mh = Lc.T @ Mp @ Lc
     asym = torch.sum(torch.abs(Mh - Mh.T)).item()
-    w2, Tp = torch.linalg.eigh(0.5 * (Mh + Mh.T))
+    w2, Tp = eigen.eigh(0.5 * (Mh + Mh.T))
     w = torch.sqrt(w2)
     Rb = (Lc @ Tp) / torch.sqrt(w)
     Lb = (Mp @ Rb) / w
@@ -358,7 +358,7 @@ def nonhermitian_davidson(products, omega, nstates, ifact=1, conv=1.0e-14, maxit
                 Mmsq = _sqrtm_spd(Mm)
                 Mh = Mmsq @ Mp @ Mmsq
                 asym = torch.sum(torch.abs(Mh - Mh.T)).item()
-                w2, Tb = torch.linalg.eigh(Mh)
+                w2, Tb = eigen.eigh(Mh)
                 w = torch.sqrt(w2)
                 Rb = (Mmsq @ Tb) / torch.sqrt(w)
                 Lb = (Mp @ Rb) / w
@@ -437,7 +437,7 @@ def nonhermitian_davidson(products, omega, nstates, ifact=1, conv=1.0e-14, maxit
         if Tb is None:
             # eigenvectors of the (A-B)^1/2 (A+B) (A-B)^1/2 form, DFTBaby's C: Tb = (Mm)^-1/2 L T'
             Mm_last, Lc, Tp = chol
-            lam, U = torch.linalg.eigh(0.5 * (Mm_last + Mm_last.T))
+            lam, U = eigen.eigh(0.5 * (Mm_last + Mm_last.T))
             Tb = (U / torch.sqrt(lam)) @ (U.T @ (Lc @ Tp[:, :k]))
         C = bs @ Tb[:, :k]
     shape = (k, nocc, nvirt)
@@ -450,7 +450,7 @@ def _ssf_ritz(Mp, Mm):
     Mp = 0.5 * (Mp + Mp.T)
     Mmsq = _sqrtm_spd(Mm)
     Mh = Mmsq @ Mp @ Mmsq
-    w2, Tb = torch.linalg.eigh(0.5 * (Mh + Mh.T))
+    w2, Tb = eigen.eigh(0.5 * (Mh + Mh.T))
     if bool((w2 <= 0.0).any()):
         raise ExcitedStatesError("the projected problem has a non-positive eigenvalue")
     w = torch.sqrt(w2)

@@ -425,6 +425,14 @@ int dftb_batched_eigh_workspace_size(int n, int batch, size_t *bytes);
 int dftb_batched_eigh(int n, int batch, double *A, double *W, void *work, size_t work_bytes, int *info, void *stream);
 const char *dftb_eigh_last_error(void);
 
+/* Small matrices, n <= DFTB_SMALL_EIGH_MAX: the whole batch in one launch of the library's own kernel, without a workspace.
+ * Matrix b, element (i, j) at A[b * batch_stride + i * row_stride + j * col_stride]; the lower triangle is read.  W:
+ * batch x n eigenvalues, ascending; V: batch x n x n, eigenvector j of matrix b in row j of block b (V may be A when A is
+ * contiguous); info: batch status words, 0 or 1 (the matrix holds a number that is not finite; W and V are NaN). */
+#define DFTB_SMALL_EIGH_MAX 128
+int dftb_small_eigh(int n, int batch, const double *A, long long batch_stride, long long row_stride, long long col_stride,
+                    double *W, double *V, int *info, void *stream);
+
 /* ---- the fused device solve ------------------------------------------------------
  * Replaces the Davidson branch of LR_TDDFTB._solve_lr_equations (DFTB/LR_TDDFTB.py:403-527)
  * for the problem without long-range correction, Solver.HermitianDavidson
