@@ -13,11 +13,13 @@
 //      Li (1993), bracketed, four lanes a root; vectors from the recomputed z of Gu and Eisenstat (1994), which keeps
 //      them orthogonal without extended precision; their product with the old vectors by FP64 tensor instructions, a
 //      warp owning 8 rows, so that it is done in place.
-//   3. The reflectors are applied to the columns, which four lanes each hold in registers; no barriers.
+//   3. The reflectors are applied in blocks of eight by FP64 tensor instructions, a warp owning 8 columns; no barriers.
 //
-// Bound by the latency of its serial steps, not by a unit.  B200, host included, against torch.linalg.eigh: n = 20 0.26
-// -> 0.11 ms, 42 0.70 -> 0.17, 64 0.94 -> 0.21, 102 1.75 -> 0.41, 128 2.11 -> 0.50; batches of 256 against cuSOLVER's
-// batched call: n = 20 0.34 -> 0.12 ms, 64 1.08 -> 0.38, 128 3.30 -> 0.96.  Residuals and orthogonality as the library's.
+// Bound by its serial steps and by instruction issue on one SM (n = 102: tridiagonalisation 266k cycles, divide and
+// conquer 249k, reflectors 42k; applying these one at a time from columns in registers took 184k).  B200, host
+// included, against torch.linalg.eigh: n = 20 0.26 -> 0.11 ms, 42 0.70 -> 0.15, 64 0.94 -> 0.19, 102 1.75 -> 0.34, 128
+// 2.11 -> 0.39; batches of 256 against cuSOLVER's batched call: n = 20 0.34 -> 0.12 ms, 64 1.08 -> 0.33, 128 3.28 ->
+// 0.75.  Residuals and orthogonality as the library's.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <math_constants.h>
@@ -45,7 +47,8 @@ struct Layout {
 
 template <int NC> struct Vectors {
     static constexpr int N = 32 * NC;
-    double d[N], e[N], tau[N], zs[N], ds[N], kd[N], kz[N], zh[N], x[N], scale[N];
+    double d[N], tau[N];
+    double e[N], zs[N], ds[N], kd[N], kz[N], zh[N], x[N], scale[N];  // step 3: 8 x 8 matrices of the reflector blocks
     double rho[N / 2];
     double red[4 * NC];
     int ord[N], slot[N], org[N], typ[N], top[N], bot[N];
@@ -77,17 +80,15 @@ template <int M> __device__ __forceinline__ double warp_sums(double (&v)[8]) {
     return s;
 }
 
-// sum / product over the four lanes that share a column or a root; they are always converged
+// sum / product over the four lanes that share a column or a root; called by whole warps
 __device__ __forceinline__ double quad_sum(double v) {
-    const unsigned m = 0xfu << (threadIdx.x & 28);
-    v += __shfl_xor_sync(m, v, 1);
-    return v + __shfl_xor_sync(m, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
 __device__ __forceinline__ double quad_product(double v) {
-    const unsigned m = 0xfu << (threadIdx.x & 28);
-    v *= __shfl_xor_sync(m, v, 1);
-    return v * __shfl_xor_sync(m, v, 2);
+    v *= __shfl_xor_sync(0xffffffffu, v, 1);
+    return v * __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
 // The root (a - s) / (2 c) of c t^2 - a t + b, s = sqrt(a^2 - 4 b c) (last: the root (a + s) / (2 c)), without
@@ -99,75 +100,73 @@ __device__ __forceinline__ double quadratic(double c, double a, double b, bool l
 }
 
 // Root j of 1/rho + sum_i z_i^2 / (d_i - lambda) (K poles d ascending, |z| = 1 at most) as lambda = d[origin] + x, the
-// origin being the nearer pole, so that d_i - lambda is known to full relative precision for every i.  Called by the
-// four lanes of a quad; lane q sums the terms q, q + 4, ...
-__device__ void secular_root(int K, int j, const double *d, const double *z, double rho, int q, int *origin, double *xout) {
+// origin being the nearer pole, so that d_i - lambda is known to full relative precision for every i.  A quad of lanes a
+// root, lane q summing the terms q, q + 4, ...; the warp's eight quads (of up to Kw poles each) iterate in step.  live: this quad has a root.
+__device__ void secular_roots(bool live, int K, int Kw, int j, const double *d, const double *z, double rho, int q,
+                              int *origin, double *xout) {
     const double ri = 1.0 / rho;
-    if (K == 1) {
-        *origin = 0;
-        *xout = rho * z[0] * z[0];
-        return;
-    }
+    const bool single = K < 2;
     const bool last = j == K - 1;
-    const int jl = last ? K - 2 : j, jr = jl + 1;  // the two poles of the interpolation
-    // psi sums the terms up to jl, phi those from jr on
-    double lo, hi, x;
-    int org;
-    {
-        // the value half way decides the origin; the terms of the two poles, exact, give the first x
-        const double base = last ? d[K - 1] : d[j];
-        const double len = last ? rho : d[j + 1] - d[j];
-        const double mid = 0.5 * len;
-        double rest = 0.0;
-        for (int i = q; i < K; i += 4)
-            if (i != jl && i != jr) rest += z[i] * z[i] / ((d[i] - base) - mid);
-        const double c = ri + quad_sum(rest);
-        const double zl = z[jl] * z[jl], zr = z[jr] * z[jr];
-        const double w = c + zl / ((d[jl] - base) - mid) + zr / ((d[jr] - base) - mid);
-        org = last ? K - 1 : (w >= 0.0 ? j : j + 1);
-        const double dl = d[jl] - d[org], dr = d[jr] - d[org];
-        if (last) {
-            lo = w <= 0.0 ? mid : 0.0;
-            hi = w <= 0.0 ? len * (1.0 + 64.0 * EPS) : mid;  // |z| = 1 up to roundoff
-        } else {
-            lo = w >= 0.0 ? 0.0 : -mid;
-            hi = w >= 0.0 ? mid : 0.0;
-        }
-        x = quadratic(c, c * (dl + dr) + zl + zr, c * dl * dr + zl * dr + zr * dl, last);
-        if (!(x > lo && x < hi)) x = 0.5 * (lo + hi);
+    const int jl = single ? 0 : (last ? K - 2 : j), jr = single ? 0 : jl + 1;  // the two poles of the interpolation
+    const double o0 = d[j], len = last ? rho : d[jr] - o0, mid = 0.5 * len;
+    // the value half way decides the origin; the terms of the two poles, exact, give the first x
+    double c = 0.0;
+    for (int i0 = 0; i0 < Kw; i0 += 8) {  // two terms share a division
+        const int i = min(i0 + q, K - 1), i2 = min(i0 + q + 4, K - 1);
+        const double z1 = i0 + q < K && i != jl && i != jr ? z[i] : 0.0, z2 = i0 + q + 4 < K && i2 != jl && i2 != jr ? z[i2] : 0.0;
+        const double a = (d[i] - o0) - mid, b = (d[i2] - o0) - mid, r = 1.0 / (a * b);
+        c += z1 * z1 * (b * r) + z2 * z2 * (a * r);
     }
+    c = ri + quad_sum(c);
+    const double zl = z[jl] * z[jl], zr = z[jr] * z[jr];
+    const double wm = c + zl / ((d[jl] - o0) - mid) + zr / ((d[jr] - o0) - mid);
+    const int org = last ? j : (wm >= 0.0 ? j : jr);
     const double o = d[org], dl = d[jl] - o, dr = d[jr] - o;
+    double lo, hi;
+    if (last) {
+        lo = wm <= 0.0 ? mid : 0.0;
+        hi = wm <= 0.0 ? len * (1.0 + 64.0 * EPS) : mid;  // |z| = 1 up to roundoff
+    } else {
+        lo = wm >= 0.0 ? 0.0 : -mid;
+        hi = wm >= 0.0 ? mid : 0.0;
+    }
+    double x = quadratic(c, c * (dl + dr) + zl + zr, c * dl * dr + zl * dr + zr * dl, last);
+    if (!(x > lo && x < hi)) x = 0.5 * (lo + hi);
+    if (single) x = rho * z[0] * z[0];
+    bool done = !live || single;
     for (int it = 0; it < SECULAR_ITERATIONS; ++it) {
-        double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
-        for (int i = q; i < K; i += 4) {
-            const double t = z[i] / ((d[i] - o) - x);
-            if (i <= jl) {
-                psi += z[i] * t;
-                dpsi += t * t;
-            } else {
-                phi += z[i] * t;
-                dphi += t * t;
-            }
+        if (__all_sync(0xffffffffu, done)) break;
+        double psi = 0.0, dpsi = 0.0, all = 0.0, dw = 0.0;  // the terms up to jl, and all of them
+        for (int i0 = 0; i0 < Kw; i0 += 8) {
+            const int i = min(i0 + q, K - 1), i2 = min(i0 + q + 4, K - 1);
+            const double z1 = i0 + q < K ? z[i] : 0.0, z2 = i0 + q + 4 < K ? z[i2] : 0.0;
+            const double a = (d[i] - o) - x, b = (d[i2] - o) - x, r = 1.0 / (a * b);
+            const double t1 = z1 * (b * r), t2 = z2 * (a * r);
+            const double l1 = i <= jl ? t1 : 0.0, l2 = i2 <= jl ? t2 : 0.0;
+            all += z1 * t1 + z2 * t2;
+            dw += t1 * t1 + t2 * t2;
+            psi += z1 * l1 + z2 * l2;
+            dpsi += l1 * l1 + l2 * l2;
         }
         psi = quad_sum(psi);
-        phi = quad_sum(phi);
+        all = quad_sum(all);
         dpsi = quad_sum(dpsi);
-        dphi = quad_sum(dphi);
-        const double w = ri + psi + phi, dw = dpsi + dphi;
-        if (fabs(w) <= EPS * (ri + 8.0 * (fabs(psi) + fabs(phi)) + fabs(x) * dw)) break;
-        if (w < 0.0)
-            lo = x;
-        else
-            hi = x;
+        dw = quad_sum(dw);
+        const double phi = all - psi, dphi = fmax(dw - dpsi, 0.0), w = ri + all;
+        done = done || fabs(w) <= EPS * (ri + 8.0 * (fabs(psi) + fabs(phi)) + fabs(x) * dw);
+        lo = w < 0.0 ? x : lo;
+        hi = w < 0.0 ? hi : x;
         const double tl = dl - x, tr = dr - x;
-        double c = w - tl * dpsi - tr * dphi;
-        if (last) c = fabs(c);
-        double eta = quadratic(c, (tl + tr) * w - tl * tr * dw, tl * tr * w, last);
+        const double cc = w - tl * dpsi - tr * dphi;
+        double eta = quadratic(last ? fabs(cc) : cc, (tl + tr) * w - tl * tr * dw, tl * tr * w, last);
         if (!(w * eta < 0.0)) eta = -w / dw;
         double xn = x + eta;
+        // a step this short against the distances to the poles is the last: its error is of second order in them
+        const bool short_step = fabs(eta) <= 1e-9 * fmin(fabs(tl), fabs(tr));
         if (!(xn > lo && xn < hi)) xn = 0.5 * (lo + hi);
-        if (xn == x || !(xn > lo && xn < hi)) break;  // the bracket has no number left inside
-        x = xn;
+        const bool full = xn == x || !(xn > lo && xn < hi);  // the bracket has no number left inside
+        if (!done && !full) x = xn;
+        done = done || full || short_step;
     }
     *origin = org;
     *xout = x;
@@ -243,14 +242,15 @@ __device__ int deflate(Vectors<NC> &sv, double *Z, int zp, int off, int s, doubl
     return K;
 }
 
-// the kept columns of one merge with elements in its upper (bit 1) or lower (bit 2) rows, as lists
+// the kept columns of one merge with elements in its upper (bit 1) or lower (bit 2) rows (bits 3: all), as lists of
+// pole | slot << 8
 template <int NC> __device__ int column_list(const Vectors<NC> &sv, int *list, int off, int K, int bit) {
     const int lane = threadIdx.x & 31;
     int n = 0;
     for (int c = 0; c < K; c += 32) {
         const bool in = c + lane < K && (sv.typ[sv.slot[off + c + lane]] & bit);
         const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (in) list[off + n + __popc(m & ((1u << lane) - 1))] = c + lane;
+        if (in) list[off + n + __popc(m & ((1u << lane) - 1))] = (c + lane) | sv.slot[off + c + lane] << 8;
         n += __popc(m);
     }
     return n;
@@ -313,56 +313,62 @@ __global__ void __launch_bounds__(128 * NC, 1)
         for (int c = 0; c < NC; ++c) a[r][c] *= down;
 
     double *hv = U, *hp = U + 2 * N;  // reflector and A v, two buffers each
+    // reflector k, H = 1 - tau v v^T, from row k of the reduced matrix (held by one warp): v = x - beta e_(k+1)
+    auto publish = [&](const double (&row)[NC], int k) {
+        double dk = 0.0, alpha = 0.0, sigma = 0.0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const double dd = __shfl_sync(0xffffffffu, row[c], k & 31);
+            const double aa = __shfl_sync(0xffffffffu, row[c], (k + 1) & 31);
+            if (c == k / 32) dk = dd;
+            if (c == (k + 1) / 32) alpha = aa;
+            if (lane + 32 * c > k + 1) sigma += row[c] * row[c];
+        }
+        sigma = warp_sum(sigma);
+        // elements below 1e-140 of the largest one are dropped: their squares underflow
+        const bool flat = !(sigma > 1e-280);
+        const double beta = flat ? alpha : -copysign(sqrt(alpha * alpha + sigma), alpha);
+        double *v = hv + (k & 1) * N;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int j = lane + 32 * c;
+            const double x = flat || j <= k ? 0.0 : (j == k + 1 ? alpha - beta : row[c]);
+            v[j] = x;
+            if (j > k && j < n) V[(size_t)k * n + j] = x;  // kept for step 3
+        }
+        if (lane == 0) {
+            sv.d[k] = dk;
+            sv.e[k] = beta;
+            sv.tau[k] = flat ? 0.0 : 1.0 / (beta * (beta - alpha));
+        }
+    };
+    if (n > 2 && warp == 0) publish(a[0], 0);
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
+        const int C0 = WARPS * r / 32;  // columns 32 C0 and earlier rows are done
         for (int t = 0; t < WARPS; ++t) {
             const int k = WARPS * r + t;
             if (k >= n - 2) break;
-            double *v = hv + (k & 1) * N, *p = hp + (k & 1) * N;
-            if (warp == t) {
-                double dk = 0.0, alpha = 0.0, sigma = 0.0;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int j = lane + 32 * c;
-                    const double dd = __shfl_sync(0xffffffffu, a[r][c], k & 31);
-                    const double aa = __shfl_sync(0xffffffffu, a[r][c], (k + 1) & 31);
-                    if (c == k / 32) dk = dd;
-                    if (c == (k + 1) / 32) alpha = aa;
-                    if (j > k + 1) sigma += a[r][c] * a[r][c];
-                }
-                sigma = warp_sum(sigma);
-                double beta = alpha, tau = 0.0, scale = 0.0;
-                if (sigma > 0.0) {
-                    beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
-                    tau = (beta - alpha) / beta;
-                    scale = 1.0 / (alpha - beta);
-                }
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int j = lane + 32 * c;
-                    const double x = j > k + 1 ? a[r][c] * scale : (j == k + 1 ? 1.0 : 0.0);
-                    v[j] = x;
-                    if (j > k && j < n) V[(size_t)k * n + j] = x;  // kept for step 3
-                }
-                if (lane == 0) {
-                    sv.d[k] = dk;
-                    sv.e[k] = beta;
-                    sv.tau[k] = tau;
-                }
-            }
+            const double *v = hv + (k & 1) * N;
+            double *p = hp + (k & 1) * N;
+            const bool next = k + 1 < n - 2 && warp == (t + 1) % WARPS;  // this warp holds row k + 1
             __syncthreads();
             const double tau = sv.tau[k];
-            if (tau == 0.0) continue;
+            if (tau == 0.0) {
+                if (next && t + 1 < WARPS) publish(a[r], k + 1);
+                if (next && t + 1 == WARPS) publish(a[r + 1 < NR ? r + 1 : r], k + 1);
+                continue;
+            }
             double vj[NC], s[8];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) vj[c] = v[lane + 32 * c];
+            for (int c = C0; c < NC; ++c) vj[c] = v[lane + 32 * c];
             // rows before WARPS r are done: NR - r values a lane
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 s[q] = 0.0;
                 if (r + q < NR)
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) s[q] += a[r + q < NR ? r + q : 0][c] * vj[c];
+                    for (int c = C0; c < NC; ++c) s[q] += a[r + q < NR ? r + q : 0][c] * vj[c];
             }
             const int left = NR - r;
             if (left > 4) {
@@ -382,22 +388,35 @@ __global__ void __launch_bounds__(128 * NC, 1)
             // A -= v w^T + w v^T, w = tau p - (tau^2 v.p / 2) v
             double wj[NC], vp = 0.0;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
+            for (int c = C0; c < NC; ++c) {
                 const int j = lane + 32 * c;
                 wj[c] = j > k ? p[j] : 0.0;
                 vp += vj[c] * wj[c];
             }
-            const double half = 0.5 * tau * tau * warp_sum(vp);
+            const double half = 0.5 * tau * (tau * warp_sum(vp));
 #pragma unroll
-            for (int c = 0; c < NC; ++c) wj[c] = tau * wj[c] - half * vj[c];
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-                if (r + q >= NR) continue;
-                const int i = warp + WARPS * (r + q);
+            for (int c = C0; c < NC; ++c) wj[c] = tau * wj[c] - half * vj[c];
+            auto update = [&](double (&row)[NC], int i) {
                 const double vi = v[i], wi = i > k ? tau * p[i] - half * vi : 0.0;
 #pragma unroll
-                for (int c = 0; c < NC; ++c) a[r + q < NR ? r + q : 0][c] -= vi * wj[c] + wi * vj[c];
+                for (int c = C0; c < NC; ++c) row[c] -= vi * wj[c] + wi * vj[c];
+            };
+            // row k + 1 first: the next reflector is a serial chain that the other warps' updates hide
+            int done = -1;
+            if (next) {
+                if (t + 1 < WARPS) {
+                    update(a[r], warp + WARPS * r);
+                    publish(a[r], k + 1);
+                    done = 0;
+                } else {
+                    update(a[r + 1 < NR ? r + 1 : r], warp + WARPS * (r + 1));
+                    publish(a[r + 1 < NR ? r + 1 : r], k + 1);
+                    done = 1;
+                }
             }
+#pragma unroll
+            for (int q = 0; q < NR; ++q)
+                if (r + q < NR && q != done) update(a[r + q < NR ? r + q : 0], warp + WARPS * (r + q));
         }
     }
 #pragma unroll
@@ -464,7 +483,8 @@ __global__ void __launch_bounds__(128 * NC, 1)
             }
             const double rho = 2.0 * fabs(sv.e[o + w - 1]), tol = 8.0 * EPS * fmax(dmax, zmax);
             const int K = deflate<NC>(sv, Z, zp, o, s, rho, tol);
-            const int nt = column_list<NC>(sv, sv.top, o, K, 1), nb = column_list<NC>(sv, sv.bot, o, K, 2);
+            // a block of 8 rows holds both halves of a merge of 4 + 4
+            const int nt = column_list<NC>(sv, sv.top, o, K, w < 8 ? 3 : 1), nb = column_list<NC>(sv, sv.bot, o, K, 2);
             if (lane == 0) {
                 sv.K[mm] = K;
                 sv.ntop[mm] = nt;
@@ -474,53 +494,72 @@ __global__ void __launch_bounds__(128 * NC, 1)
         }
         __syncthreads();
         const int K = merging ? sv.K[m] : 0;
-        const double *kd = sv.kd + off, *kz = sv.kz + off;
-        if (jj < K) {
-            int org;
-            double x;
-            secular_root(K, jj, kd, kz, sv.rho[m], q4, &org, &x);
-            if (q4 == 0) {
-                sv.org[pos] = org;
-                sv.x[pos] = x;
-            }
+        const int Kw = __reduce_max_sync(0xffffffffu, K), Kc = max(K, 1);
+        const bool live = jj < K;
+        const int jc = live ? jj : 0;
+        const double *kd = sv.kd + (merging ? off : 0), *kz = sv.kz + (merging ? off : 0);
+        int org = 0;
+        double x = 0.0;
+        if (Kw > 0) secular_roots(live, Kc, Kw, jc, kd, kz, merging ? sv.rho[m] : 1.0, q4, &org, &x);
+        if (live && q4 == 0) {
+            sv.org[pos] = org;
+            sv.x[pos] = x;
         }
         __syncthreads();
         // the z for which these roots are exact: z_i^2 = prod_j (lambda_j - d_i) / prod_(j != i) (d_j - d_i), up to a factor
-        if (jj < K) {
-            const double di = kd[jj];
+        const int base = merging ? off : 0;
+        {
+            const double di = kd[jc];
             double pr = 1.0;
-            for (int j = q4; j < K; j += 4) {
-                const double num = (kd[sv.org[off + j]] - di) + sv.x[off + j];
-                const double den = j < jj ? kd[j] - di : (j < K - 1 ? kd[j + 1] - di : 1.0);
+            for (int j0 = q4; j0 < Kw; j0 += 16) {  // four ratios share a division
+                double num = 1.0, den = 1.0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int j = j0 + 4 * u, jm = min(j, Kc - 1);
+                    const double a = (kd[live ? sv.org[base + jm] : 0] - di) + sv.x[base + jm];
+                    const double b = kd[jm < jj ? jm : min(jm + 1, Kc - 1)] - di;
+                    num *= j < K ? a : 1.0;
+                    den *= j < K && !(j >= jj && j == K - 1) ? b : 1.0;
+                }
                 pr *= num / den;
             }
+            __syncwarp();
             pr = quad_product(pr);
-            if (q4 == 0) sv.zh[pos] = copysign(sqrt(fabs(pr)), kz[jj]);
+            if (live && q4 == 0) sv.zh[pos] = copysign(sqrt(fabs(pr)), kz[jc]);
         }
         __syncthreads();
         // vectors of the merged problem, 64 columns at a time, and their product with the old ones
         constexpr int CHUNKS = NC > 2 ? 2 : 1;
-        const double lam = jj < K ? kd[sv.org[pos]] + sv.x[pos] : 0.0;
+        const double o = kd[org], lam = o + x;
         auto vectors = [&](int ch) {
-            if (jj < K && jj / 64 == ch) {
-                const double o = kd[sv.org[pos]], x = sv.x[pos];
+            const bool mine = live && jj / 64 == ch;
+            if (__any_sync(0xffffffffu, mine)) {
                 double ss = 0.0;
-                for (int i = q4; i < K; i += 4) {
-                    const double u = sv.zh[off + i] / ((kd[i] - o) - x);
-                    U[(off + i) * up + jj - 64 * ch] = u;
-                    ss += u * u;
+                double *col = U + base * up + jj - 64 * ch;
+                for (int i0 = 0; i0 < Kw; i0 += 8) {  // two elements share a division
+                    const int i = min(i0 + q4, Kc - 1), i2 = min(i0 + q4 + 4, Kc - 1);
+                    const double a = (kd[i] - o) - x, b = (kd[i2] - o) - x, r = 1.0 / (a * b);
+                    const double u1 = sv.zh[base + i] * (b * r), u2 = sv.zh[base + i2] * (a * r);
+                    if (mine && i0 + q4 < K) {
+                        col[i * up] = u1;
+                        ss += u1 * u1;
+                    }
+                    if (mine && i0 + q4 + 4 < K) {
+                        col[i2 * up] = u2;
+                        ss += u2 * u2;
+                    }
                 }
                 ss = quad_sum(ss);
-                if (q4 == 0) sv.scale[pos] = 1.0 / sqrt(ss);
+                if (mine && q4 == 0) sv.scale[pos] = 1.0 / sqrt(ss);
             }
         };
         if (2 * w >= 8) {
             // warp: rows 8 warp .. + 7, inside one merge
             const int r0 = 8 * warp, ro = r0 / (2 * w) * (2 * w), rm = r0 / (2 * w);
-            const bool live = r0 < n && ro + w < n;
-            const int RK = live ? sv.K[rm] : 0;
-            const bool upper = r0 < ro + w, lower = r0 + 7 >= ro + w;
-            const int cnt = upper && lower ? RK : (upper ? (live ? sv.ntop[rm] : 0) : (live ? sv.nbot[rm] : 0));
+            const bool rows = r0 < n && ro + w < n;
+            const int RK = rows ? sv.K[rm] : 0;
+            const bool upper = r0 < ro + w;
+            const int cnt = rows ? (upper ? sv.ntop[rm] : sv.nbot[rm]) : 0;
             const int *list = upper ? sv.top + ro : sv.bot + ro;
             double acc[CHUNKS][8][2];
 #pragma unroll
@@ -531,16 +570,18 @@ __global__ void __launch_bounds__(128 * NC, 1)
 #pragma unroll
                 for (int t = 0; t < 8; ++t) acc[ch][t][0] = acc[ch][t][1] = 0.0;
                 const int cols = RK - 64 * ch;
-                if (cols > 0)
+                if (cols > 0 && cnt > 0) {
+                    int next = list[min(lane & 3, cnt - 1)];
                     for (int k0 = 0; k0 < cnt; k0 += 4) {
-                        const int kq = k0 + (lane & 3), kc = min(kq, cnt - 1);
-                        const int ki = upper && lower ? kc : list[kc];
-                        const double av = kq < cnt ? Z[(r0 + (lane >> 2)) * zp + sv.slot[ro + ki]] : 0.0;
-                        const double *ur = U + (ro + ki) * up + (lane >> 2);
+                        const int cur = next;
+                        next = list[min(k0 + 4 + (lane & 3), cnt - 1)];
+                        const double av = k0 + (lane & 3) < cnt ? Z[(r0 + (lane >> 2)) * zp + (cur >> 8)] : 0.0;
+                        const double *ur = U + (ro + (cur & 255)) * up + (lane >> 2);
 #pragma unroll
                         for (int t = 0; t < 8; ++t)
                             if (8 * t < cols) dmma884(acc[ch][t][0], acc[ch][t][1], av, ur[8 * t]);
                     }
+                }
             }
             __syncwarp();
             const int r = r0 + (lane >> 2);
@@ -566,21 +607,22 @@ __global__ void __launch_bounds__(128 * NC, 1)
             __syncthreads();
             if (mine) Z[pos * zp + sv.slot[off + q4]] = v;
         }
-        if (jj < K && q4 == 0) sv.d[sv.slot[pos]] = lam;
+        if (live && q4 == 0) sv.d[sv.slot[pos]] = lam;
         __syncthreads();
     }
 
-    // ---------------- 3. reflectors, in the order n - 3 .. 0, on this quad's column; ascending order
-    // reflector k from element base(k) + k + 1 on; base(k) is even, so that pairs of rows come in 16-byte reads
-    auto base = [&](int k) {
-        // rows of n - k + 1 elements, rounded up to even, minus the k leading ones that are not stored (even part)
-        const int kk = k / 2;  // reflectors 2 kk and 2 kk + 1 both start at row 2 kk
-        const int len = (n + 1) & ~1;
-        return (k & 1 ? (len - 2 * kk) : 0) + 2 * (kk * len - kk * (kk - 1)) - 2 * kk;
-    };
-    for (int k = warp; k < n - 2; k += WARPS) {
-        double *dst = U + base(k);
-        for (int j = (k & ~1) + lane; j < ((n + 1) & ~1); j += 32) dst[j] = j > k && j < n ? V[(size_t)k * n + j] : 0.0;
+    // ---------------- 3. reflectors, blocks of eight from the last to the first, on the warp's eight columns:
+    // H_k ... H_(k+7) = 1 - R T R^T with the reflectors as the columns of R and a triangular T
+    // block b: eight rows (reflectors) of the elements from 8 b on, pitch 4 mod 8 doubles
+    auto block = [&](int b) { return U + 8 * (b * (lay.rows + 4) - 4 * b * (b - 1)); };
+    const int blocks = n > 2 ? (n - 2 + 7) / 8 : 0;
+    for (int k = warp; k < 8 * blocks; k += WARPS) {
+        const int b = k / 8, len = lay.rows - 8 * b;
+        double *dst = block(b) + (k & 7) * (len + 4);
+        for (int i = lane; i < len; i += 32) {
+            const int j = 8 * b + i;
+            dst[i] = k < n - 2 && j > k && j < n ? V[(size_t)k * n + j] : 0.0;
+        }
     }
     const double ev = pos < n ? sv.d[pos] : 0.0;
     int rank = 0;
@@ -591,45 +633,80 @@ __global__ void __launch_bounds__(128 * NC, 1)
     rank += __shfl_xor_sync(0xffffffffu, rank, 1);
     rank += __shfl_xor_sync(0xffffffffu, rank, 2);
     __syncthreads();  // V has been read
-    double y[N / 8][2];  // rows 8 t + 2 q4, + 1
-#pragma unroll
-    for (int t = 0; t < N / 8; ++t)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = 8 * t + 2 * q4 + h;
-            y[t][h] = i < n && pos < n ? Z[i * zp + pos] : 0.0;
-        }
-    for (int k = n - 3; k >= 0; --k) {
-        const double tau = sv.tau[k];
-        if (tau == 0.0) continue;
-        const double *v = U + base(k) + 2 * q4;
-        const int t0 = k / 8;  // earlier blocks of rows are zero in v
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-        for (int t = 0; t < N / 8; ++t)
-            if (t >= t0 && 8 * t + 2 * q4 < n && 8 * t + 2 * q4 >= (k & ~1)) {
-                const double2 x = *reinterpret_cast<const double2 *>(v + 8 * t);
-                s0 += x.x * y[t][0];
-                s1 += x.y * y[t][1];
-            }
-        const double f = tau * quad_sum(s0 + s1);
-#pragma unroll
-        for (int t = 0; t < N / 8; ++t)
-            if (t >= t0 && 8 * t + 2 * q4 < n && 8 * t + 2 * q4 >= (k & ~1)) {
-                const double2 x = *reinterpret_cast<const double2 *>(v + 8 * t);
-                y[t][0] -= f * x.x;
-                y[t][1] -= f * x.y;
-            }
+    if (pos < n && q4 == 0) {
+        W[rank] = ev * back;
+        sv.ord[pos] = rank;
     }
-    if (pos < n) {
-        if (q4 == 0) W[rank] = ev * back;
+    const int fr = lane >> 2, fc = lane & 3;  // fragment row (A) or column (B), and the other index
+    double *tm = sv.e;                        // T of block b at 64 b
+    if (warp < blocks) {
+        const int len = lay.rows - 8 * warp, pitch = len + 4;
+        const double *R = block(warp);
+        double g0 = 0.0, g1 = 0.0;
+        for (int i = 0; i < len; i += 4) {
+            const double x = R[fr * pitch + i + fc];
+            dmma884(g0, g1, x, x);
+        }
+        double *T = tm + 64 * warp;
+        T[fr * 8 + 2 * fc] = g0;
+        T[fr * 8 + 2 * fc + 1] = g1;
+        __syncwarp();
+        // row l of T: T_lj = -T_jj sum_(m < j) T_lm (R^T R)_mj
+        double row[8];
+        const int l = lane & 7;
 #pragma unroll
-        for (int t = 0; t < N / 8; ++t)
+        for (int j = 0; j < 8; ++j) {
+            const double tj = 8 * warp + j < n - 2 ? sv.tau[8 * warp + j] : 0.0;
+            double x = 0.0;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = 8 * t + 2 * q4 + h;
-                if (i < n) V[(size_t)rank * n + i] = y[t][h];
+            for (int m = 0; m < j; ++m) x += row[m] * T[m * 8 + j];
+            row[j] = j < l ? 0.0 : (j == l ? tj : -tj * x);
+        }
+        __syncwarp();
+        if (lane < 8)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) T[l * 8 + j] = row[j];
+    }
+    __syncthreads();
+    const int c0 = 8 * warp;
+    if (c0 < n) {
+        // accumulator layout (row fr, columns 2 fc, + 1) to B operand (row 4 s + fc, column fr)
+        auto operand = [&](double d0, double d1, int s) {
+            const int src = (4 * s + fc) * 4 + (fr >> 1);
+            const double x0 = __shfl_sync(0xffffffffu, d0, src), x1 = __shfl_sync(0xffffffffu, d1, src);
+            return fr & 1 ? x1 : x0;
+        };
+        for (int b = blocks - 1; b >= 0; --b) {
+            const int len = lay.rows - 8 * b, pitch = len + 4;
+            const double *R = block(b), *T = tm + 64 * b;
+            double *Zb = Z + 8 * b * zp + c0;
+            double w0 = 0.0, w1 = 0.0, u0 = 0.0, u1 = 0.0;
+#pragma unroll 4
+            for (int i = 0; i < len; i += 8) {
+                dmma884(w0, w1, R[fr * pitch + i + fc], Zb[(i + fc) * zp + fr]);
+                dmma884(u0, u1, R[fr * pitch + i + 4 + fc], Zb[(i + 4 + fc) * zp + fr]);
             }
+            w0 += u0;
+            w1 += u1;
+            double x0 = 0.0, x1 = 0.0;
+            dmma884(x0, x1, T[fr * 8 + fc], operand(w0, w1, 0));
+            dmma884(x0, x1, T[fr * 8 + 4 + fc], operand(w0, w1, 1));
+            const double b0 = -operand(x0, x1, 0), b1 = -operand(x0, x1, 1);
+            __syncwarp();
+#pragma unroll 4
+            for (int i = 0; i < len; i += 8) {
+                double2 *z = reinterpret_cast<double2 *>(Zb + (i + fr) * zp + 2 * fc);
+                double2 x = *z;
+                dmma884(x.x, x.y, R[fc * pitch + i + fr], b0);
+                dmma884(x.x, x.y, R[(4 + fc) * pitch + i + fr], b1);
+                *z = x;
+            }
+            __syncwarp();
+        }
+        for (int c = c0; c < min(c0 + 8, n); ++c) {
+            double *dst = V + (size_t)sv.ord[c] * n;
+            for (int i = lane; i < n; i += 32) dst[i] = Z[i * zp + c];
+        }
     }
     if (tid == 0) info[blockIdx.x] = 0;
 }

@@ -27,8 +27,8 @@ def small_eigh(A):
 
 
 def eigh(A):
-    """torch.linalg.eigh(A).  The kernel is the faster one at every size it takes (B200: 0.08 and 0.16 ms at n = 5, 0.50
-    and 2.11 ms at n = 128; a batch of 256 at n = 128 0.96 and 3.30 ms); one SM holds no larger matrix."""
+    """torch.linalg.eigh(A).  The kernel is the faster one at every size it takes (B200: 0.08 and 0.16 ms at n = 5, 0.39
+    and 2.11 ms at n = 128; a batch of 256 at n = 128 0.75 and 3.28 ms); one SM holds no larger matrix."""
     if not small(A):
         return torch.linalg.eigh(A)
     w, V, info = small_eigh(A)
