@@ -14,13 +14,11 @@
 //   * store the result as a BF16 hi/lo pair, row-major and/or transposed
 //     (the transposed store is coalesced across a warp).
 //
-// Structure per CTA (128 threads, one 128x128 output tile):
-//   warp 0 lane 0 : TMA producer, 4-stage ring of 128x64 A and B tiles
-//                   (128-byte swizzle), mbarrier::complete_tx completion;
-//   warp 1 lane 0 : issues tcgen05.mma (M=128, N=128, K=16 per instruction)
-//                   into a 128-column TMEM accumulator; tcgen05.commit frees
-//                   ring slots and finally signals the epilogue;
-//   warps 0..3    : epilogue, tcgen05.ld 32x32b of their 32 TMEM lanes.
+// Structure per CTA (320 threads, 128 x 128 or 128 x 256 output tiles; pairs of CTAs: 256 x 256):
+//   warp 0 lane 0 : TMA producer, ring of operand tiles, mbarrier::complete_tx completion;
+//   warp 1 lane 0 : issues tcgen05.mma into one of two TMEM accumulators; tcgen05.commit frees ring slots and finally
+//                   signals the epilogue;
+//   warps 2..9    : epilogue, tcgen05.ld 32x32b of their 32 TMEM lanes, under the next tile's MMAs.
 // Every mbarrier wait is bounded; on timeout the kernel records an error
 // code, stops issuing work, drains the copies it started and releases TMEM.
 
@@ -99,21 +97,24 @@ constexpr int EPI_WARPS = 8, EPI_THREADS = 32 * EPI_WARPS, THREADS = 64 + EPI_TH
 constexpr int TPITCH = 40;
 constexpr int TSTAGE_BYTES = EPI_WARPS * 32 * TPITCH * 2;
 
-template <bool SPLIT, bool WIDE = false> struct Cfg {
+template <bool SPLIT, bool WIDE = false, bool PAIR = false> struct Cfg {
     // 128 x 128 output tiles with 64-element K blocks (128-byte swizzle); WIDE (split mode only): 128 x 256
     // tiles with 32-element K blocks (64-byte swizzle), so four stages of A_hi, A_lo, B_hi, B_lo fit and a
     // stage carries the same MMA work with a quarter fewer operand bytes.  (128 x 256 tiles with 64-element
-    // blocks leave room for two stages only, which measured slower.)
+    // blocks leave room for two stages only, which measured slower.)  PAIR (WIDE only): 256 x 256 tiles of a
+    // CTA pair, each CTA holding half the rows of A and of B.
+    static constexpr int BMX = PAIR ? 2 * BM : BM;
     static constexpr int BNX = WIDE ? 256 : 128;
-    static constexpr int BKX = WIDE ? 32 : BK;
+    static constexpr int BKX = WIDE && !PAIR ? 32 : BK;
+    static constexpr int KU = WIDE ? 32 : BK;  // K ranges (split-K) come in multiples of this
     static constexpr int TILE_AX = BM * BKX * 2;
-    static constexpr int TILE_BX = BNX * BKX * 2;
-    static constexpr int STAGES = WIDE ? 4 : (SPLIT ? 3 : 4);
+    static constexpr int TILE_BX = (PAIR ? BNX / 2 : BNX) * BKX * 2;
+    static constexpr int STAGES = PAIR ? 3 : (WIDE ? 4 : (SPLIT ? 3 : 4));
     static constexpr int STAGE_BYTES = SPLIT ? 2 * (TILE_AX + TILE_BX) : TILE_AX + TILE_BX;
     static constexpr int SMEM_BYTES =
         STAGES * STAGE_BYTES + TSTAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BNX >> 3) << 17) |
-                                      ((uint32_t)(BM >> 4) << 24);
+                                      ((uint32_t)(BMX >> 4) << 24);
 };
 
 struct Maps {
@@ -187,6 +188,15 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_c, uint64_t da, uint64_t
         "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
 }
 
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t accumulate,
+                                               uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+        "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
     uint32_t r[16];
     asm volatile(
@@ -210,16 +220,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
 // Output tile t of a launch: tiles run M-fastest, then N, then the K range (split-K index), so the
 // CTAs working at one time share B tiles and the A operand stays in L2.
 struct TileCoords {
-    int m0, n0, kb0, kblocks;
+    int m0, n0, k0, kend, kblocks;  // kblocks of bkx elements cover k0 .. kend
 };
 
-__device__ __forceinline__ TileCoords tile_coords(int t, int mt, int nt, int bnx, int kblocks_all, int kper) {
+// kper: units of ku elements in a K range
+__device__ __forceinline__ TileCoords tile_coords(int t, int mt, int nt, int bmx, int bnx, int bkx, int ku, int kper, int K) {
     TileCoords c;
     const int mi = t % mt, rest = t / mt;
-    c.m0 = mi * BM;
+    c.m0 = mi * bmx;
     c.n0 = (rest % nt) * bnx;
-    c.kb0 = (rest / nt) * kper;
-    c.kblocks = max(0, min(kblocks_all, c.kb0 + kper) - c.kb0);
+    c.k0 = (rest / nt) * kper * ku;
+    c.kend = min(K, c.k0 + kper * ku);
+    c.kblocks = max(0, (c.kend - c.k0 + bkx - 1) / bkx);
     return c;
 }
 
@@ -234,11 +246,18 @@ __device__ __forceinline__ TileCoords tile_coords(int t, int mt, int nt, int bnx
 // MLP (segment mode): the epilogue of a dense layer of the pair-scoring network, forward (bias and ReLU) or backward
 // (ReLU mask and bias gradient), instead of an FP32 result that another kernel would read again.  B200, 65536 samples x
 // 256 units: product and bias_relu 32 + 46 us, product and relu_backward 32 + 80 us; here 25 to 40 us.
-template <bool SPLIT, bool WIDE, bool MLP = false>
+// PAIR (clusters of two): a 128 x 256 split tile makes each SM read 12 KiB of operands per MMA of 128 cycles from shared
+// memory while TMA writes 8 KiB, 160 of the 128 bytes a cycle that it moves, and all of B crosses the L2 for every 128 rows
+// of A.  In cta_group::2 each CTA reads and is sent half of B: 8 KiB and 5.3 KiB.  The even CTA issues the MMAs of both; its
+// full (bytes of both CTAs) and tempty barriers count for the pair, empty and tfull are committed to both.  The K order of an
+// element is that of the other tiles, so the results are the same bits.  B200, the exchange's shapes, us without and with:
+// W 8292 x 1225 x 1225 77 -> 71, N 8292 x 8292 x 1225 (Hadamard, both outputs) 514 -> 441, P 1225 x 16640 x 8292 723 -> 678
+// (1.50 PFLOP/s), K 2450 x 1225 x 8292 164 -> 147.
+template <bool SPLIT, bool WIDE, bool MLP = false, bool PAIR = false>
 __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
-    using C = Cfg<SPLIT, WIDE>;
+    using C = Cfg<SPLIT, WIDE, PAIR>;
     constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES;
-    constexpr int BNX = C::BNX, TILE_BX = C::TILE_BX, TILE_AX = C::TILE_AX, BKX = C::BKX;
+    constexpr int BMX = C::BMX, BNX = C::BNX, TILE_BX = C::TILE_BX, TILE_AX = C::TILE_AX, BKX = C::BKX;
     constexpr uint32_t IDESC = C::IDESC;
     static_assert(BNX % 32 == 0 && (!WIDE || SPLIT), "tile columns come in 32-column chunks; WIDE is split-only");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -252,9 +271,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int mt = (p.M + BM - 1) / BM, nt = (p.N + BNX - 1) / BNX;
+    const uint32_t rank = PAIR ? cluster_rank() : 0;
+    const int tile0 = PAIR ? blockIdx.x / 2 : blockIdx.x, tstep = PAIR ? gridDim.x / 2 : gridDim.x;
+    const int mt = (p.M + BMX - 1) / BMX, nt = (p.N + BNX - 1) / BNX;
     const int ntiles = mt * nt * p.ksplit;
-    const int kblocks_all = (p.K + BKX - 1) / BKX;
+    const int kblocks_all = (p.K + C::KU - 1) / C::KU;
     const int kper = (kblocks_all + p.ksplit - 1) / p.ksplit;
 
     if (threadIdx.x == 0) {
@@ -264,7 +285,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&tfull[a], 1);
-            mbar_init(&tempty[a], EPI_THREADS);
+            mbar_init(&tempty[a], PAIR ? 2 * EPI_WARPS : EPI_THREADS);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -273,11 +294,22 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
     __syncwarp();
     if (warp == 0) {
         // two accumulators of BNX columns (128 lanes x 2 BNX FP32)
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(2 * BNX));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                         "r"(2 * BNX));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                         "r"(2 * BNX));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        }
     }
     __syncthreads();
+    if constexpr (PAIR) {
+        __syncwarp();
+        cluster_sync();  // both CTAs' barriers exist before either signals the other's
+    }
+    auto wait = [](uint64_t *bar, uint32_t parity) { return PAIR ? mbar_wait_cluster(bar, parity) : mbar_wait(bar, parity); };
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
@@ -286,12 +318,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
             // ---------------- TMA producer
             int it = 0;  // copies issued (ring position)
             bool stop = false;
-            for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
-                const TileCoords tc = tile_coords(t, mt, nt, BNX, kblocks_all, kper);
+            for (int t = tile0; t < ntiles && !stop; t += tstep) {
+                const TileCoords tc = tile_coords(t, mt, nt, BMX, BNX, BKX, C::KU, kper, p.K);
                 const int total = SPLIT ? tc.kblocks : tc.kblocks * p.nseg;
                 for (int i = 0; i < total; ++i) {
                     const int s = it % STAGES;
-                    if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1)) {
+                    if (it >= STAGES && !wait(&empty[s], ((it / STAGES) - 1) & 1)) {
                         atomicExch(p.err, 1);
                         *(volatile int *)abort_flag = 1;
                         stop = true;
@@ -302,36 +334,46 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                         break;
                     }
                     uint8_t *sa = smem + s * STAGE_BYTES;
-                    mbar_expect_tx(&full[s], STAGE_BYTES);
-                    if (SPLIT) {
+                    if (!PAIR) mbar_expect_tx(&full[s], STAGE_BYTES);
+                    if constexpr (PAIR) {
+                        // this CTA's halves; the even CTA's barrier counts the bytes of both
+                        const int kx = tc.k0 + i * BKX, ya = tc.m0 + (int)rank * BM, yb = tc.n0 + (int)rank * (BNX / 2);
+                        if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                        const uint32_t bar = map_cta(&full[s], 0);
+                        tma_load_2d_pair(sa, &maps.a[0], bar, kx, ya);
+                        tma_load_2d_pair(sa + TILE_AX, &maps.a[1], bar, kx, ya);
+                        tma_load_2d_pair(sa + 2 * TILE_AX, &maps.b[0], bar, kx, yb);
+                        tma_load_2d_pair(sa + 2 * TILE_AX + TILE_BX, &maps.b[1], bar, kx, yb);
+                    } else if (SPLIT) {
                         // stage layout: A_hi | A_lo | B_hi | B_lo
-                        const int kx = (tc.kb0 + i) * BKX;
+                        const int kx = tc.k0 + i * BKX;
                         tma_load_2d(sa, &maps.a[0], &full[s], kx, tc.m0);
                         tma_load_2d(sa + TILE_AX, &maps.a[1], &full[s], kx, tc.m0);
                         tma_load_2d(sa + 2 * TILE_AX, &maps.b[0], &full[s], kx, tc.n0);
                         tma_load_2d(sa + 2 * TILE_AX + TILE_BX, &maps.b[1], &full[s], kx, tc.n0);
                     } else {
-                        const int seg = i / tc.kblocks, kb = tc.kb0 + i % tc.kblocks;
-                        tma_load_2d(sa, &maps.a[seg], &full[s], kb * BKX, tc.m0);
-                        tma_load_2d(sa + TILE_AX, &maps.b[seg], &full[s], kb * BKX, tc.n0);
+                        const int seg = i / tc.kblocks, kx = tc.k0 + i % tc.kblocks * BKX;
+                        tma_load_2d(sa, &maps.a[seg], &full[s], kx, tc.m0);
+                        tma_load_2d(sa + TILE_AX, &maps.b[seg], &full[s], kx, tc.n0);
                     }
                     ++it;
                 }
             }
             // drain: wait (bounded) until every copy that was started has landed
-            for (int j = max(0, it - STAGES); j < it; ++j) mbar_wait(&full[j % STAGES], (j / STAGES) & 1);
+            // (pairs: until the MMAs have read it, which both CTAs see)
+            for (int j = max(0, it - STAGES); j < it; ++j) wait(PAIR ? &empty[j % STAGES] : &full[j % STAGES], (j / STAGES) & 1);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---------------- MMA issuer
+        if (lane == 0 && rank == 0) {
+            // ---------------- MMA issuer (of both CTAs)
             int it = 0, j = 0;
             bool stop = false;
-            for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x, ++j) {
-                const TileCoords tc = tile_coords(t, mt, nt, BNX, kblocks_all, kper);
+            for (int t = tile0; t < ntiles && !stop; t += tstep, ++j) {
+                const TileCoords tc = tile_coords(t, mt, nt, BMX, BNX, BKX, C::KU, kper, p.K);
                 const int total = SPLIT ? tc.kblocks : tc.kblocks * p.nseg;
                 const int acc = j & 1;
                 const uint32_t tacc = tmem + (uint32_t)(acc * BNX);
-                if (j >= 2 && !mbar_wait(&tempty[acc], ((j >> 1) - 1) & 1)) {
+                if (j >= 2 && !wait(&tempty[acc], ((j >> 1) - 1) & 1)) {
                     atomicExch(p.err, 4);
                     *(volatile int *)abort_flag = 1;
                     break;
@@ -339,7 +381,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int i = 0; i < total; ++i) {
                     const int s = it % STAGES;
-                    if (!mbar_wait(&full[s], (it / STAGES) & 1)) {
+                    if (!wait(&full[s], (it / STAGES) & 1)) {
                         atomicExch(p.err, 2);
                         *(volatile int *)abort_flag = 1;
                         stop = true;
@@ -351,7 +393,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-                    if (SPLIT) {
+                    if constexpr (PAIR) {
+                        const uint32_t sal = sa + TILE_AX, sb = sa + 2 * TILE_AX, sbl = sb + TILE_BX;
+                        const int ks = min(BKX / 16, (tc.kend - tc.k0 - i * BKX + 15) / 16);  // none past the K range
+                        for (int k = 0; k < ks; ++k) {
+                            const uint32_t o = k * 32;
+                            umma_bf16_pair(tacc, smem_desc_k128(sa + o), smem_desc_k128(sb + o), (i > 0 || k > 0) ? 1u : 0u,
+                                           IDESC);
+                            umma_bf16_pair(tacc, smem_desc_k128(sa + o), smem_desc_k128(sbl + o), 1u, IDESC);
+                            umma_bf16_pair(tacc, smem_desc_k128(sal + o), smem_desc_k128(sb + o), 1u, IDESC);
+                        }
+                    } else if (SPLIT) {
                         const uint32_t sal = sa + TILE_AX, sb = sa + 2 * TILE_AX, sbl = sb + TILE_BX;
 #pragma unroll
                         for (int k = 0; k < BKX / 16; ++k) {
@@ -371,10 +423,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                                       (i > 0 || k > 0) ? 1u : 0u);
                         }
                     }
-                    umma_commit(&empty[s]);  // slot s may be refilled once these MMAs have read it
+                    if constexpr (PAIR)
+                        umma_commit_pair(&empty[s]);
+                    else
+                        umma_commit(&empty[s]);  // slot s may be refilled once these MMAs have read it
                     ++it;
                 }
-                umma_commit(&tfull[acc]);  // accumulator complete (or abandoned) -> epilogue
+                if constexpr (PAIR)
+                    umma_commit_pair(&tfull[acc]);
+                else
+                    umma_commit(&tfull[acc]);  // accumulator complete (or abandoned) -> epilogue
             }
         }
     } else {
@@ -423,11 +481,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
             }
         };
         int j = 0;
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++j) {
-            const TileCoords tc = tile_coords(t, mt, nt, BNX, kblocks_all, kper);
+        for (int t = tile0; t < ntiles; t += tstep, ++j) {
+            const TileCoords tc = tile_coords(t, mt, nt, BMX, BNX, BKX, C::KU, kper, p.K);
             const int total = SPLIT ? tc.kblocks : tc.kblocks * p.nseg;
             const int acc = j & 1;
-            const int m0 = tc.m0, n0 = tc.n0;
+            const int m0 = tc.m0 + (int)rank * BM, n0 = tc.n0;
             const int row = m0 + rloc;
             if (p.G && p.ksplit == 1 && row < p.M) {
                 // pull this tile's G row into L2 while its MMAs run (128-byte lines, inside the matrix)
@@ -436,7 +494,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                 for (int c = chunk0; c < ncols; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + c));
             }
             const float *bias_s = MLP && p.bias ? p.bias + n0 : nullptr;
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(&tfull[acc], (j >> 1) & 1) ? 1 : 0) != 0;
+            const bool ok = __all_sync(0xffffffffu, wait(&tfull[acc], (j >> 1) & 1) ? 1 : 0) != 0;
             if (!ok && lane == 0) atomicExch(p.err, 3);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool live = ok && !*(volatile int *)abort_flag && total > 0;  // warp-uniform
@@ -530,14 +588,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
             }
             // the accumulator has been read: hand it back to the MMA issuer
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(&tempty[acc]);
+            if constexpr (PAIR) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_cta(&tempty[acc], 0));
+            } else {
+                mbar_arrive(&tempty[acc]);
+            }
             if (!ok) break;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) {
+        __syncwarp();
+        cluster_sync();  // neither CTA leaves while the other may signal its barriers or its MMAs read its memory
+    }
     if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BNX));
+        if constexpr (PAIR)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BNX));
+        else
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BNX));
     }
 }
 
@@ -612,14 +682,23 @@ int make_map(CUtensorMap *map, const void *base, int rows, int cols, long long l
     return 0;
 }
 
-// mode: 0 segments, 1 split, 2 split with 128 x 256 tiles, 3 segments with a dense layer's epilogue
+// 128 x 256 split tiles go to CTA pairs unless less than one round of tiles meets a short K range: there the pair's start
+// and finish cost more than its main loop saves.  B200, cold L2, us with pairs and without: 1281 x 1281 x 640 (66 tiles)
+// 26.6 and 24.6, 808 x 808 x 202 30.7 and 28.7; 385 x 8192 x 4096 (128 tiles) 78 and 84, 3000 x 3000 x 1000 (288) 49 and
+// 51, 2436 x 2436 x 609 (200) 57 and 57, 2450 x 1225 x 8292 in four K ranges 171 and 194.
+bool pair_tiles(int M, int N, int K, int ksplit) {
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256) * ksplit;
+    return M > BM && (tiles > 148 || K / ksplit >= 1024);
+}
+
+// mode: 0 segments, 1 split, 2 split with 128 x 256 tiles, 3 segments with a dense layer's epilogue, 4 split with pair tiles
 int launch(const Maps &maps, const Params &p, int mode, void *stream) {
     using Kernel = void (*)(const Maps, const Params);
-    static const Kernel kernels[4] = {gemm_kernel<false, false>, gemm_kernel<true, false>, gemm_kernel<true, true>,
-                                      gemm_kernel<false, false, true>};
-    static const int smem[4] = {Cfg<false>::SMEM_BYTES, Cfg<true>::SMEM_BYTES, Cfg<true, true>::SMEM_BYTES,
-                                Cfg<false>::SMEM_BYTES};
-    static bool attr_set[4][64] = {{false}};
+    static const Kernel kernels[5] = {gemm_kernel<false, false>, gemm_kernel<true, false>, gemm_kernel<true, true>,
+                                      gemm_kernel<false, false, true>, gemm_kernel<true, true, false, true>};
+    static const int smem[5] = {Cfg<false>::SMEM_BYTES, Cfg<true>::SMEM_BYTES, Cfg<true, true>::SMEM_BYTES,
+                                Cfg<false>::SMEM_BYTES, Cfg<true, true, true>::SMEM_BYTES};
+    static bool attr_set[5][64] = {{false}};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !attr_set[mode][dev]) {
@@ -629,9 +708,10 @@ int launch(const Maps &maps, const Params &p, int mode, void *stream) {
         }
         if (dev >= 0 && dev < 64) attr_set[mode][dev] = true;
     }
-    const int bnx = mode == 2 ? Cfg<true, true>::BNX : Cfg<false>::BNX;
+    const int group = mode == 4 ? 2 : 1, bmx = group * BM;  // CTAs that share a tile
+    const int bnx = mode == 2 || mode == 4 ? Cfg<true, true>::BNX : Cfg<false>::BNX;
     // persistent launch: one CTA per SM (the shared-memory footprint admits one), each walking tiles
-    const long long ntiles = (long long)((p.M + BM - 1) / BM) * ((p.N + bnx - 1) / bnx) * p.ksplit;
+    const long long ntiles = (long long)((p.M + bmx - 1) / bmx) * ((p.N + bnx - 1) / bnx) * p.ksplit;
     if (ntiles > (1LL << 30)) return DFTB_ERR_BAD_SIZE;
     static int sm_count[64] = {0};
     if (dev >= 0 && dev < 64 && sm_count[dev] == 0) {
@@ -640,8 +720,27 @@ int launch(const Maps &maps, const Params &p, int mode, void *stream) {
         sm_count[dev] = n;
     }
     const int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 148;
-    kernels[mode]<<<(unsigned)(ntiles < sms ? ntiles : sms), THREADS, smem[mode], reinterpret_cast<cudaStream_t>(stream)>>>(
-        maps, p);
+    const unsigned ctas = group * (unsigned)(ntiles < sms / group ? ntiles : sms / group);
+    if (mode == 4) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(THREADS);
+        cfg.dynamicSmemBytes = smem[mode];
+        cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cudaLaunchKernelEx(&cfg, kernels[mode], maps, p) != cudaSuccess) {
+            snprintf(g_err, sizeof(g_err), "gemm_kernel: %s", cudaGetErrorString(cudaGetLastError()));
+            return DFTB_ERR_CUDA;
+        }
+    } else {
+        kernels[mode]<<<ctas, THREADS, smem[mode], reinterpret_cast<cudaStream_t>(stream)>>>(maps, p);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         snprintf(g_err, sizeof(g_err), "gemm_kernel: %s", cudaGetErrorString(e));
@@ -691,6 +790,7 @@ int dftb_bf16x3_gemm_ex(int M, int N, int K, int nseg, int shared_split, int ksp
     if (get_encode()) return DFTB_ERR_CUDA;
     Maps maps;
     memset(&maps, 0, sizeof(maps));
+    const bool pair = shared_split == 2 && pair_tiles(M, N, K, ksplit);
     for (int s = 0; s < nseg; ++s) {
         if (!A[s] || !B[s]) return DFTB_ERR_NULL;
         if ((reinterpret_cast<uintptr_t>(A[s]) & 15) || (reinterpret_cast<uintptr_t>(B[s]) & 15)) {
@@ -698,8 +798,8 @@ int dftb_bf16x3_gemm_ex(int M, int N, int K, int nseg, int shared_split, int ksp
             return DFTB_ERR_BAD_SIZE;
         }
         const bool wide = shared_split == 2;
-        const int bkx = wide ? Cfg<true, true>::BKX : BK;
-        const int bnx = wide ? Cfg<true, true>::BNX : (shared_split ? Cfg<true>::BNX : Cfg<false>::BNX);
+        const int bkx = wide && !pair ? Cfg<true, true>::BKX : BK;
+        const int bnx = wide && !pair ? Cfg<true, true>::BNX : BN;
         if (make_map(&maps.a[s], A[s], M, K, lda, BM, bkx) || make_map(&maps.b[s], B[s], N, K, ldb, bnx, bkx))
             return DFTB_ERR_CUDA;
     }
@@ -725,7 +825,7 @@ int dftb_bf16x3_gemm_ex(int M, int N, int K, int nseg, int shared_split, int ksp
     p.mask = nullptr;
     p.ldm = 0;
     p.colsum = nullptr;
-    return tcg::launch(maps, p, shared_split, stream);
+    return tcg::launch(maps, p, pair ? 4 : shared_split, stream);
 }
 
 int dftb_mlp_dense(int ns, int nout, int nin, const void *X, int ldx, const void *W, int ldw, const float *bias,
