@@ -93,6 +93,20 @@ class ExchangeAO:
         K1, K2 = self.exchange(V)
         return coul - K1 - K2, omv + K2 - K1
 
+    def _products(self, V):
+        """__call__ from the interleaved K1^T, K2^T of _exchange_interleaved: one pass forms both results."""
+        if not self.lc:
+            return ExchangeAO.__call__(self, V)
+        self.products_applied += V.shape[1]
+        V = V.contiguous()
+        U = self.coulomb(V)
+        Kall = self._exchange_interleaved(V)
+        W = torch.empty_like(V)
+        omega = self.omega.contiguous()
+        native.call("dftb_exchange_combine", V.shape[1], self.nvirt, self.nocc, int(Kall.dtype == torch.float64),
+                    native.ptr(Kall), native.ptr(omega), native.ptr(V), native.ptr(U), native.ptr(W), native.stream())
+        return U, W
+
 
 class ExchangeMixed(ExchangeAO):
     """(A+B).V and (A-B).V with the exchange contractions on the tensor cores.
@@ -189,7 +203,10 @@ class ExchangeMixed(ExchangeAO):
         T.gemm(self.QOVT, Gt, K=self.nat, out=U)
         return self.omega[:, None] * V + 4.0 * U[:, :m].double()
 
-    def exchange(self, V):
+    def __call__(self, V):
+        return self._products(V)
+
+    def _exchange_interleaved(self, V):
         T = self.T
         nov, m = V.shape
         no, nv, norb = self.nocc, self.nvirt, self.norb
@@ -207,6 +224,11 @@ class ExchangeMixed(ExchangeAO):
             T.gemm(self.YbarT, self.NB, K=2 * norb, out_pair=self.P12, refine=rf)
             # K1^T and K2^T interleaved by rows, in one launch
             T.gemm(self.Pint, self.XbarT, K=2 * norb, alpha=0.25, out=Kall[c], refine=rf)
+        return Kall
+
+    def exchange(self, V):
+        Kall = self._exchange_interleaved(V)
+        m, no, nv = V.shape[1], self.nocc, self.nvirt
         # (m, nv, no) -> (no, nv, m) = the (nov, m) column block, widened to FP64
         K1 = torch.empty((no * nv, m), dtype=torch.float64, device=V.device)
         K2 = torch.empty_like(K1)
@@ -250,14 +272,15 @@ class ExchangeOzaki(ExchangeAO):
         self.WT = torch.empty((2 * norb, nocc), dtype=torch.float64, device=dev)
         self.N = torch.empty((2 * norb, 2 * norb), dtype=torch.float64, device=dev)
         self.P12 = torch.empty((nvirt, 4 * norb), dtype=torch.float64, device=dev)
-        self.K12t = torch.empty((2 * nvirt, nocc), dtype=torch.float64, device=dev)
 
-    def exchange(self, V):
+    def __call__(self, V):
+        return self._products(V)
+
+    def _exchange_interleaved(self, V):
         O = self.O
         nov, m = V.shape
         no, nv, norb = self.nocc, self.nvirt, self.norb
-        K1 = torch.empty_like(V)
-        K2 = torch.empty_like(V)
+        Kall = torch.empty((m, 2 * nv, no), dtype=torch.float64, device=V.device)
         Vt = native.transpose(V)
         for c in range(m):
             self.opV.set(Vt[c].view(no, nv))
@@ -268,10 +291,14 @@ class ExchangeOzaki(ExchangeAO):
             self.opNB.set(self.N.T, row0=2 * norb)
             O.product(self.opYbarT, self.opNB, out=self.P12)
             self.opP.set(self.P12.view(2 * nv, 2 * norb))
-            O.product(self.opP, self.opXbarT, out=self.K12t, alpha=0.25)
-            K1[:, c].view(no, nv).copy_(self.K12t[0::2].T)
-            K2[:, c].view(no, nv).copy_(self.K12t[1::2].T)
-        return K1, K2
+            O.product(self.opP, self.opXbarT, out=Kall[c], alpha=0.25)
+        return Kall
+
+    def exchange(self, V):
+        Kall = self._exchange_interleaved(V)
+        m, no, nv = V.shape[1], self.nocc, self.nvirt
+        K = Kall.view(m, nv, 2, no).permute(2, 3, 1, 0).reshape(2, no * nv, m)
+        return K[0], K[1]
 
 
 class LR_TDDFTB:

@@ -62,6 +62,7 @@ _SIGNATURES = {
     "dftb_davidson_residual": (_I, [_I, _I, _P, _I, _P, _I, _P, _P, _I, _P, _P]),
     "dftb_transpose_f64": (_I, [_I, _I, _P, _I, _P, _I, _P]),
     "dftb_exchange_unpack": (_I, [_I, _I, _I, _P, _P, _P, _P]),
+    "dftb_exchange_combine": (_I, [_I, _I, _I, _I, _P, _P, _P, _P, _P, _P]),
     "dftb_dgemm": (_I, [_I, _I, _I, _I, _I, _D, _P, _I, _P, _I, _D, _P, _I, _P]),
     "dftb_bf16x3_gemm": (_I, [_I, _I, _I, _I, ctypes.POINTER(_P), _I, ctypes.POINTER(_P), _I, ctypes.c_float, _P, _I,
                               _P, _I, _P, _P, _I, _P, _P, _I, _P, _P]),

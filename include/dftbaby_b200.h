@@ -286,6 +286,10 @@ int dftb_transpose_f64(int rows, int cols, const double *X, int ldx, double *Y, 
  * 2a and 2a + 1 hold K1^T and K2^T of product column c:
  *   K_y[(i nvirt + a) m + c] = Kall[c][2a + y][i];  nvirt <= 65535. */
 int dftb_exchange_unpack(int m, int nvirt, int nocc, const float *Kall, double *K1, double *K2, void *stream);
+/* U <- U - K1 - K2 and W = omega V + K2 - K1 for (nocc nvirt x m) column blocks from the same Kall (double when fp64): the
+ * products (A+B) V and (A-B) V from the Coulomb products U. */
+int dftb_exchange_combine(int m, int nvirt, int nocc, int fp64, const void *Kall, const double *omega, const double *V,
+                          double *U, double *W, void *stream);
 
 /* General FP64 product C = alpha * op(A) . op(B) + beta * C on row-major
  * matrices (op = transpose when trans != 0), the contraction engine behind the
