@@ -936,6 +936,22 @@ __global__ void rv_inplace_kernel(long long total, int nvec, const double *omega
     us[i] = omega[i / nvec] * vs[i] + fac * us[i];
 }
 
+// a launch that may overlap the end of the kernel before it on the stream
+template <typename K, typename P>
+cudaError_t launch_overlapped(K kernel, dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const P &p, bool overlap) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 template <int NT, bool HERM>
 int launch_qv(const QvP &p, unsigned rows, unsigned ks, unsigned cols, cudaStream_t st) {
     static bool attr_set[64] = {false};
@@ -947,7 +963,10 @@ int launch_qv(const QvP &p, unsigned rows, unsigned ks, unsigned cols, cudaStrea
             return fail(DFTB_ERR_CUDA, "coulomb: shared memory");
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    qv_kernel<NT, HERM><<<dim3(rows, ks, cols), QV_THREADS, Skinny<NT>::SMEM, st>>>(p);
+    if (p.after)
+        launch_overlapped(qv_kernel<NT, HERM>, dim3(rows, ks, cols), QV_THREADS, Skinny<NT>::SMEM, st, p, true);
+    else
+        qv_kernel<NT, HERM><<<dim3(rows, ks, cols), QV_THREADS, Skinny<NT>::SMEM, st>>>(p);
     return check_launch("qv_kernel");
 }
 
@@ -959,14 +978,14 @@ int launch_qv(const QvP &p, unsigned rows, unsigned ks, unsigned cols, cudaStrea
 // T = Q (s o V) for up to 32 columns at a time (T zeroed by the caller): the columns of Q are cut so that two
 // CTAs per SM are in flight
 int skinny_product(int M, int K, const double *Q, const double *V, int ncol, double *T, const double *omega,
-                   cudaStream_t st) {
+                   cudaStream_t st, bool after = false) {
     const unsigned rows = cdiv(M, QV_M), cols = cdiv(ncol, 32);
     const long long want = 296 / ((long long)rows * cols);
     const long long chunks = cdiv(K, QV_K);
     long long ks = want < 1 ? 1 : (want > chunks ? chunks : want);
     const long long per = (chunks + ks - 1) / ks;
     ks = (chunks + per - 1) / per;
-    const QvP p{M, K, Q, V, ncol, ncol, T, ncol, omega, (int)(per * QV_K)};
+    const QvP p{M, K, Q, V, ncol, ncol, T, ncol, omega, (int)(per * QV_K), after};
     switch (cols > 1 ? 4 : (int)cdiv(ncol, 8)) {
         case 1: return launch_qv<1>(p, rows, (unsigned)ks, cols, st);
         case 2: return launch_qv<2>(p, rows, (unsigned)ks, cols, st);
@@ -982,6 +1001,10 @@ int skinny_product(int M, int K, const double *Q, const double *V, int ncol, dou
 // and 8.1 ms in cuBLAS, 60 columns 12.6 ms in cuBLAS and 17 ms in two blocks).  The Hermitian form has no cuBLAS
 // route and takes as many blocks as it needs.
 constexpr int COULOMB_SKINNY = 32;
+// Kernels overlap at their seams up to this size of q_ov.  B200, 10 columns, overlapped and in turn: 0.1 MB 14.2 and 16.4 us,
+// 0.9 MB 20.5 and 24.6, 6.7 MB 27.6 and 29.7, 22 MB 38.1 and 37.9, 66 MB 52.0 and 51.8; beyond, the waiting CTAs of the last
+// kernel cost the first one more than the seams (997 MB, 30 columns: 841 and 799 us).
+constexpr long long OVERLAP_BYTES = 16 << 20;
 int coulomb_product(int nat, int nov, int nvec, const double *gamma, const double *q_ov, const double *omega,
                     const double *vs, double *us, double *T, double *G, int hermitian, cudaStream_t st) {
     // T and G are adjacent in the workspace: one memset zeroes both
@@ -1003,16 +1026,17 @@ int coulomb_product(int nat, int nov, int nvec, const double *gamma, const doubl
         rv_inplace_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(total, nvec, omega, vs, us, 4.0);
         return check_launch("rv_inplace_kernel");
     }
+    const bool overlap = 8LL * nat * nov <= OVERLAP_BYTES;
     if ((rc = skinny_product(nat, nov, q_ov, vs, nvec, T, hermitian ? omega : nullptr, st))) return rc;
-    if ((rc = skinny_product(nat, nat, gamma, T, nvec, G, nullptr, st))) return rc;
+    if ((rc = skinny_product(nat, nat, gamma, T, nvec, G, nullptr, st, overlap))) return rc;
     const QgP p{nov, nat, q_ov, G, nvec, nvec, omega, vs, us, 4.0, hermitian};
     const unsigned cols = cdiv(nvec, 32);
     const dim3 grid(cdiv(nov, QG_THREADS), cols);
     switch (cols > 1 ? 4 : (int)cdiv(nvec, 8)) {
-        case 1: qg_kernel<1><<<grid, QG_THREADS, 0, st>>>(p); break;
-        case 2: qg_kernel<2><<<grid, QG_THREADS, 0, st>>>(p); break;
-        case 3: qg_kernel<3><<<grid, QG_THREADS, 0, st>>>(p); break;
-        default: qg_kernel<4><<<grid, QG_THREADS, 0, st>>>(p); break;
+        case 1: launch_overlapped(qg_kernel<1>, grid, QG_THREADS, 0, st, p, overlap); break;
+        case 2: launch_overlapped(qg_kernel<2>, grid, QG_THREADS, 0, st, p, overlap); break;
+        case 3: launch_overlapped(qg_kernel<3>, grid, QG_THREADS, 0, st, p, overlap); break;
+        default: launch_overlapped(qg_kernel<4>, grid, QG_THREADS, 0, st, p, overlap); break;
     }
     return check_launch("qg_kernel");
 }
@@ -1612,7 +1636,7 @@ extern "C" int dftb_trans_charges_noalloc(int norb, int nat, int nocc, int nvirt
                  {q_vv, cv, scv, cv, scv, nvirt, nvirt}};
     for (auto &b : blks) {
         if (!b.out || b.n1 == 0 || b.n2 == 0) continue;
-        if ((rc = launch_tc(nat, b.n1, b.n2, first, b.c1, b.s1, b.c2, b.s2, b.out, st, "tc_tile_kernel (noalloc)")))
+        if ((rc = launch_tc(nat, b.n1, b.n2, first, b.c1, b.s1, b.c2, b.s2, b.out, st, "tc_kernel (noalloc)")))
             return rc;
     }
     return DFTB_OK;

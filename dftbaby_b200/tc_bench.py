@@ -1,4 +1,4 @@
-"""Microbenchmark of the transition-charge entry point (the source of the tc_tile_kernel profile).
+"""Microbenchmark of the transition-charge entry point (kernel times of tc_kernel and the S C product).
 
     python -m dftbaby_b200.tc_bench NAT NOCC NVIRT [REPS]
 
@@ -62,7 +62,7 @@ def main(argv=None):
     for k in prof.key_averages():
         if k.device_type.name == "CUDA" and k.device_time_total > 0:
             ms = k.device_time_total / 1e3
-            extra = " -> %.0f GB/s of q_ov writes" % (gb / (ms / 1e3)) if "tc_tile" in k.key else ""
+            extra = " -> %.0f GB/s of q_ov writes" % (gb / (ms / 1e3)) if "tc_kernel" in k.key else ""
             name = k.key.replace("(anonymous namespace)::", "").split("(")[0] or k.key
             print("  %-60s %8.3f ms%s" % (name[:60], ms, extra))
 
