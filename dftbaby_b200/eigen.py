@@ -8,10 +8,11 @@ SMALL = 128  # largest matrix of dftb_small_eigh: its orthogonal factor fills on
 
 
 def small(A):
-    """True for matrices (or batches of them) that dftb_small_eigh takes; autograd stays with torch."""
+    """True for matrices (or batches of them) that dftb_small_eigh takes; autograd and other devices than the current one
+    stay with torch."""
     return (type(A) is torch.Tensor and A.is_cuda and A.dtype == torch.float64 and A.dim() in (2, 3)
             and 0 < A.shape[-1] <= SMALL and A.shape[-2] == A.shape[-1] and A.shape[0] > 0
-            and not (A.requires_grad and torch.is_grad_enabled()))
+            and A.get_device() == torch.cuda.current_device() and not (A.requires_grad and torch.is_grad_enabled()))
 
 
 def small_eigh(A):
