@@ -33,7 +33,10 @@ namespace {
 #include "dmma.cuh"
 
 constexpr double EPS = 1.1102230246251565e-16;  // unit roundoff
-constexpr int SECULAR_ITERATIONS = 80;          // the bracket alone converges in fewer
+// The bracket alone converges in fewer: it is at most 4 wide, and deflation keeps a root at least 1e-33 from its pole, so
+// about 110 halvings reach the root's magnitude and 53 more its last bit.  (6 to 45 steps on tridiagonals of small
+// integers, Clement, Wilkinson and glued matrices.)
+constexpr int SECULAR_ITERATIONS = 192;
 
 // Shared memory: Z (rows in blocks of 8, pitch 4 mod 16 doubles: conflict-free reads of the tensor instruction's A
 // operand), U (pitch 8 mod 16: its B operand; 64 columns at a time), the vectors below.
@@ -101,8 +104,9 @@ __device__ __forceinline__ double quadratic(double c, double a, double b, bool l
 
 // Root j of 1/rho + sum_i z_i^2 / (d_i - lambda) (K poles d ascending, |z| = 1 at most) as lambda = d[origin] + x, the
 // origin being the nearer pole, so that d_i - lambda is known to full relative precision for every i.  A quad of lanes a
-// root, lane q summing the terms q, q + 4, ...; the warp's eight quads (of up to Kw poles each) iterate in step.  live: this quad has a root.
-__device__ void secular_roots(bool live, int K, int Kw, int j, const double *d, const double *z, double rho, int q,
+// root, lane q summing the terms q, q + 4, ...; the warp's eight quads (of up to Kw poles each) iterate in step.  live: this
+// quad has a root.  Returns whether this quad's root converged.
+__device__ bool secular_roots(bool live, int K, int Kw, int j, const double *d, const double *z, double rho, int q,
                               int *origin, double *xout) {
     const double ri = 1.0 / rho;
     const bool single = K < 2;
@@ -133,6 +137,10 @@ __device__ void secular_roots(bool live, int K, int Kw, int j, const double *d, 
     double x = quadratic(c, c * (dl + dr) + zl + zr, c * dl * dr + zl * dr + zr * dl, last);
     if (!(x > lo && x < hi)) x = 0.5 * (lo + hi);
     if (single) x = rho * z[0] * z[0];
+    // The middle is an end of the bracket but no pole, and a root may lie on it (matrices of small integers, symmetric
+    // chains): it is tried as a value when a step first leads there.
+    const double end = last || wm >= 0.0 ? mid : -mid;
+    bool untried = true;
     bool done = !live || single;
     for (int it = 0; it < SECULAR_ITERATIONS; ++it) {
         if (__all_sync(0xffffffffu, done)) break;
@@ -161,15 +169,22 @@ __device__ void secular_roots(bool live, int K, int Kw, int j, const double *d, 
         double eta = quadratic(last ? fabs(cc) : cc, (tl + tr) * w - tl * tr * dw, tl * tr * w, last);
         if (!(w * eta < 0.0)) eta = -w / dw;
         double xn = x + eta;
-        // a step this short against the distances to the poles is the last: its error is of second order in them
-        const bool short_step = fabs(eta) <= 1e-9 * fmin(fabs(tl), fabs(tr));
-        if (!(xn > lo && xn < hi)) xn = 0.5 * (lo + hi);
-        const bool full = xn == x || !(xn > lo && xn < hi);  // the bracket has no number left inside
+        // a step this short against the distances to the poles is the last, if it is taken: its error is of second order
+        // in them
+        bool last_step = fabs(eta) <= 1e-9 * fmin(fabs(tl), fabs(tr)), full = xn == x;
+        if (!full && !(xn > lo && xn < hi)) {
+            const bool try_end = untried && (w < 0.0 ? hi : lo) == end;
+            xn = try_end ? end : 0.5 * (lo + hi);
+            untried = untried && !try_end;
+            full = !try_end && !(xn > lo && xn < hi);  // the bracket has no number left inside
+            last_step = false;
+        }
         if (!done && !full) x = xn;
-        done = done || full || short_step;
+        done = done || full || last_step;
     }
     *origin = org;
     *xout = x;
+    return done;
 }
 
 // Deflation of one merge (positions off .. off + s of the sorted d and z) by one warp: the kept poles to kd, kz, slot;
@@ -257,7 +272,8 @@ template <int NC> __device__ int column_list(const Vectors<NC> &sv, int *list, i
 }
 
 // n <= 32 NC.  A: lower triangle of batch matrices, element (i, j) at A[b * sb + i * si + j * sj].  W: ascending
-// eigenvalues (batch x n).  V: vector j of matrix b at V[(b n + j) n ..].  info[b]: 0, or 1 for a matrix that is not finite.
+// eigenvalues (batch x n).  V: vector j of matrix b at V[(b n + j) n ..].  info[b]: 0, 1 for a matrix that is not finite, or 2
+// for a root that did not converge.
 // V may be A when si = n, sj = 1, sb = n n: it is written after A has been read.
 template <int NC>
 __global__ void __launch_bounds__(128 * NC, 1)
@@ -500,7 +516,7 @@ __global__ void __launch_bounds__(128 * NC, 1)
         const double *kd = sv.kd + (merging ? off : 0), *kz = sv.kz + (merging ? off : 0);
         int org = 0;
         double x = 0.0;
-        if (Kw > 0) secular_roots(live, Kc, Kw, jc, kd, kz, merging ? sv.rho[m] : 1.0, q4, &org, &x);
+        if (Kw > 0 && !secular_roots(live, Kc, Kw, jc, kd, kz, merging ? sv.rho[m] : 1.0, q4, &org, &x)) sv.bad = 2;
         if (live && q4 == 0) {
             sv.org[pos] = org;
             sv.x[pos] = x;
@@ -708,7 +724,7 @@ __global__ void __launch_bounds__(128 * NC, 1)
             for (int i = lane; i < n; i += 32) dst[i] = Z[i * zp + c];
         }
     }
-    if (tid == 0) info[blockIdx.x] = 0;
+    if (tid == 0) info[blockIdx.x] = sv.bad;
 }
 
 template <int NC>

@@ -34,5 +34,6 @@ def eigh(A):
         return torch.linalg.eigh(A)
     w, V, info = small_eigh(A)
     if bool(info.any()):
-        raise torch.linalg.LinAlgError("linalg.eigh: the input matrix contains non-finite values")
+        raise torch.linalg.LinAlgError("linalg.eigh: " + ("the input matrix contains non-finite values" if bool(
+            (info == 1).any()) else "the eigenvalues did not converge"))
     return w, V

@@ -432,7 +432,8 @@ const char *dftb_eigh_last_error(void);
 /* Small matrices, n <= DFTB_SMALL_EIGH_MAX: the whole batch in one launch of the library's own kernel, without a workspace.
  * Matrix b, element (i, j) at A[b * batch_stride + i * row_stride + j * col_stride]; the lower triangle is read.  W:
  * batch x n eigenvalues, ascending; V: batch x n x n, eigenvector j of matrix b in row j of block b (V may be A when A is
- * contiguous); info: batch status words, 0 or 1 (the matrix holds a number that is not finite; W and V are NaN). */
+ * contiguous); info: batch status words, 0, 1 (the matrix holds a number that is not finite; W and V are NaN) or 2 (an
+ * eigenvalue did not converge). */
 #define DFTB_SMALL_EIGH_MAX 128
 int dftb_small_eigh(int n, int batch, const double *A, long long batch_stride, long long row_stride, long long col_stride,
                     double *W, double *V, int *info, void *stream);
