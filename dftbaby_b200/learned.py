@@ -70,6 +70,20 @@ def _ksplit(M, N, K):
     return max(1, min(64, tcgemm.SMS // tiles, K // 512))
 
 
+def _plain(x, shape, like):
+    """x can go to a kernel as it is: a contiguous FP32 tensor of this shape on the device of `like`."""
+    return (type(x) is torch.Tensor and x.dtype == torch.float32 and x.shape == shape and x.is_contiguous()
+            and x.device == like.device)
+
+
+def _assigned(x, shape, like):
+    """x as an assignment to an FP32 tensor of this shape on the device of `like` would put it there: broadcast, converted
+    and copied from another device."""
+    out = torch.empty(shape, dtype=torch.float32, device=like.device)
+    out[...] = x
+    return out
+
+
 class GuessNet:
     """The pair-scoring network: FP32 master weights, BF16 copies, Adam state, feature statistics."""
 
@@ -109,13 +123,20 @@ class GuessNet:
         (64 x Ns) and the sum of the weights, added to msum."""
         n = feats.shape[0]
         ns = (n + SPAD - 1) // SPAD * SPAD
-        F = torch.broadcast_to(feats.float(), (n, NFEAT))
-        if F.stride(1) != 1 or F.stride(0) < F.shape[1]:
-            F = F.contiguous()
+        mean, std = self.mean, self.std
+        if (feats.device == self.W1.device and feats.shape == (n, NFEAT) and _plain(mean, (NFEAT,), self.W1)
+                and _plain(std, (NFEAT,), self.W1)):
+            F = feats.float()
+            if F.stride(1) != 1 or F.stride(0) < NFEAT:
+                F = F.contiguous()
+        else:
+            # torch's own rules on shapes, types and devices; the kernel then subtracts 0 and divides by 1
+            F = _assigned((feats.float() - mean) / std, (n, NFEAT), self.W1)
+            mean, std = torch.zeros_like(F[0]), torch.ones_like(F[0])
         X = torch.empty((ns, FPAD), dtype=torch.bfloat16, device=self.device)
         XT = torch.empty((FPAD, ns), dtype=torch.bfloat16, device=self.device) if weights is not None else None
         P = native.ptr
-        native.call("dftb_mlp_inputs", n, ns, NFEAT, FPAD, P(F), max(NFEAT, F.stride(0)), P(self.mean), P(self.std),
+        native.call("dftb_mlp_inputs", n, ns, NFEAT, FPAD, P(F), max(NFEAT, F.stride(0)), P(mean), P(std),
                     P(X), FPAD, P(XT), ns, P(weights), P(msum), native.stream())
         return X, XT, ns
 
@@ -156,7 +177,9 @@ class GuessNet:
         against the CPU oracle."""
         dev, P, st = self.device, native.ptr, native.stream()
         n = feats.shape[0]
-        m = torch.broadcast_to(weights.float().to(dev), (n,)).contiguous()
+        m = weights.float()
+        if not _plain(m, (n,), self.W1):
+            m = _assigned(m, (n,), self.W1)
         # one zeroed buffer for everything that is summed into (each gradient on a 16-byte boundary); the forward pass
         # is launched before its views are made
         sizes = [(p.numel() + 3) // 4 * 4 for p in self.params]
@@ -164,13 +187,16 @@ class GuessNet:
         loss, msum = flat[-4:].view(torch.float64).split(1)
         X, XT, ns = self._inputs(feats, m, msum)
         H1, H1T, H2 = self._forward(X, ns, keep=True)
-        T = torch.broadcast_to(targets.float(), (n, NOUT)).contiguous()
+        T, tscale = targets.float(), self.target_scale
+        if not (_plain(T, (n, NOUT), self.W1) and _plain(tscale, (NOUT,), self.W1)):
+            T = _assigned(T * tscale, (n, NOUT), self.W1)
+            tscale = torch.ones_like(T[0])
         grads = [f[:p.numel()].view(p.shape) for f, p in zip(flat[:-4].split(sizes), self.params)]
         dW1, db1, dW2, db2, dW3, db3 = grads
         dZ2 = torch.empty((ns, HIDDEN), dtype=torch.bfloat16, device=dev)
         dZ2T = torch.empty((HIDDEN, ns), dtype=torch.bfloat16, device=dev)
         native.call("dftb_mlp_head", ns, n, HIDDEN, P(H2), HIDDEN, P(self.W3b), HIDDEN, P(self.b3), P(T),
-                    P(self.target_scale), P(m), float(out_weights[0]), float(out_weights[1]), P(msum), None, P(dZ2),
+                    P(tscale), P(m), float(out_weights[0]), float(out_weights[1]), P(msum), None, P(dZ2),
                     HIDDEN, P(dZ2T), ns, P(dW3), P(db3), P(db2), P(loss), st)
         _mm(dZ2T, H1T, HIDDEN, HIDDEN, ns, dW2, _ksplit(HIDDEN, HIDDEN, ns), zeroed=True)
         _, dZ1T = self._dense(dZ2, self.W2bT, HIDDEN, ns, mask=H1, out=False, out_t=True, colsum=db1)
