@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(256) head_kernel(int ns, int n, int nh_, const
 #pragma unroll
         for (int o = 0; o < HEAD_NO; ++o)
             wl[o][e] = 8 * lane < nh ? __bfloat162float(W[(size_t)o * ldw + 8 * lane + e]) : 0.0f;
-    const float inv_norm = T ? (float)(1.0 / fmax(*msum, 1e-30)) : 0.0f;
+    const double wsum = T ? *msum : 1.0;
+    const float inv_norm = (float)(1.0 / (wsum < 1e-30 ? 1e-30 : wsum));  // not a number if a weight is not
     float2 dw0 = make_float2(0.0f, 0.0f), dw1 = dw0, dbh = dw0;  // of units u0 and u0 + 1, for one half of each tile's samples
     const int u0 = 2 * (tid & 127), half = tid >> 7;
     float dbo = 0.0f;  // output tid % 2
