@@ -10,6 +10,7 @@
 #pragma once
 
 #include "dmma.cuh"
+#include "qv_pieces.cuh"
 
 __device__ __forceinline__ void cp_async8(void *dst, const double *src, bool valid) {
     // 8-byte asynchronous copy; with src-size 0 the destination is zero-filled and nothing is read
@@ -39,7 +40,7 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 // form four warps turn omega into sqrt(omega) every fourth stage (a square root is a long serial chain, so it should
 // hold the stage's barrier up as seldom as possible), and the V fragments are multiplied as they are read.  Two CTAs per SM keep ~100 KB in flight.  The row pitches are 4 (mod 16) doubles, which keeps the fragment
 // reads (nearly) conflict-free.
-constexpr int QV_M = 64, QV_K = 32, QV_P = 36, QV_STAGES = 4, QV_THREADS = 256;
+constexpr int QV_M = 64, QV_P = 36, QV_STAGES = 4, QV_THREADS = 256;
 
 template <int NT> struct Skinny {  // NT tiles of 8 columns
     static constexpr int PITCH = 8 * NT + 4;
@@ -70,25 +71,17 @@ __global__ void __launch_bounds__(QV_THREADS, 2) qv_kernel(const QvP p) {
     const int ncol = min(NCOL, p.ncol - c0);
     const int kbeg = blockIdx.y * p.kper, kend = min(p.K, kbeg + p.kper);
     const int niter = kend > kbeg ? (kend - kbeg + QV_K - 1) / QV_K : 0;
-    // 1 for a row whose window (from a multiple of 32 columns) starts 8 bytes off the 16-byte grid
     grid_launch_dependents();
     if (p.after) grid_wait();
-    auto phase = [&](int row) {
-        return (int)(((reinterpret_cast<uintptr_t>(p.Q) >> 3) + (size_t)row * p.K + kbeg) & 1);
-    };
+    auto phase = [&](int row) { return qv_phase(p.Q, p.K, row, kbeg); };
     // this thread's pieces of Q: number tid % 16 of rows tid / 16 + 16 j, and the 17th of row tid
     const int pc = tid & 15;
-    const double *src[ROWS], *src17 = nullptr;
-    int left[ROWS];  // elements from the piece's first to the end of the range (<= 0: nothing to read)
+    QvPiece piece[ROWS];
+    const double *src17 = nullptr;
 #pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-        const int row = row0 + (tid >> 4) + 16 * j;
-        const bool v = row < p.M;
-        const int ph = v ? phase(row) : 0, k = kbeg - ph + 2 * pc;
-        src[j] = v ? p.Q + ((ptrdiff_t)row * p.K + k) : p.Q;
-        left[j] = v ? kend - k : 0;
-    }
-    if (tid < QV_M && row0 + tid < p.M && phase(row0 + tid)) src17 = p.Q + ((size_t)(row0 + tid) * p.K + kbeg + 31);
+    for (int j = 0; j < ROWS; ++j) piece[j] = qv_piece(p.Q, p.M, p.K, row0 + (tid >> 4) + 16 * j, kbeg, kend, pc);
+    if (tid < QV_M && row0 + tid < p.M && phase(row0 + tid))
+        src17 = qv_piece(p.Q, p.M, p.K, row0 + tid, kbeg, kend, 16).src;
     auto stage = [&](int it) {
         if (it < niter) {
             double *q = qv_sm + (it % QV_STAGES) * C::STAGE, *v = q + QV_M * QV_P;
@@ -96,9 +89,9 @@ __global__ void __launch_bounds__(QV_THREADS, 2) qv_kernel(const QvP p) {
 #pragma unroll
             for (int j = 0; j < ROWS; ++j) {
                 double *dst = q + ((tid >> 4) + 16 * j) * QV_P + 2 * pc;
-                const int n = min(2, max(0, left[j] - k0));
-                if (src[j] + k0 >= p.Q)
-                    cp_async16(dst, n > 0 ? src[j] + k0 : src[j] + (p.Q > src[j]), 8 * n);
+                const int n = min(2, max(0, piece[j].left - k0));
+                if (piece[j].src + k0 >= p.Q)
+                    cp_async16(dst, qv_source(piece[j], p.Q, k0, n), 8 * n);
                 else  // the very first element of a Q that is itself off the grid: nothing lies before it
                     cp_async8(dst + 1, p.Q, n > 1);
             }
