@@ -1,18 +1,27 @@
 """Symmetric eigensolver of the SCC and of the projected problems: the library's own one-launch kernel for small FP64
 matrices on the GPU, torch.linalg.eigh for all others."""
 import torch
+import torch.autograd.forward_ad as forward_ad
 
 from . import native
 
 SMALL = 128  # largest matrix of dftb_small_eigh: its orthogonal factor fills one SM's shared memory
 
 
+def _watched():
+    """Inside vmap and the other function transforms, forward-mode differentiation or tracing: the values in memory are not
+    all that a call has to hand on, so it belongs to torch."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing())
+
+
 def small(A):
-    """True for matrices (or batches of them) that dftb_small_eigh takes; autograd and other devices than the current one
-    stay with torch."""
+    """True for matrices (or batches of them) that dftb_small_eigh takes; autograd, function transforms, tracing and other
+    devices than the current one stay with torch."""
     return (type(A) is torch.Tensor and A.is_cuda and A.dtype == torch.float64 and A.dim() in (2, 3)
             and 0 < A.shape[-1] <= SMALL and A.shape[-2] == A.shape[-1] and A.shape[0] > 0
-            and A.get_device() == torch.cuda.current_device() and not (A.requires_grad and torch.is_grad_enabled()))
+            and A.get_device() == torch.cuda.current_device() and not (A.requires_grad and torch.is_grad_enabled())
+            and not A.is_neg() and not _watched())
 
 
 def small_eigh(A):
