@@ -81,14 +81,24 @@ def contract(geo, par, r_lr, XS, XH, Yg, Ylr, vrep):
     P = native.ptr
     t = par.device_tables(dev)
     r, x, y, z = geo.dircos
-    rows = lambda A: A if A is None or (A.stride(1) == 1 and A.stride(0) >= norb) else A.contiguous()
-    ld = lambda A: 0 if A is None else max(norb, A.stride(0))
-    XS, XH, Yg, Ylr = rows(XS), rows(XH), rows(Yg), rows(Ylr)
+    shape, index = (norb, norb), geo.pos.get_device()
+
+    def rows(A):
+        if A is None:
+            return None, 0
+        if A.shape != shape:
+            A = A.expand(shape)
+        if A.dtype != torch.float64 or A.get_device() != index or A.is_meta:
+            raise RuntimeError("contract: adjoints are FP64 tensors on the molecule's device")
+        s0, s1 = A.stride()
+        return (A, s0) if s1 == 1 and s0 >= norb else (A.contiguous(), norb)
+
+    (XS, ldxs), (XH, ldxh), (Yg, ldyg), (Ylr, ldylr) = rows(XS), rows(XH), rows(Yg), rows(Ylr)
     out = torch.empty(3 * nat, dtype=torch.float64, device=dev)
     native.call("dftb_gradient_contract", norb, nat, P(geo.ind), P(geo.typ), P(geo.ls), P(geo.ms), P(r), P(x), P(y), P(z),
                 P(geo.mprox), par.deg, P(t["tab_filled_SH0"]), P(t["S_knots"]), P(t["S_coefs"]), P(t["H_knots"]),
                 P(t["H_coefs"]), par.npair, par.nsk, par.npts, P(geo.pos), P(geo.atype), P(geo.sigma), float(r_lr), P(XS),
-                ld(XS), P(XH), ld(XH), P(Yg), ld(Yg), P(Ylr), ld(Ylr), P(t["vrep_knots"]) if vrep else None,
+                ldxs, P(XH), ldxh, P(Yg), ldyg, P(Ylr), ldylr, P(t["vrep_knots"]) if vrep else None,
                 P(t["vrep_coefs"]), P(t["vrep_dmax"]), par.vrep_nknots, P(out), native.stream())
     return out
 
