@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(QG_THREADS) qg_kernel(const QgP p) {
     const int c0 = blockIdx.y * NCOL, ncol = min(NCOL, p.ncol - c0);
     const int ia0 = (blockIdx.x * (QG_THREADS / 32) + warp) * 32;
     const int nchunk = (p.nat + QG_K - 1) / QG_K;
+    grid_launch_dependents();
     double gr[GREG];
     auto load_g = [&](int ch) {
 #pragma unroll

@@ -435,12 +435,12 @@ constexpr int PITCH_K = BK + 4, PITCH_MN = BM + 4;  // operand tiles [m or n][k]
 
 // AK: A is contiguous along k (else staged along m); BNC: B is contiguous along n (else staged along k)
 template <int EPI, bool AK, bool BNC>
-__global__ void __launch_bounds__(GEMM_THREADS) dgemm_kernel(const GemmP p) {
+__device__ __forceinline__ void dgemm_tile(const GemmP &p, int bx, int by, int bz) {
     constexpr int A_ELEMS = AK ? BM * PITCH_K : BK * PITCH_MN, B_ELEMS = BNC ? BK * PITCH_MN : BN * PITCH_K;
     extern __shared__ __align__(16) double gemm_sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int bm = blockIdx.y * p.mstep, bn = blockIdx.x * BN, M = min(p.M, bm + p.mstep);
-    const int zb = blockIdx.z / p.ksplit, zk = blockIdx.z % p.ksplit;
+    const int bm = by * p.mstep, bn = bx * BN, M = min(p.M, bm + p.mstep);
+    const int zb = bz / p.ksplit, zk = bz % p.ksplit;
     const double *A = p.A + zb * p.sa1, *B = p.B + zb * p.sb1;
     double *C = p.C + zb * p.sc1;
     const int kchunk = ((p.K + p.ksplit - 1) / p.ksplit + BK - 1) / BK * BK;
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) dgemm_kernel(const GemmP p) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
     // neighbouring CTAs swap the upper and lower warps, so that short tiles do not all fall to the same SM quarters
-    const int wm = 32 * ((warp ^ blockIdx.x) & 1), wn = 32 * (warp >> 1);
+    const int wm = 32 * ((warp ^ bx) & 1), wn = 32 * (warp >> 1);
     const int mtiles = min(4, max(0, (M - bm - wm + 7) / 8)), ntiles = min(4, max(0, (p.N - bn - wn + 7) / 8));
     const int arow = wm + (lane >> 2), acol = lane & 3, bcol_l = wn + (lane >> 2);
     for (int s = 0; s < GEMM_STAGES - 1; ++s) stage(s);
@@ -549,6 +549,59 @@ __global__ void __launch_bounds__(GEMM_THREADS) dgemm_kernel(const GemmP p) {
         }
 }
 
+template <int EPI, bool AK, bool BNC>
+__global__ void __launch_bounds__(GEMM_THREADS) dgemm_kernel(const GemmP p) {
+    dgemm_tile<EPI, AK, BNC>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Several independent products in one launch: CTAs first[t] .. first[t + 1] - 1 take the tiles of product t.
+constexpr int GROUP = 4;
+struct GemmGroup {
+    GemmP p[GROUP];
+    int gx[GROUP], gy[GROUP], first[GROUP + 1];
+    int n;
+};
+
+// WAIT_FIRST: the operands come from the kernel before, which this launch may overlap; else they do not, and the wait at the
+// end only hands the order of the launches on to the next one.
+template <int EPI, bool WAIT_FIRST>
+__global__ void __launch_bounds__(GEMM_THREADS) dgemm_group_kernel(const __grid_constant__ GemmGroup g) {
+    int t = 0;
+    while (t + 1 < g.n && (int)blockIdx.x >= g.first[t + 1]) ++t;
+    const GemmP &p = g.p[t];
+    const int b = blockIdx.x - g.first[t], bx = b % g.gx[t], r = b / g.gx[t], by = r % g.gy[t], bz = r / g.gy[t];
+    grid_launch_dependents();
+    if (WAIT_FIRST) grid_wait();
+    if (p.sbn == 1) {
+        if (p.sak == 1)
+            dgemm_tile<EPI, true, true>(p, bx, by, bz);
+        else
+            dgemm_tile<EPI, false, true>(p, bx, by, bz);
+    } else {
+        if (p.sak == 1)
+            dgemm_tile<EPI, true, false>(p, bx, by, bz);
+        else
+            dgemm_tile<EPI, false, false>(p, bx, by, bz);
+    }
+    if (!WAIT_FIRST) grid_wait();
+}
+
+// a launch that may overlap the end of the kernel before it on the stream
+template <typename K, typename P>
+cudaError_t launch_overlapped(K kernel, dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const P &p, bool overlap) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 GemmP gemm_defaults() {
     GemmP p;
     memset(&p, 0, sizeof(p));
@@ -574,17 +627,35 @@ int launch_gemm_as(const GemmP &p, dim3 grid, cudaStream_t st) {
     return check_launch("dgemm_kernel");
 }
 
-int launch_gemm(GemmP p, int epi, int nbatch, cudaStream_t st) {
-    if (p.M <= 0 || p.N <= 0 || nbatch <= 0) return DFTB_OK;
+// the grid of a product, and its parameters brought to the form that the kernel reads; an error code
+int plan_gemm(GemmP &p, int nbatch, dim3 &grid) {
     if (p.K <= 0) return fail(DFTB_ERR_BAD_SIZE, "gemm: K <= 0");
     if (p.K2 == 0) p.K2 = p.K;
     if (p.N2 == 0) p.N2 = p.N;
+    // an inner index of one value: its stride is never taken, and the outer one says how the operand lies in memory
+    if (p.K2 == 1) {
+        p.sak = p.sak1;
+        p.K2 = p.K;
+    }
+    if (p.N2 == 1) {
+        p.sbn = p.sbn1;
+        p.scn = p.scn1;
+        p.N2 = p.N;
+    }
     const int mblocks = (int)cdiv(p.M, BM);
     p.mstep = 8 * (int)cdiv(cdiv(p.M, 8), mblocks);
-    dim3 grid(cdiv(p.N, BN), mblocks, (unsigned)(nbatch * p.ksplit));
+    grid = dim3(cdiv(p.N, BN), mblocks, (unsigned)(nbatch * p.ksplit));
     if (grid.y > 65535u || grid.z > 65535u) return fail(DFTB_ERR_BAD_SIZE, "gemm: grid too large");
+    if (p.K2 != p.K && p.sak != 1) return fail(DFTB_ERR_BAD_SIZE, "gemm: two-level k");
+    return DFTB_OK;
+}
+
+int launch_gemm(GemmP p, int epi, int nbatch, cudaStream_t st) {
+    if (p.M <= 0 || p.N <= 0 || nbatch <= 0) return DFTB_OK;
+    dim3 grid;
+    const int rc = plan_gemm(p, nbatch, grid);
+    if (rc) return rc;
     const bool ak = p.sak == 1, bn = p.sbn == 1;
-    if (p.K2 != p.K && !ak) return fail(DFTB_ERR_BAD_SIZE, "gemm: two-level k");
     if (epi == EPI_STORE)
         return ak ? (bn ? launch_gemm_as<EPI_STORE, true, true>(p, grid, st)
                         : launch_gemm_as<EPI_STORE, true, false>(p, grid, st))
@@ -596,11 +667,37 @@ int launch_gemm(GemmP p, int epi, int nbatch, cudaStream_t st) {
                     : launch_gemm_as<EPI_ATOMIC, false, false>(p, grid, st));
 }
 
-// K ranges so that about two CTAs per SM are in flight, at least four stages each (C40H42's 32 tiles of K = 8282: two
-// CTAs 76 us, four 80 us a product; C20H22's five tiles of K = 2142: four stages 9 us, sixteen 21 us)
-int pick_ksplit(int M, int N, int K) {
+// n products in one launch that may overlap the end of the kernel before it
+template <int EPI, bool WAIT_FIRST>
+int launch_gemm_group(const GemmP *p, const int *nbatch, int n, cudaStream_t st) {
+    constexpr int smem = GEMM_STAGES * (int)sizeof(double) * 2 * BM * PITCH_K;  // the larger staging order of both operands
+    GemmGroup g;
+    memset(&g, 0, sizeof(g));
+    g.n = n;
+    long long ctas = 0;
+    for (int t = 0; t < n; ++t) {
+        dim3 grid;
+        g.p[t] = p[t];
+        const int rc = plan_gemm(g.p[t], nbatch[t], grid);
+        if (rc) return rc;
+        g.gx[t] = (int)grid.x;
+        g.gy[t] = (int)grid.y;
+        g.first[t] = (int)ctas;
+        ctas += (long long)grid.x * grid.y * grid.z;
+    }
+    if (ctas > (1LL << 30)) return fail(DFTB_ERR_BAD_SIZE, "gemm: grid too large");
+    g.first[n] = (int)ctas;
+    cudaError_t e = cudaFuncSetAttribute(dgemm_group_kernel<EPI, WAIT_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem);
+    if (e != cudaSuccess) return fail(DFTB_ERR_CUDA, "gemm: shared memory");
+    launch_overlapped(dgemm_group_kernel<EPI, WAIT_FIRST>, dim3((unsigned)ctas), GEMM_THREADS, smem, st, g, true);
+    return check_launch("dgemm_group_kernel");
+}
+
+// K ranges so that about `ctas` CTAs are in flight, of at least `stages` stages each
+int pick_ksplit(int M, int N, int K, int ctas, int stages) {
     const long long tiles = (long long)cdiv(M, BM) * cdiv(N, BN);
-    const long long want = (148LL * 2) / tiles, most = K / (4 * BK);
+    const long long want = ctas / tiles, most = K / (stages * BK);
     return (int)(want < 1 || most < 1 ? 1 : (want < most ? want : most));
 }
 
@@ -923,6 +1020,7 @@ __global__ void sqrt_kernel(int n, double *x) {
 // us = omega o vs (the first term of (A-B).v without Coulomb)
 __global__ void omega_scale_kernel(long long nov, int nvec, const double *omega, const double *vs, double *us) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_launch_dependents();  // the exchange products may start
     if (idx >= nov * nvec) return;
     us[idx] = omega[idx / nvec] * vs[idx];
 }
@@ -934,22 +1032,6 @@ __global__ void rv_inplace_kernel(long long total, int nvec, const double *omega
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     us[i] = omega[i / nvec] * vs[i] + fac * us[i];
-}
-
-// a launch that may overlap the end of the kernel before it on the stream
-template <typename K, typename P>
-cudaError_t launch_overlapped(K kernel, dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const P &p, bool overlap) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 template <int NT, bool HERM>
@@ -1043,122 +1125,130 @@ int coulomb_product(int nat, int nov, int nvec, const double *gamma, const doubl
 
 // Exchange terms in the transition-charge form, accumulated into us:
 //   us += sK1 * K1 v + sK2 * K2 v
-// Each term is a batched product per atom, laid out so that the sum over atoms and one orbital index is then a single
+//   K1 v(i; a,c) = sum_{B,j} Z[B](i,j) Y[B][j](a,c),  Z[B](i,j) = sum_A g_lr[A][B] q_oo[A](i,j),
+//                                                     Y[B][j](a,c) = sum_b q_vv[B](a,b) v(j,b,c)
+//   K2 v(i; a,c) = sum_{B,b} Z2[B](i,b) W[B][b](a,c),  Z2[B](i,b) = sum_A g_lr[A][B] q_ov[A](i,b),
+//                                                      W[B][b](a,c) = sum_j q_ov[B](j,a) v(j,b,c)
+// Y and W are batched products per atom, laid out so that the sum over atoms and one orbital index is then a single
 // product of that length with whole (orbital, vector) rows (a product per atom and vector, added into us with atomics,
 // ran at 7 TFLOP/s).  B200, C40H42 (82 atoms, 101 x 101 orbitals), 10 vectors, (A+B).V and (A-B).V: 1820 -> 840 us.
+//
+// Small molecules are bound by launches and by the latency of a chain of short products: for them Z, Y, Z2 and W, which do
+// not depend on one another, are one launch, and the two sums another; the first runs beside the Coulomb product's last
+// kernel.  (A+B).V on B200, us with six launches and with two: C6H8 (14 atoms, 16 x 16 orbitals), 1 vector 37 and 16 (a
+// product per atom and vector: 25), C10H12 46 and 22 (40), C20H22, 10 vectors 78 and 55 (125).  Up to this much scratch for
+// both terms: C44H46, 1 vector, 35 MB, 126 and 120 us; C30H32, 10 vectors, 63 MB, 199 and 228.
+constexpr size_t EXCHANGE_GROUPED_BYTES = (size_t)36 << 20;
+
+// scratch elements of the two terms
+void exchange_scratch(int nat, int nocc, int nvirt, int nvec, size_t *k1, size_t *k2) {
+    const size_t no = nocc, nv = nvirt, m = nvec, na = nat;
+    *k1 = na * no * no + na * no * nv * m;
+    *k2 = na * no * nv + na * nv * nv * m;
+}
+
 int exchange_products(int nat, int nocc, int nvirt, int nvec, const double *g_lr, const double *q_oo,
                       const double *q_ov, const double *q_vv, const double *vs, double *us, double sK1, double sK2,
-                      double *work, cudaStream_t st) {
+                      double *work, size_t work_bytes, cudaStream_t st) {
     const long long no = nocc, nv = nvirt, m = nvec;
+    size_t k1, k2;
+    exchange_scratch(nat, nocc, nvirt, nvec, &k1, &k2);
+    const size_t both = sizeof(double) * (k1 + k2);
+    const bool grouped = both <= EXCHANGE_GROUPED_BYTES && work_bytes >= both;
+    double *Z = work, *Y = Z + nat * no * no, *Z2 = grouped ? work + k1 : work, *W = Z2 + nat * no * nv;
+    GemmP q[4], k[2];  // Z, Y, Z2, W; K1 v, K2 v
+    for (int t = 0; t < 4; t += 2) {  // (A, orbital pairs) from the charges of all atoms
+        GemmP &p = q[t] = gemm_defaults();
+        const long long pairs = no * (t ? nv : no);
+        p.M = nat;
+        p.N = (int)pairs;
+        p.K = nat;
+        p.A = g_lr;
+        p.sam = 1;
+        p.sak = nat;
+        p.B = t ? q_ov : q_oo;
+        p.sbk = pairs;
+        p.sbn = 1;
+        p.C = t ? Z2 : Z;
+        p.scm = pairs;
+        p.scn = 1;
+    }
+    {
+        GemmP &p = q[1] = gemm_defaults();
+        p.M = (int)nv;        // a
+        p.N = (int)(no * m);  // (j, c)
+        p.N2 = (int)m;
+        p.K = (int)nv;  // b
+        p.A = q_vv;
+        p.sam = nv;
+        p.sak = 1;
+        p.sa1 = nv * nv;
+        p.B = vs;
+        p.sbk = m;
+        p.sbn1 = nv * m;
+        p.sbn = 1;
+        p.C = Y;
+        p.scm = m;
+        p.scn1 = nv * m;
+        p.scn = 1;
+        p.sc1 = no * nv * m;
+    }
+    {
+        GemmP &p = q[3] = gemm_defaults();
+        p.M = (int)nv;        // a
+        p.N = (int)(nv * m);  // (b, c)
+        p.N2 = (int)m;
+        p.K = (int)no;  // j
+        p.A = q_ov;
+        p.sam = 1;
+        p.sak = nv;
+        p.sa1 = no * nv;
+        p.B = vs;
+        p.sbk = nv * m;
+        p.sbn1 = m;
+        p.sbn = 1;
+        p.C = W;
+        p.scm = m;
+        p.scn1 = nv * m;
+        p.scn = 1;
+        p.sc1 = nv * nv * m;
+    }
+    for (int t = 0; t < 2; ++t) {
+        GemmP &p = k[t] = gemm_defaults();
+        const long long n = t ? nv : no;  // the orbital of the sum
+        p.M = (int)no;                    // i
+        p.N = (int)(nv * m);              // (a, c)
+        p.K = (int)(nat * n);
+        p.K2 = (int)n;
+        p.A = t ? Z2 : Z;
+        p.sam = n;
+        p.sak1 = no * n;
+        p.sak = 1;
+        p.B = t ? W : Y;
+        p.sbk = nv * m;
+        p.sbn = 1;
+        p.C = us;
+        p.scm = nv * m;
+        p.scn = 1;
+        p.alpha = t ? sK2 : sK1;
+        // Two CTAs per SM: C40H42's 32 tiles of K = 8282 take 76 us, with four 80; C20H22's five of K = 2142 9 us in ranges of
+        // four stages, 21 of sixteen.  Side by side the terms share them, and shorter ranges pay: C6H8's one tile of K = 224
+        // 19 us a call with four stages, 16 with two.
+        p.ksplit = grouped ? pick_ksplit(p.M, p.N, p.K, 148, 2) : pick_ksplit(p.M, p.N, p.K, 296, 4);
+    }
+    const int batch[4] = {1, nat, 1, nat};
     int rc;
-    // ---- K1: us(i; a,c) += sK1 sum_{B,j} Z[B](i,j) Y[B][j](a,c),
-    //          Z[B](i,j) = sum_A g_lr[A][B] q_oo[A](i,j),  Y[B][j](a,c) = sum_b q_vv[B](a,b) v(j,b,c)
-    double *Z = work, *Y = work + nat * no * no;
-    GemmP p = gemm_defaults();
-    p.M = nat;
-    p.N = (int)(no * no);
-    p.K = nat;
-    p.A = g_lr;
-    p.sam = 1;
-    p.sak = nat;
-    p.B = q_oo;
-    p.sbk = no * no;
-    p.sbn = 1;
-    p.C = Z;
-    p.scm = no * no;
-    p.scn = 1;
-    if ((rc = launch_gemm(p, EPI_STORE, 1, st))) return rc;
-    p = gemm_defaults();
-    p.M = (int)nv;  // a
-    p.N = (int)(no * m);  // (j, c)
-    p.N2 = (int)m;
-    p.K = (int)nv;  // b
-    p.A = q_vv;
-    p.sam = nv;
-    p.sak = 1;
-    p.sa1 = nv * nv;
-    p.B = vs;
-    p.sbk = m;
-    p.sbn1 = nv * m;
-    p.sbn = 1;
-    p.C = Y;
-    p.scm = m;
-    p.scn1 = nv * m;
-    p.scn = 1;
-    p.sc1 = no * nv * m;
-    if ((rc = launch_gemm(p, EPI_STORE, nat, st))) return rc;
-    p = gemm_defaults();
-    p.M = (int)no;  // i
-    p.N = (int)(nv * m);  // (a, c)
-    p.K = (int)(nat * no);  // (B, j)
-    p.K2 = (int)no;
-    p.A = Z;
-    p.sam = no;
-    p.sak1 = no * no;
-    p.sak = 1;
-    p.B = Y;
-    p.sbk = nv * m;
-    p.sbn = 1;
-    p.C = us;
-    p.scm = nv * m;
-    p.scn = 1;
-    p.alpha = sK1;
-    p.ksplit = pick_ksplit(p.M, p.N, p.K);
-    if ((rc = launch_gemm(p, EPI_ATOMIC, 1, st))) return rc;
-    // ---- K2: us(i; a,c) += sK2 sum_{A,b} q_ov[A](i,b) W[A][b](a,c),
-    //          Z2[A](j,a) = sum_B g_lr[A][B] q_ov[B](j,a),  W[A][b](a,c) = sum_j Z2[A](j,a) v(j,b,c)
-    double *Z2 = work, *W = work + nat * no * nv;
-    p = gemm_defaults();
-    p.M = nat;
-    p.N = (int)(no * nv);
-    p.K = nat;
-    p.A = g_lr;
-    p.sam = nat;
-    p.sak = 1;
-    p.B = q_ov;
-    p.sbk = no * nv;
-    p.sbn = 1;
-    p.C = Z2;
-    p.scm = no * nv;
-    p.scn = 1;
-    if ((rc = launch_gemm(p, EPI_STORE, 1, st))) return rc;
-    p = gemm_defaults();
-    p.M = (int)nv;  // a
-    p.N = (int)(nv * m);  // (b, c)
-    p.N2 = (int)m;
-    p.K = (int)no;  // j
-    p.A = Z2;
-    p.sam = 1;
-    p.sak = nv;
-    p.sa1 = no * nv;
-    p.B = vs;
-    p.sbk = nv * m;
-    p.sbn1 = m;
-    p.sbn = 1;
-    p.C = W;
-    p.scm = m;
-    p.scn1 = nv * m;
-    p.scn = 1;
-    p.sc1 = nv * nv * m;
-    if ((rc = launch_gemm(p, EPI_STORE, nat, st))) return rc;
-    p = gemm_defaults();
-    p.M = (int)no;  // i
-    p.N = (int)(nv * m);  // (a, c)
-    p.K = (int)(nat * nv);  // (A, b)
-    p.K2 = (int)nv;
-    p.A = q_ov;
-    p.sam = nv;
-    p.sak1 = no * nv;
-    p.sak = 1;
-    p.B = W;
-    p.sbk = nv * m;
-    p.sbn = 1;
-    p.C = us;
-    p.scm = nv * m;
-    p.scn = 1;
-    p.alpha = sK2;
-    p.ksplit = pick_ksplit(p.M, p.N, p.K);
-    return launch_gemm(p, EPI_ATOMIC, 1, st);
+    if (grouped) {
+        if ((rc = launch_gemm_group<EPI_STORE, false>(q, batch, 4, st))) return rc;
+        const int one[2] = {1, 1};
+        return launch_gemm_group<EPI_ATOMIC, true>(k, one, 2, st);
+    }
+    for (int t = 0; t < 2; ++t) {  // one term after the other in the same scratch
+        for (int h = 2 * t; h < 2 * t + 2; ++h)
+            if ((rc = launch_gemm(q[h], EPI_STORE, batch[h], st))) return rc;
+        if ((rc = launch_gemm(k[t], EPI_ATOMIC, 1, st))) return rc;
+    }
+    return DFTB_OK;
 }
 
 int check_products(int nat, int nocc, int nvirt, int nvec, int lc, const double *g, const double *g_lr,
@@ -1167,8 +1257,12 @@ int check_products(int nat, int nocc, int nvirt, int nvec, int lc, const double 
     if (nat <= 0 || nocc <= 0 || nvirt <= 0 || nvec <= 0) return fail(DFTB_ERR_BAD_SIZE, "apbv: sizes");
     if (!g || !q_ov || !omega || !vs || !us) return fail(DFTB_ERR_NULL, "apbv: null");
     if (lc && (!g_lr || !q_oo || !q_vv)) return fail(DFTB_ERR_NULL, "apbv: lc needs g_lr, q_oo, q_vv");
-    const size_t need = lc ? dftb_apbv_workspace_size(nat, nocc, nvirt, nvec)
-                           : dftb_hermitian_rv_workspace_size(nat, nvec);
+    size_t need = dftb_hermitian_rv_workspace_size(nat, nvec);
+    if (lc) {  // one exchange term at a time; dftb_apbv_workspace_size may ask for more, to run both side by side
+        size_t k1, k2;
+        exchange_scratch(nat, nocc, nvirt, nvec, &k1, &k2);
+        need += align256(sizeof(double) * (k1 > k2 ? k1 : k2));
+    }
     if (!work || work_bytes < need) return fail(DFTB_ERR_WORKSPACE, "apbv: workspace too small");
     return DFTB_OK;
 }
@@ -1412,10 +1506,12 @@ int dftb_hermitian_rv(int nat, int nocc, int nvirt, int nvec, const double *gamm
 
 size_t dftb_apbv_workspace_size(int nat, int nocc, int nvirt, int nvec) {
     if (nat <= 0 || nocc <= 0 || nvirt <= 0 || nvec <= 0) return 0;
-    const size_t no = nocc, nv = nvirt, m = nvec, na = nat;
-    const size_t k1 = na * no * no + na * no * nv * m;
-    const size_t k2 = na * no * nv + na * nv * nv * m;
-    return align256(sizeof(double) * (k1 > k2 ? k1 : k2)) + dftb_hermitian_rv_workspace_size(nat, nvec);
+    size_t k1, k2;
+    exchange_scratch(nat, nocc, nvirt, nvec, &k1, &k2);
+    const size_t serial = sizeof(double) * (k1 > k2 ? k1 : k2), both = sizeof(double) * (k1 + k2);
+    // never less for more atoms, orbitals or vectors, so that the size of the largest call serves the smaller ones
+    const size_t grouped = both < EXCHANGE_GROUPED_BYTES ? both : EXCHANGE_GROUPED_BYTES;
+    return align256(serial > grouped ? serial : grouped) + dftb_hermitian_rv_workspace_size(nat, nvec);
 }
 
 int dftb_apbv(int nat, int nocc, int nvirt, int nvec, int lc, const double *g, const double *g_lr,
@@ -1431,7 +1527,7 @@ int dftb_apbv(int nat, int nocc, int nvirt, int nvec, int lc, const double *g, c
     rc = coulomb_product(nat, nocc * nvirt, nvec, g, q_ov, omega, vs, us, T, G, 0, st);
     if (rc || !lc) return rc;
     return exchange_products(nat, nocc, nvirt, nvec, g_lr, q_oo, q_ov, q_vv, vs, us, -1.0, -1.0,
-                             (double *)((char *)work + coul), st);
+                             (double *)((char *)work + coul), work_bytes - coul, st);
 }
 
 int dftb_ambv(int nat, int nocc, int nvirt, int nvec, int lc, const double *g, const double *g_lr,
@@ -1446,7 +1542,7 @@ int dftb_ambv(int nat, int nocc, int nvirt, int nvec, int lc, const double *g, c
     if (!lc) return DFTB_OK;
     const size_t coul = dftb_hermitian_rv_workspace_size(nat, nvec);
     return exchange_products(nat, nocc, nvirt, nvec, g_lr, q_oo, q_ov, q_vv, vs, us, -1.0, +1.0,
-                             (double *)((char *)work + coul), st);
+                             (double *)((char *)work + coul), work_bytes - coul, st);
 }
 
 int dftb_davidson_precondition(int nov, int nnew, const double *W, int ldw, const int *src, const int *state,
