@@ -1077,30 +1077,59 @@ int skinny_product(int M, int K, const double *Q, const double *V, int ncol, dou
 }
 
 //   T = q_ov . (s o V)   (atomic over the column ranges), G = gamma . T,  us = epilogue(q_ov^T G)
-// The non-Hermitian form (s = 1) of more than COULOMB_SKINNY columns runs its two large GEMMs in cuBLAS when it
-// is available: row-major X (r x c) is the column-major X^T, so T^T = V^T q_ov^T and us^T = G^T q_ov.  The line is
-// where a second block of 32 columns would read q_ov again (C1014H90: 30 columns 8.4 ms here, 16 columns 5.3 ms here
-// and 8.1 ms in cuBLAS, 60 columns 12.6 ms in cuBLAS and 17 ms in two blocks).  The Hermitian form has no cuBLAS
-// route and takes as many blocks as it needs.
-constexpr int COULOMB_SKINNY = 32;
+// The Hermitian form takes as many blocks of 32 columns as it needs.  The non-Hermitian form (s = 1) runs its two large
+// GEMMs in cuBLAS, when it is available, where that is faster: row-major X (r x c) is the column-major X^T, so
+// T^T = V^T q_ov^T and us^T = G^T q_ov.  B200, us here and in cuBLAS:
+//   - more than 32 columns, where q_ov would be read a third and fourth time: 1104 atoms x 1225 x 1225, 60 columns 17000 and
+//     12600;
+//   - 25 to 32 columns, bound by the FP64 pipe, for many pairs: 1104 x 109k 661 and 690, 336 x 40k 116 and 147, but
+//     600 x 160k 570 and 542, 336 x 371k 765 and 655, 1104 x 1.5M 9050 and 7800 (24 columns: 589 and 650, 7470 and 7700);
+//   - one column of a long odd number of pairs, where every other row is off the 16-byte grid: 336 x 371k 346 and 374, but
+//     1104 x 642k 2005 and 1953, 700 x 1.5M 3430 and 2650 (even, 1104 x 1.0M: 2840 and 3010; two columns: 5000 and 7560).
+bool coulomb_in_blas(int nov, int nvec) {
+    return nvec > 32 || (nvec > 24 && nov > 120000) || (nvec == 1 && nov % 2 == 1 && nov > 500000);
+}
+// Atoms up to which the cuBLAS route forms gamma . T in one plain product: two launches less count for more there than
+// splitting the sum (14 atoms, 33 columns: 26 -> 23 us a call).
+constexpr int COULOMB_PLAIN = 48;
 // Kernels overlap at their seams up to this size of q_ov.  B200, 10 columns, overlapped and in turn: 0.1 MB 14.2 and 16.4 us,
 // 0.9 MB 20.5 and 24.6, 6.7 MB 27.6 and 29.7, 22 MB 38.1 and 37.9, 66 MB 52.0 and 51.8; beyond, the waiting CTAs of the last
 // kernel cost the first one more than the seams (997 MB, 30 columns: 841 and 799 us).
 constexpr long long OVERLAP_BYTES = 16 << 20;
 int coulomb_product(int nat, int nov, int nvec, const double *gamma, const double *q_ov, const double *omega,
                     const double *vs, double *us, double *T, double *G, int hermitian, cudaStream_t st) {
-    // T and G are adjacent in the workspace: one memset zeroes both
-    const size_t bytes = (size_t)((char *)G - (char *)T) + sizeof(double) * (size_t)nat * nvec;
-    cudaError_t e = cudaMemsetAsync(T, 0, bytes, st);
-    if (e != cudaSuccess) return fail(DFTB_ERR_CUDA, "memset T");
     int rc;
-    cublasHandle_t bh = hermitian || nvec <= COULOMB_SKINNY ? nullptr : blas_handle(st);
+    cublasHandle_t bh = hermitian || !coulomb_in_blas(nov, nvec) ? nullptr : blas_handle(st);
+    const bool plain = bh && nat <= COULOMB_PLAIN;
+    if (!plain) {
+        // T and G are adjacent in the workspace: one memset zeroes both
+        const size_t bytes = (size_t)((char *)G - (char *)T) + sizeof(double) * (size_t)nat * nvec;
+        if (cudaMemsetAsync(T, 0, bytes, st) != cudaSuccess) return fail(DFTB_ERR_CUDA, "memset T");
+    }
     if (bh) {
         const double one = 1.0, zero = 0.0;
         if (blas().dgemm(bh, CUBLAS_OP_N, CUBLAS_OP_N, nvec, nat, nov, &one, vs, nvec, q_ov, nov, &zero, T, nvec) !=
             CUBLAS_STATUS_SUCCESS)
             return fail(DFTB_ERR_CUDA, "coulomb: cublasDgemm (q_ov V) failed");
-        if ((rc = skinny_product(nat, nat, gamma, T, nvec, G, nullptr, st))) return rc;
+        if (plain) {
+            GemmP p = gemm_defaults();
+            p.M = nat;
+            p.N = nvec;
+            p.K = nat;
+            p.A = gamma;
+            p.sam = nat;
+            p.sak = 1;
+            p.B = T;
+            p.sbk = nvec;
+            p.sbn = 1;
+            p.C = G;
+            p.scm = nvec;
+            p.scn = 1;
+            rc = launch_gemm(p, EPI_STORE, 1, st);
+        } else {
+            rc = skinny_product(nat, nat, gamma, T, nvec, G, nullptr, st);
+        }
+        if (rc) return rc;
         if (blas().dgemm(bh, CUBLAS_OP_N, CUBLAS_OP_T, nvec, nov, nat, &one, G, nvec, q_ov, nov, &zero, us, nvec) !=
             CUBLAS_STATUS_SUCCESS)
             return fail(DFTB_ERR_CUDA, "coulomb: cublasDgemm (q_ov^T G) failed");
