@@ -446,12 +446,15 @@ __device__ __forceinline__ void dgemm_tile(const GemmP &p, int bx, int by, int b
     const int kchunk = ((p.K + p.ksplit - 1) / p.ksplit + BK - 1) / BK * BK;
     const int k0 = zk * kchunk, k1 = min(p.K, k0 + kchunk);
     const int niter = k1 > k0 ? (k1 - k0 + BK - 1) / BK : 0;
-    auto noff = [&](int n, long long s1, long long s2) { return (n / p.N2) * s1 + (n % p.N2) * s2; };
+    auto noff = [&](int n, long long s1, long long s2) {
+        const int q = p.N2 >= p.N ? 0 : n / p.N2;  // no division for a plain index
+        return q * s1 + (n - q * p.N2) * s2;
+    };
 
     // this thread's part of a stage: eight elements of each operand, along its contiguous index from thread to thread
     const int ka = AK ? tid & 15 : tid >> 6, ma = AK ? tid >> 4 : tid & 63;
     const int kb = BNC ? tid >> 6 : tid & 15, nb = BNC ? tid & 63 : tid >> 4;
-    int kq = (k0 + ka) / p.K2, kr = (k0 + ka) % p.K2;  // two-level k of A (AK)
+    int kq = p.K2 >= p.K ? 0 : (k0 + ka) / p.K2, kr = k0 + ka - kq * p.K2;  // two-level k of A (AK)
     const double *bcol = B + (BNC && bn + nb < p.N ? noff(bn + nb, p.sbn1, p.sbn) : 0);
     long long boff[8];
     if (!BNC) {
