@@ -70,23 +70,6 @@ __device__ __forceinline__ void load_row16(const float *src, int n, float out[16
     }
 }
 
-__device__ __forceinline__ void store_row16(float *dst, int n, const float v[16]) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(dst);
-    if (n == 16 && (a & 15) == 0) {
-        float4 *d4 = reinterpret_cast<float4 *>(dst);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-    } else if (n == 16 && (a & 7) == 0) {
-        float2 *d2 = reinterpret_cast<float2 *>(dst);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) d2[q] = make_float2(v[2 * q], v[2 * q + 1]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (j < n) dst[j] = v[j];
-    }
-}
-
 // Eight epilogue warps, two per TMEM lane quarter with every other 32-column chunk each: the epilogues with a Hadamard
 // factor or a transposed output are instruction-bound, and with four warps they outlasted the next tile's MMAs (a dense
 // layer of 65536 x 256: 50 us with four warps, 32 us with eight).
@@ -492,6 +475,39 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                 write_block(T, p.ldt, col0, row0, p.N, p.M);
             }
         };
+        // this warp's block of FP32 values (a row per lane) to C, 16 columns at a time through the same staging rows: 64-byte
+        // pieces of eight rows a store, or of two where rows are off the 16-byte grid.  (16 bytes of 32 rows a store, by eight
+        // warps at a time, took more: 8292 x 8292 x 1225 on 128 x 128 tiles 679 us, 2312 x 8252 x 44 45 us.)
+        const bool vec_c = ((reinterpret_cast<uintptr_t>(p.C) | (uintptr_t)p.ldc * sizeof(float)) & 15) == 0;
+        auto write_f32 = [&](const float *x, int row0, int col0) {
+            float *sf = reinterpret_cast<float *>(sh);
+            constexpr int PITCH = TPITCH / 2;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    *reinterpret_cast<float4 *>(sf + lane * PITCH + 4 * q) =
+                        make_float4(x[16 * h + 4 * q], x[16 * h + 4 * q + 1], x[16 * h + 4 * q + 2], x[16 * h + 4 * q + 3]);
+                __syncwarp();
+                if (vec_c && p.N - col0 >= 32) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int rl = q * 8 + (lane >> 2), r = row0 + rl, cl = 4 * (lane & 3);
+                        if (r < p.M)
+                            *reinterpret_cast<float4 *>(p.C + (long long)r * p.ldc + col0 + 16 * h + cl) =
+                                *reinterpret_cast<const float4 *>(sf + rl * PITCH + cl);
+                    }
+                } else {
+                    const int cl = lane & 15, c = col0 + 16 * h + cl;
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) {
+                        const int rl = q * 2 + (lane >> 4), r = row0 + rl;
+                        if (r < p.M && c < p.N) p.C[(long long)r * p.ldc + c] = sf[rl * PITCH + cl];
+                    }
+                }
+                __syncwarp();
+            }
+        };
         int j = 0;
         for (int t = tile0; t < ntiles; t += tstep, ++j) {
             const TileCoords tc = tile_coords(PAIR, t, mt, nt, BMX, BNX, BKX, C::KU, kper, p.K);
@@ -582,12 +598,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
 #pragma unroll
                             for (int q = 0; q < 32; ++q) v[q] *= g[q];
                         }
-                        if (p.C) {
-                            store_row16(p.C + (long long)row * p.ldc + col0, n1, v);
-                            if (n2 > 0) store_row16(p.C + (long long)row * p.ldc + col0 + 16, n2, v + 16);
-                        }
                     }
                 }
+                if (p.C && p.ksplit == 1 && live && col0 < p.N) write_f32(v, m0 + rq * 32, col0);
                 if ((p.Ohi || p.Thi) && p.ksplit == 1 && live && col0 < p.N) {  // rows beyond M are staged, not written
                     __nv_bfloat16 x[32];
 #pragma unroll
