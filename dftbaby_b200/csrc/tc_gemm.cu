@@ -710,10 +710,15 @@ int make_map(CUtensorMap *map, const void *base, int rows, int cols, long long l
 // 128 x 256 split tiles go to CTA pairs unless less than one round of tiles meets a short K range: there the pair's start
 // and finish cost more than its main loop saves.  B200, cold L2, us with pairs and without: 1281 x 1281 x 640 (66 tiles)
 // 26.6 and 24.6, 808 x 808 x 202 30.7 and 28.7; 385 x 8192 x 4096 (128 tiles) 78 and 84, 3000 x 3000 x 1000 (288) 49 and
-// 51, 2436 x 2436 x 609 (200) 57 and 57, 2450 x 1225 x 8292 in four K ranges 171 and 194.
+// 51, 2436 x 2436 x 609 (200) 57 and 57, 2450 x 1225 x 8292 in four K ranges 171 and 194.  Nor are they better with few tiles
+// (warm L2: 7234 x 131 x 1170, 57 tiles, 28.8 and 26.7, 256 x 8192 x 2000, 64 tiles, 39.0 and 37.6; 2048 x 1280 x 1100, 80
+// tiles, 26.7 and 28.8), or where an odd number of row tiles gives the pairs more rounds of the GPU, a round of theirs being
+// about a tenth shorter (1104 x 128 x 200000 in 16 K ranges, two rounds of 80 pairs or one of 144 tiles, 377 and 258).
 bool pair_tiles(int M, int N, int K, int ksplit) {
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256) * ksplit;
-    return M > BM && (tiles > 148 || K / ksplit >= 1024);
+    const long long columns = (long long)((N + 255) / 256) * ksplit;
+    const long long tiles = (M + BM - 1) / BM * columns, pairs = (M + 2 * BM - 1) / (2 * BM) * columns;
+    const long long rounds = (tiles + 147) / 148, pair_rounds = (pairs + 73) / 74;
+    return M > BM && (tiles > 148 || (tiles >= 80 && K / ksplit >= 1024)) && 9 * pair_rounds <= 10 * rounds;
 }
 
 // mode: 0 segments, 1 split, 2 split with 128 x 256 tiles, 3 segments with a dense layer's epilogue, 4 split with pair tiles
