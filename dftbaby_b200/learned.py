@@ -22,9 +22,10 @@ the Mulliken transition charges about the centroid), the participation ratio
 (sum q^2)^2 / sum q^4, and log(1 + rank of omega_ia).
 
 The network is 64 (zero-padded features) -> 256 -> 256 -> 2 with ReLU, BF16 weights and
-activations, FP32 accumulation.  Its matrix products run on the tcgen05 tensor cores
-(dftb_bf16x3_gemm_ex with one BF16 segment); bias/ReLU, the loss and its gradient, the ReLU
-backward pass and Adam are the dftb_mlp_* kernels.  Training uses these kernels only.
+activations, FP32 accumulation.  Its hidden layers run on the tcgen05 tensor cores with bias, ReLU, mask
+and bias gradient in the epilogue (dftb_mlp_dense; the weight gradients by dftb_bf16x3_gemm_ex with one
+BF16 segment); the output layer with the loss and its gradient, the standardised inputs and Adam are
+the other dftb_mlp_* kernels.  Training uses these kernels only.
 """
 import ctypes
 import math
@@ -39,12 +40,7 @@ NFEAT = 8
 FPAD = 64
 HIDDEN = 256
 NOUT = 2
-OPAD = 128      # rows of the output-layer weight block handed to the GEMM (rows >= NOUT are zero)
 SPAD = 128      # sample counts are padded to this multiple
-
-
-def _bf16(rows, cols, dev):
-    return torch.zeros((rows, cols), dtype=torch.bfloat16, device=dev)
 
 
 def _mm(A, B, M, N, K, C, ksplit=1, zeroed=False):
@@ -108,14 +104,10 @@ class GuessNet:
         self._refresh_bf16()
 
     def _refresh_bf16(self):
-        dev = self.device
         self.W1b = self.W1.to(torch.bfloat16).contiguous()
         self.W2b = self.W2.to(torch.bfloat16).contiguous()
         self.W2bT = self.W2.T.to(torch.bfloat16).contiguous()
-        self.W3b = _bf16(OPAD, HIDDEN, dev)
-        self.W3b[:NOUT] = self.W3.to(torch.bfloat16)
-        self.W3bT = _bf16(HIDDEN, FPAD, dev)
-        self.W3bT[:, :NOUT] = self.W3.T.to(torch.bfloat16)
+        self.W3b = self.W3.to(torch.bfloat16).contiguous()
 
     # ------------------------------------------------------------ data layout
     def _inputs(self, feats, weights=None, msum=None):
@@ -208,7 +200,7 @@ class GuessNet:
         self.step += 1
         P, st = native.ptr, native.stream()
         bf = [(self.W1b, FPAD, None, 0), (None, 0, None, 0), (self.W2b, HIDDEN, self.W2bT, HIDDEN), (None, 0, None, 0),
-              (self.W3b, HIDDEN, self.W3bT, FPAD), (None, 0, None, 0)]
+              (self.W3b, HIDDEN, None, 0), (None, 0, None, 0)]
         for p, g, (m1, m2), (wb, ldwb, wbt, ldwbt) in zip(self.params, grads, self.mom, bf):
             rows, cols = (p.shape[0], p.shape[1]) if p.dim() == 2 else (1, p.shape[0])
             native.call("dftb_mlp_adam", rows, cols, P(p), P(g), P(m1), P(m2), float(lr), 0.9, 0.999, 1e-8,
