@@ -374,7 +374,10 @@ const char *dftb_grad_last_error(void);
  * for the initial Davidson vectors and corrects the diagonal preconditioner.
  * Its matrix products run through dftb_bf16x3_gemm_ex (one BF16 segment, FP32
  * accumulation); these kernels do the work in between.  Activations and
- * weight copies are BF16 (passed as void *), everything else FP32; row-major. */
+ * weight copies are BF16 (passed as void *), everything else FP32; row-major.
+ * dftb_mlp_bias_relu, _relu_backward and _output are the layers' parts one by one,
+ * for callers of this interface; the Python network runs on the fused layers
+ * further down. */
 
 /* H = relu(Z + b) for ns samples x nh units; H (ldh) and, unless HT is NULL,
  * H^T (nh x ns, ldht). */
