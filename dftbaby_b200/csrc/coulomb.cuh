@@ -38,8 +38,8 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 // 16-byte grid: its window then begins one element early (at the row's `phase`) and takes a 17th piece, and the
 // fragment reads add the phase.  Warps are 4 (rows) x 2 (halves of a stage), two row tiles each; for the Hermitian
 // form four warps turn omega into sqrt(omega) every fourth stage (a square root is a long serial chain, so it should
-// hold the stage's barrier up as seldom as possible), and the V fragments are multiplied as they are read.  Two CTAs per SM keep ~100 KB in flight.  The row pitches are 4 (mod 16) doubles, which keeps the fragment
-// reads (nearly) conflict-free.
+// hold the stage's barrier up as seldom as possible), and the V fragments are multiplied as they are read.  Two CTAs per SM
+// keep ~100 KB in flight.  The row pitches are 4 (mod 16) doubles, which keeps the fragment reads (nearly) conflict-free.
 constexpr int QV_M = 64, QV_P = 36, QV_STAGES = 4, QV_THREADS = 256;
 
 template <int NT> struct Skinny {  // NT tiles of 8 columns

@@ -45,7 +45,7 @@ constexpr int kModuli[MAXMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 22
 constexpr int KMAX = 131071;                // 128 * 128 * K < 2^31: exact int32 accumulation
 constexpr int SCALE_NONFINITE = -(1 << 20);  // row/column exponent marking an Inf or NaN entry
 
-// Per modulus p; residues are symmetric (|r| <= p / 2) and formed in FP32, see symres().
+// Per modulus p; residues are symmetric (|r| <= p / 2) and formed in FP32, see symres2().
 struct Tables {
     float2 np[MAXMOD], invp[MAXMOD];    // -p and 1 / p, twice: the FP32 pair operands
     uint32_t blo[MAXMOD], bhi[MAXMOD];  // int8 weights 2^(8 j) mod p of the bytes j = 0..3 and 4..7
@@ -146,7 +146,7 @@ __global__ void ozaki_rowscale_kernel(int rows, int rpad, int K, const double *X
 }
 
 // The same for rows that are strided in memory (Y(r, k) = X[k * ldx + r]): a cluster of RC_SPLIT CTAs takes 32 rows
-// (consecutive in memory), each CTA a range of k with 16 phases, and the first CTA joins their maxima.
+// (consecutive in memory), each CTA a range of k with RC_PHASES phases, and the first CTA joins their maxima.
 // Split because 4146 rows are 130 blocks, too few loads in flight for one pass over 137 MB: 42 -> 39 us for 4146 x 4146,
 // and 96 us before with 32 phases in one block.
 constexpr int RC_SPLIT = 8, RC_PHASES = 8;

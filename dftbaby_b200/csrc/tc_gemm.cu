@@ -206,9 +206,9 @@ struct TileCoords {
     int m0, n0, k0, kend, kblocks;  // kblocks of bkx elements cover k0 .. kend
 };
 
-// Pair tiles of tall outputs run in bands of BAND tile columns, N-fastest, so that the tiles at work at one time (74) are
-// about as many rows as columns and
-// touch little of both operands (33 x 33 tiles M-fastest send all 41 MB of A past the outputs' stream in every round).
+// Pair tiles of tall outputs run in bands of BAND tile columns, N-fastest, so that the tiles at work at one time (74) span
+// about as many rows as columns and touch little of both operands (33 x 33 tiles M-fastest send all 41 MB of A past the
+// outputs' stream in every round).
 // B200, N 8292 x 8292 x 1225: DRAM reads 883 -> 640 MB, 452 -> 427 us; the products' order is unchanged.
 constexpr int BAND = 8, BAND_ROWS = 16;
 

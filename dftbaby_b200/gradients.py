@@ -12,10 +12,9 @@ gradient_nolc, :713-981), reorganised for the GPU:
   <W, F[v]>_n or <W, F^lr[v]>_n, so here the operators are transposed once per (v, W)
   pair into adjoint matrices X (Norb x Norb) and Y (Nat x Nat) with
   <W, F[v]>_n = <gradS_n, X> + <gradGamma_n, Y> (a few Norb^3 GEMMs in total);
-* the native kernels then evaluate the spline derivatives of every orbital pair on
-  the fly and contract them with X (dftb_sk_gradient_contract), and the gamma,
-  gamma^lr and repulsive-potential derivatives of every atom pair with Y
-  (dftb_pair_gradients): the 3 Nat Norb^2 tensors are never written;
+* one native kernel per molecule (dftb_gradient_contract) then evaluates the spline
+  derivatives of every atom pair and contracts them with X, and the gamma, gamma^lr and
+  repulsive-potential derivatives with Y: the 3 Nat Norb^2 tensors are never written;
 * the Z-vector equation (A+B) Z = R is solved by DFTBaby's Krylov scheme
   (Solver.py:921-1012) on the device with the same (A+B) products the Davidson
   solver uses.
@@ -27,7 +26,8 @@ from . import native
 
 
 def _block_sum(Y, ind, nat):
-    """Atom-block sums A[I][J] = sum_{a on I, b on J} Y[a][b]."""
+    """Atom-block sums A[I][J] = sum_{a on I, b on J} Y[a][b], as dftb_gradient_contract forms them (the adjoint tests'
+    restatement)."""
     dev = Y.device
     Aop = torch.zeros((nat, Y.shape[0]), dtype=Y.dtype, device=dev)
     Aop[ind.long(), torch.arange(Y.shape[0], device=dev)] = 1.0
