@@ -1346,9 +1346,9 @@ __global__ void __launch_bounds__(256) exchange_unpack_kernel(int m, int nv, int
 }
 
 // (A+B) v = (u - K1) - K2 and (A-B) v = (omega v + K2) - K1 from the same Kall (FP32 or FP64), u = Coulomb products, in
-// place of one pass that unpacks K1 and K2 and five element-wise ones; each operand moves once, at 3.1 TB/s, half the rate
-// of a copy: a block's loads wait for the barrier of its transposed tile, one round at a time.  A block takes 32 i and as
-// many a as make 64 of the contiguous (a, c); rounded as the separate passes were.  B200, 1225 x 1225: 700 us -> 315 us
+// place of one pass that unpacks K1 and K2 and five element-wise ones; each operand moves once, at 3.1 to 3.5 TB/s, half the
+// rate of a copy: the warps wait for the transposed tile in shared memory (two thirds of their stalls) and for its index
+// divisions.  A block takes 32 i and as many a as make 64 of the contiguous (a, c); rounded as the separate passes were.  B200, 1225 x 1225: 700 us -> 315 us
 // (FP32, 16 columns, 0.96 GB), 253 -> 91 us (FP64, 4 columns, 0.29 GB).  Four elements a thread in flight made it 450 us.
 template <typename T>
 __global__ void __launch_bounds__(256) exchange_combine_kernel(int m, int nv, int no, const T *__restrict__ Kall,
