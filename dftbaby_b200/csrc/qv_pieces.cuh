@@ -25,14 +25,16 @@ struct QvPiece {
 
 // piece pc of the first stage of a row; further stages begin QV_K columns on each
 QV_FN QvPiece qv_piece(const double *Q, int M, int K, int row, int kbeg, int kend, int pc) {
-    if (row >= M) return {Q + ((reinterpret_cast<uintptr_t>(Q) >> 3) & 1), 0};
-    const int k = kbeg - qv_phase(Q, K, row, kbeg) + 2 * pc;
-    return {Q + ((ptrdiff_t)row * K + k), kend - k};
+    // rows beyond the matrix read nothing from a place in its last row (a piece further on, so not before a lone first row)
+    const bool in = row < M;
+    const int r = in ? row : M - 1;
+    const int k = kbeg - qv_phase(Q, K, r, kbeg) + 2 * (in ? pc : pc + 1);
+    return {Q + ((ptrdiff_t)r * K + k), in ? kend - k : 0};
 }
 
 // source of a copy of n elements in the stage at column k0: the piece's own start where there is nothing to read.  (A piece
 // that starts before Q has elements to read in every stage of its range, so the sum in the second case is src; without it
-// the kernel takes 2 % longer at 336 atoms x 370881 pairs, 10 columns.)
+// the kernel's registers are dealt differently and it takes 2 % longer at 336 atoms x 370881 pairs, 10 columns.)
 QV_FN const double *qv_source(const QvPiece &p, const double *Q, int k0, int n) {
     return n > 0 ? p.src + k0 : p.src + (Q > p.src);
 }

@@ -64,7 +64,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("off", [0, 1])
-@pytest.mark.parametrize("M,K,kbeg,kend", [(1, 1, 0, 1), (37, 99, 0, 99), (64, 33, 0, 33), (65, 31, 0, 31), (3, 64, 32, 64),
+@pytest.mark.parametrize("M,K,kbeg,kend", [(1, 1, 0, 1), (1, 99, 0, 99), (1, 97, 32, 97), (37, 99, 0, 99), (64, 33, 0, 33), (65, 31, 0, 31), (3, 64, 32, 64),
                                            (5, 257, 64, 192), (5, 257, 192, 257), (63, 32, 0, 32), (2, 95, 64, 95)])
 def test_copies(program, M, K, kbeg, kend, off):
     r = subprocess.run([program] + [str(x) for x in (M, K, off, kbeg, kend)], capture_output=True, text=True)
