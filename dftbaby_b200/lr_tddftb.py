@@ -94,8 +94,10 @@ class ExchangeAO:
         return coul - K1 - K2, omv + K2 - K1
 
     def _products(self, V):
-        """__call__ from the interleaved K1^T, K2^T of _exchange_interleaved: one pass forms both results."""
-        if not self.lc:
+        """__call__ from the interleaved K1^T, K2^T of _exchange_interleaved: one pass forms both results.  Not for objects
+        with an exchange() or coulomb() of their own, whose results are used as they are."""
+        own = any(getattr(type(self), n) is not f or n in self.__dict__ for n, f in self._terms.items())
+        if own or not self.lc:
             return ExchangeAO.__call__(self, V)
         self.products_applied += V.shape[1]
         V = V.contiguous()
@@ -237,6 +239,9 @@ class ExchangeMixed(ExchangeAO):
         return K1, K2
 
 
+ExchangeMixed._terms = {"exchange": ExchangeMixed.exchange, "coulomb": ExchangeMixed.coulomb}
+
+
 class ExchangeOzaki(ExchangeAO):
     """(A+B).V and (A-B).V with the exchange in FP64, its products on the int8 tensor cores.
 
@@ -299,6 +304,9 @@ class ExchangeOzaki(ExchangeAO):
         m, no, nv = V.shape[1], self.nocc, self.nvirt
         K = Kall.view(m, nv, 2, no).permute(2, 3, 1, 0).reshape(2, no * nv, m)
         return K[0], K[1]
+
+
+ExchangeOzaki._terms = {"exchange": ExchangeOzaki.exchange, "coulomb": ExchangeOzaki.coulomb}
 
 
 class LR_TDDFTB:
