@@ -1067,7 +1067,13 @@ int skinny_product(int M, int K, const double *Q, const double *V, int ncol, dou
     const unsigned rows = cdiv(M, QV_M), cols = cdiv(ncol, 32);
     const long long want = 296 / ((long long)rows * cols);
     const long long chunks = cdiv(K, QV_K);
+    // Up to four stages a range where there are ranges enough: each range adds all of T once more, to the same few elements
+    // where Q has few rows.  B200, Hermitian product, us with one, two and four stages at least: 54 atoms x 6084 pairs, 10
+    // columns 24.3, 18.5, 16.4, 32 columns 32.1, 25.4, 23.5; 90 x 12321, 10 columns 28.9 (three) and 23.1; but 14 x 256 12.3,
+    // 12.3 and 14.4.
+    const long long least = chunks < 48 ? 1 : (chunks < 96 ? chunks / 24 : 4);
     long long ks = want < 1 ? 1 : (want > chunks ? chunks : want);
+    if (ks > chunks / least) ks = chunks / least;
     const long long per = (chunks + ks - 1) / ks;
     ks = (chunks + per - 1) / per;
     const QvP p{M, K, Q, V, ncol, ncol, T, ncol, omega, (int)(per * QV_K), after};
