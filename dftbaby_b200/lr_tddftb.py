@@ -96,8 +96,9 @@ class ExchangeAO:
     def _products(self, V):
         """__call__ from the interleaved K1^T, K2^T of _exchange_interleaved: one pass forms both results.  Not for objects
         with an exchange() or coulomb() of their own, whose results are used as they are."""
-        own = any(getattr(type(self), n) is not f or n in self.__dict__ for n, f in self._terms.items())
-        if own or not self.lc:
+        cls, own = type(self), self.__dict__
+        if (not self.lc or cls.exchange is not self._terms[0] or cls.coulomb is not self._terms[1] or "exchange" in own
+                or "coulomb" in own):
             return ExchangeAO.__call__(self, V)
         self.products_applied += V.shape[1]
         V = V.contiguous()
@@ -239,7 +240,7 @@ class ExchangeMixed(ExchangeAO):
         return K1, K2
 
 
-ExchangeMixed._terms = {"exchange": ExchangeMixed.exchange, "coulomb": ExchangeMixed.coulomb}
+ExchangeMixed._terms = (ExchangeMixed.exchange, ExchangeMixed.coulomb)
 
 
 class ExchangeOzaki(ExchangeAO):
@@ -306,7 +307,7 @@ class ExchangeOzaki(ExchangeAO):
         return K[0], K[1]
 
 
-ExchangeOzaki._terms = {"exchange": ExchangeOzaki.exchange, "coulomb": ExchangeOzaki.coulomb}
+ExchangeOzaki._terms = (ExchangeOzaki.exchange, ExchangeOzaki.coulomb)
 
 
 class LR_TDDFTB:
